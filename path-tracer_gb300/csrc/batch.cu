@@ -163,40 +163,41 @@ constexpr int blocks_for(int kMinBlocks, int kBaseThreads, int kThreads) {
     return kMinBlocks * kBaseThreads / kThreads > 0 ? kMinBlocks * kBaseThreads / kThreads : 1;
 }
 
+template <bool kWide>
+PTD LaneScene lane_scene(const SceneDev* sc) {
+    return LaneScene{&sc->w, &sc->f, kWide ? sc->f.wide : sc->f.pairs, sc->f.tri4};
+}
+
 template <bool kAlpha, bool kWide, int kThreads = kExtendThreads>
 __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS, kExtendThreads, kThreads))
     extend_kernel(const SceneDev* scenes, WaveBufs b, int cur, uint32_t steps_per_refill) {
     static_assert(!(kAlpha && kWide), "the wide form runs opaque scenes only");
     const Stage st = stage_of(b.q, cur);
     const uint32_t count = *st.count;
-    typename std::conditional<kWide, WideTraverser<false>, Traverser<false, kAlpha, false>>::type tr;
+    using Ray = typename std::conditional<kWide, WideRay<false, LaneScene>,
+                                          BinaryRay<false, kAlpha, false, false, LaneScene>>::type;
+    Ray ray(LaneScene{});
     constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
     __shared__ uint2 stack_top[kShared > 0u ? kShared * kThreads : 1u];
     LaneStack<kThreads, kShared> stack;
     stack.col = stack_top + threadIdx.x;
     uint32_t istack[1];
-    const SceneDev* sc = scenes;
     uint32_t slot = 0;
-    __shared__ FilerSlots<kThreads> filer_slots;
-    ResultFiler filer = filer_slots.of_warp(lane_id());
-    lane_refill_loop(
-        &b.q.cnt[3], count, kWide ? (uint32_t)kWideStepsPerRefill : steps_per_refill, kRefillBelow,
+    traverse_queue(
+        count, kWide ? kWideStepsPerRefill : steps_per_refill, ray, stack, istack,
         [&](uint32_t i) {
             slot = i;
             const float4 o4 = st.o[i], d4 = st.d[i];
-            sc = scenes + (b.tag[__float_as_uint(o4.w)] & 0xffu);
-            tr.rng.s = __float_as_uint(d4.w);
-            stack.reset();
-            tr.init(sc->f, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1);
+            ray.sc = lane_scene<kWide>(scenes + (b.tag[__float_as_uint(o4.w)] & 0xffu));
+            ray.rng.s = __float_as_uint(d4.w);
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1);
         },
-        [&]() {
-            if (!tr.step(sc->w, sc->f, stack, istack)) return false;
-            b.q.hit[slot] = make_float4(tr.hit_t, __int_as_float(tr.hit), tr.hv, tr.hw);
-            if constexpr (kAlpha) st.d[slot].w = __uint_as_float(tr.rng.s);
-            filer.file(slot, tr.hit != -1);
-            return true;
-        },
-        [&]() { filer.flush(b.q, lane_id()); });
+        [&](uint32_t want) {
+            if constexpr (kAlpha) {
+                if (ray.todo == kFinished) st.d[slot].w = __uint_as_float(ray.rng.s);
+            }
+            return file_and_fetch(b.q, ray, slot, want);
+        });
 }
 
 template <bool kAlpha, int kThreads = kShadeThreads>
@@ -269,35 +270,33 @@ template <bool kWide, int kThreads = kExtendThreads>
 __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS, kExtendThreads, kThreads))
     shadow_kernel(const SceneDev* scenes, WaveBufs b, uint32_t steps_per_refill) {
     const uint32_t count = b.q.cnt[2];
-    typename std::conditional<kWide, WideTraverser<true>, Traverser<false, false, true, false, PT_SHADOW_TRI_PER_STEP != 0>>::type tr;
+    using Ray = typename std::conditional<kWide, WideRay<true, LaneScene>,
+                                          BinaryRay<false, false, true, false, LaneScene>>::type;
+    Ray ray(LaneScene{});
     constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
     __shared__ uint2 stack_top[kShared > 0u ? kShared * kThreads : 1u];
     LaneStack<kThreads, kShared> stack;
     stack.col = stack_top + threadIdx.x;
     uint32_t istack[1];
-    const SceneDev* sc = scenes;
     uint32_t path = 0;
-    float4 contribution = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    lane_refill_loop(
-        &b.q.cnt[4], count, kWide ? (uint32_t)kWideStepsPerRefill : steps_per_refill, kRefillBelow,
+    f3 contribution = mk(0.0f, 0.0f, 0.0f);
+    traverse_queue(
+        count, kWide ? kWideStepsPerRefill : steps_per_refill, ray, stack, istack,
         [&](uint32_t i) {
-            const float4 o4 = b.q.so[i], d4 = b.q.sd[i];
-            contribution = b.q.sc[i];
+            const float4 o4 = b.q.so[i], d4 = b.q.sd[i], c4 = b.q.sc[i];
+            contribution = mk(c4.x, c4.y, c4.z);
             path = __float_as_uint(o4.w);
-            sc = scenes + (b.tag[path] & 0xffu);
-            stack.reset();
-            tr.init(sc->f, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(contribution.w));
+            ray.sc = lane_scene<kWide>(scenes + (b.tag[path] & 0xffu));
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w));
         },
-        [&]() {
-            if (!tr.step(sc->w, sc->f, stack, istack)) return false;
-            if (tr.hit != 1) {
+        [&](uint32_t want) {
+            if (ray.todo == kFinished && ray.hit != 1) {
                 const float4 col = b.q.color[path];
-                const f3 sum = mk(col.x, col.y, col.z) + mk(contribution.x, contribution.y, contribution.z);
+                const f3 sum = mk(col.x, col.y, col.z) + contribution;
                 b.q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
             }
-            return true;
-        },
-        NoRound(), step_kind<PT_MAJORITY_SHADOW && !kWide>(tr, [&]() -> const Fast& { return sc->f; }));
+            return fetch_entries(&b.q.cnt[4], want);
+        });
 }
 
 // accumulate, trace.slang:1299-1308: one block per item, samples in order;

@@ -125,39 +125,35 @@ __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : P
     static_assert(!(kWide && (kRec || kAlpha)), "the wide form keeps no records and runs opaque scenes only");
     const Stage st = stage_of(q, cur);
     const uint32_t count = *st.count;
-    const bool ordered = PT_RAY_ORDER && q.cnt[8] != 0u;
-    typename std::conditional<kWide, WideTraverser<false, kTri36>, Traverser<kRec, kAlpha, false, kTri36>>::type tr;
+    using Ray = typename std::conditional<kWide, WideRay<false, OneScene>,
+                                          BinaryRay<kRec, kAlpha, false, kTri36, OneScene>>::type;
+    Ray ray(OneScene{w, f});
     constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
     __shared__ uint2 stack_top[kShared > 0u ? kShared * kExtendThreads : 1u];
     LaneStack<kExtendThreads, kShared> stack;
     stack.col = stack_top + threadIdx.x;
     uint32_t istack[kRec ? 64 : 1];
     uint32_t slot = 0, path = 0;
-    __shared__ FilerSlots<kExtendThreads> filer_slots;
-    ResultFiler filer = filer_slots.of_warp(lane_id());
-    lane_refill_loop(
-        &q.cnt[3], count, kWide ? kWideStepsPerRefill : kStepsPerRefill, kRefillBelow,
+    traverse_queue(
+        count, kWide ? kWideStepsPerRefill : kStepsPerRefill, ray, stack, istack,
         [&](uint32_t i) {
-            slot = ordered ? q.hit_sorted[i] : i;
+            slot = i;
             const float4 o4 = st.o[slot], d4 = st.d[slot];
             path = __float_as_uint(o4.w);
-            tr.rng.s = __float_as_uint(d4.w);
-            if constexpr (kRec) tr.c = q.rec[path];
-            stack.reset();
-            tr.init(f, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1);
+            ray.rng.s = __float_as_uint(d4.w);
+            if constexpr (kRec) ray.c = q.rec[path];
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1);
         },
-        [&]() {
-            if (!tr.step(w, f, stack, istack)) return false;
-            q.hit[slot] = make_float4(tr.hit_t, __int_as_float(tr.hit), tr.hv, tr.hw);
-            if constexpr (kAlpha) st.d[slot].w = __uint_as_float(tr.rng.s);
-            if constexpr (kRec) {
-                q.rec[path] = tr.c;
-                if (bounce < PT_RECORD_MAX_BOUNCES) q.rec_hits[(size_t)path * PT_RECORD_MAX_BOUNCES + bounce] = tr.hit;
+        [&](uint32_t want) {
+            if (ray.todo == kFinished) {
+                if constexpr (kAlpha) st.d[slot].w = __uint_as_float(ray.rng.s);
+                if constexpr (kRec) {
+                    q.rec[path] = ray.c;
+                    if (bounce < PT_RECORD_MAX_BOUNCES) q.rec_hits[(size_t)path * PT_RECORD_MAX_BOUNCES + bounce] = ray.hit;
+                }
             }
-            filer.file(slot, tr.hit != -1, min((uint32_t)tr.hit >> q.key_shift, kSortBuckets - 1u));
-            return true;
-        },
-        [&]() { filer.flush(q, lane_id()); }, step_kind<PT_MAJORITY_EXTEND && !kWide>(tr, [&]() -> const Fast& { return f; }));
+            return file_and_fetch(q, ray, slot, want);
+        });
 }
 
 template <bool kRec, bool kAlpha>
@@ -234,38 +230,36 @@ template <bool kRec, bool kTri36 = false, bool kWide = false>
 __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS) shadow_kernel(World w, Fast f, Queues q) {
     static_assert(!(kWide && kRec), "the wide form keeps no records");
     const uint32_t count = q.cnt[2];
-    const bool ordered = PT_SHADOW_ORDER && q.cnt[9] != 0u;
-    typename std::conditional<kWide, WideTraverser<true, kTri36>,
-                              Traverser<kRec, false, true, kTri36, PT_SHADOW_TRI_PER_STEP != 0>>::type tr;
+    using Ray = typename std::conditional<kWide, WideRay<true, OneScene>,
+                                          BinaryRay<kRec, false, true, kTri36, OneScene>>::type;
+    Ray ray(OneScene{w, f});
     constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
     __shared__ uint2 stack_top[kShared > 0u ? kShared * kExtendThreads : 1u];
     LaneStack<kExtendThreads, kShared> stack;
     stack.col = stack_top + threadIdx.x;
     uint32_t istack[kRec ? 64 : 1];
     uint32_t path = 0;
-    float4 contribution = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    lane_refill_loop(
-        &q.cnt[4], count, kWide ? kWideStepsPerRefill : kStepsPerRefill, kRefillBelow,
+    f3 contribution = mk(0.0f, 0.0f, 0.0f);
+    traverse_queue(
+        count, kWide ? kWideStepsPerRefill : kStepsPerRefill, ray, stack, istack,
         [&](uint32_t i) {
-            const uint32_t slot = ordered ? q.hit_sorted[i] : i;
-            const float4 o4 = q.so[slot], d4 = q.sd[slot];
-            contribution = q.sc[slot];
+            const float4 o4 = q.so[i], d4 = q.sd[i], c4 = q.sc[i];
+            contribution = mk(c4.x, c4.y, c4.z);
             path = __float_as_uint(o4.w);
-            if constexpr (kRec) tr.c = q.rec[path];
-            stack.reset();
-            tr.init(f, mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(contribution.w));
+            if constexpr (kRec) ray.c = q.rec[path];
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w));
         },
-        [&]() {
-            if (!tr.step(w, f, stack, istack)) return false;
-            if (tr.hit != 1) {
-                const float4 col = q.color[path];
-                const f3 sum = mk(col.x, col.y, col.z) + mk(contribution.x, contribution.y, contribution.z);
-                q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
+        [&](uint32_t want) {
+            if (ray.todo == kFinished) {
+                if (ray.hit != 1) {
+                    const float4 col = q.color[path];
+                    const f3 sum = mk(col.x, col.y, col.z) + contribution;
+                    q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
+                }
+                if constexpr (kRec) q.rec[path] = ray.c;
             }
-            if constexpr (kRec) q.rec[path] = tr.c;
-            return true;
-        },
-        NoRound(), step_kind<PT_MAJORITY_SHADOW && !kWide>(tr, [&]() -> const Fast& { return f; }));
+            return fetch_entries(&q.cnt[4], want);
+        });
 }
 
 // accumulate, trace.slang:1299-1308, samples of the group in order
@@ -386,14 +380,18 @@ __global__ void debug_intersect_wide_kernel(World w, Fast f, uint64_t n, const f
                                             const float* t_max, int32_t* hit, float* hit_t) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    WideTraverser<false> tr;
+    WideRay<false, OneScene> ray(OneScene{w, f});
     LocalStack stack;
-    tr.init(f, mk(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2]),
-            mk(directions[3 * i], directions[3 * i + 1], directions[3 * i + 2]), t_max ? t_max[i] : kFltMax, -1);
-    while (!tr.step(w, f, stack, nullptr)) {
+    ray.init(mk(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2]),
+             mk(directions[3 * i], directions[3 * i + 1], directions[3 * i + 2]), t_max ? t_max[i] : kFltMax, -1);
+    while (ray.todo >= 0) {
+        if (ray.todo == 0)
+            ray.visit(stack, nullptr);
+        else
+            ray.test(stack, nullptr);
     }
-    hit[i] = tr.hit;
-    hit_t[i] = tr.hit_t;
+    hit[i] = ray.hit;
+    hit_t[i] = ray.hit_t();
 }
 
 }  // namespace ptd
