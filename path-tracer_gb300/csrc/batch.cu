@@ -164,23 +164,23 @@ constexpr int blocks_for(int kMinBlocks, int kBaseThreads, int kThreads) {
 }
 
 template <bool kWide>
-PTD LaneScene lane_scene(const SceneDev* sc) {
-    return LaneScene{&sc->w, &sc->f, kWide ? sc->f.wide : sc->f.pairs, sc->f.tri4};
+PTD LaneScene<SceneDev> lane_scene(const SceneDev* scenes, uint32_t index) {
+    const Fast& f = scenes[index].f;
+    return LaneScene<SceneDev>{scenes, index, kWide ? f.wide : f.packed, f.tri4};
 }
 
-template <bool kAlpha, bool kWide, int kThreads = kExtendThreads>
+template <bool kAlpha, bool kWide, bool kPacked, int kThreads>
 __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS, kExtendThreads, kThreads))
     extend_kernel(const SceneDev* scenes, WaveBufs b, int cur, uint32_t steps_per_refill) {
     static_assert(!(kAlpha && kWide), "the wide form runs opaque scenes only");
+    static_assert(!(kPacked && kWide), "one form of the BVH");
     const Stage st = stage_of(b.q, cur);
     const uint32_t count = *st.count;
-    using Ray = typename std::conditional<kWide, WideRay<false, LaneScene>,
-                                          BinaryRay<false, kAlpha, false, false, LaneScene>>::type;
-    Ray ray(LaneScene{});
-    constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
-    __shared__ uint2 stack_top[kShared > 0u ? kShared * kThreads : 1u];
-    LaneStack<kThreads, kShared> stack;
-    stack.col = stack_top + threadIdx.x;
+    RayOf<false, kAlpha, false, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
+    using Stacks = BlockStack<kThreads, kWide, kPacked>;
+    __shared__ Stacks stacks;
+    typename Stacks::Lane stack;
+    stacks.bind(stack);
     uint32_t istack[1];
     uint32_t slot = 0;
     traverse_queue(
@@ -188,13 +188,13 @@ __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCK
         [&](uint32_t i) {
             slot = i;
             const float4 o4 = st.o[i], d4 = st.d[i];
-            ray.sc = lane_scene<kWide>(scenes + (b.tag[__float_as_uint(o4.w)] & 0xffu));
+            ray.sc = lane_scene<kWide>(scenes, b.tag[__float_as_uint(o4.w)] & 0xffu);
             ray.rng.s = __float_as_uint(d4.w);
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1);
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1, stack);
         },
         [&](uint32_t want) {
             if constexpr (kAlpha) {
-                if (ray.todo == kFinished) st.d[slot].w = __uint_as_float(ray.rng.s);
+                if (ray.finished()) st.d[slot].w = __uint_as_float(ray.rng.s);
             }
             return file_and_fetch(b.q, ray, slot, want);
         });
@@ -266,17 +266,15 @@ __global__ void __launch_bounds__(kThreads, blocks_for(PT_SHADE_MIN_BLOCKS, kSha
     }
 }
 
-template <bool kWide, int kThreads = kExtendThreads>
+template <bool kWide, bool kPacked, int kThreads>
 __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS, kExtendThreads, kThreads))
     shadow_kernel(const SceneDev* scenes, WaveBufs b, uint32_t steps_per_refill) {
     const uint32_t count = b.q.cnt[2];
-    using Ray = typename std::conditional<kWide, WideRay<true, LaneScene>,
-                                          BinaryRay<false, false, true, false, LaneScene>>::type;
-    Ray ray(LaneScene{});
-    constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
-    __shared__ uint2 stack_top[kShared > 0u ? kShared * kThreads : 1u];
-    LaneStack<kThreads, kShared> stack;
-    stack.col = stack_top + threadIdx.x;
+    RayOf<false, false, true, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
+    using Stacks = BlockStack<kThreads, kWide, kPacked>;
+    __shared__ Stacks stacks;
+    typename Stacks::Lane stack;
+    stacks.bind(stack);
     uint32_t istack[1];
     uint32_t path = 0;
     f3 contribution = mk(0.0f, 0.0f, 0.0f);
@@ -286,11 +284,11 @@ __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCK
             const float4 o4 = b.q.so[i], d4 = b.q.sd[i], c4 = b.q.sc[i];
             contribution = mk(c4.x, c4.y, c4.z);
             path = __float_as_uint(o4.w);
-            ray.sc = lane_scene<kWide>(scenes + (b.tag[path] & 0xffu));
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w));
+            ray.sc = lane_scene<kWide>(scenes, b.tag[path] & 0xffu);
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w), stack);
         },
         [&](uint32_t want) {
-            if (ray.todo == kFinished && ray.hit != 1) {
+            if (ray.finished() && ray.hit != 1) {
                 const float4 col = b.q.color[path];
                 const f3 sum = mk(col.x, col.y, col.z) + contribution;
                 b.q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
@@ -421,7 +419,8 @@ struct Scene {
     int caller_refs = 0;  // pte_scene_add minus pte_scene_release
     int job_refs = 0;     // accumulations using it
     uint64_t last_use = 0;
-    Buf geo, attr, mat, nodes, srgb, linear, sky, sky_alias, scene_alias, lut, pairs, tri4;
+    bool packable = false;  // its BVH fits the packed form
+    Buf geo, attr, mat, nodes, srgb, linear, sky, sky_alias, scene_alias, lut, packed, tri4;
     Buf wide, links, attr_h, sky_h;  // precision form (links: parent per node, leaf per triangle)
 };
 
@@ -448,12 +447,18 @@ struct Job {
     uint64_t pending_paths = 0;
     uint32_t rounds = 0;  // bounce rounds its paths can take (max_bounces + 1)
     bool alpha = false;   // its scene has non-opaque materials
+    bool plain = false;   // its scene's BVH does not fit the packed form
     std::chrono::steady_clock::time_point submitted;
 };
 
 struct Flight {
     cudaEvent_t start, stop;
 };
+
+// What a wave's kernels must handle: jobs of non-opaque scenes (bit 0), and
+// jobs of scenes without a packed BVH (bit 1: every job then traverses the
+// uploaded nodes).
+constexpr uint32_t kWaveAlpha = 1, kWavePlain = 2, kWaveKinds = 4;
 
 int hbm_fail(std::string& err, const char* what, uint64_t need, uint64_t used, uint64_t budget) {
     char msg[256];
@@ -581,8 +586,8 @@ struct pt_engine {
     ptb::WaveBufs wb{};
     uint32_t max_items = 0;
     bool wave_ready = false;
-    // one captured wave per kind (opaque / non-opaque) and number of bounce rounds
-    cudaGraphExec_t graph[2][kRounds] = {};
+    // one captured wave per kind and number of bounce rounds
+    cudaGraphExec_t graph[kWaveKinds][kRounds] = {};
     std::deque<Flight> flights;
     std::vector<cudaEvent_t> event_pool;
     pt_engine_stats stats{};
@@ -691,7 +696,7 @@ void launch_persistent(void (*kernel)(P...), pt_engine* e, int threads, A&&... a
 }
 
 // the launches of one wave (captured into a graph, or issued directly)
-template <bool kAlpha, bool kWideBvh>
+template <bool kAlpha, bool kWideBvh, bool kPacked>
 cudaError_t issue_wave(pt_engine* e, uint32_t rounds) {
     const cudaStream_t s = e->stream;
     const ItemDev* ring = e->d_ring.as<const ItemDev>();
@@ -704,10 +709,13 @@ cudaError_t issue_wave(pt_engine* e, uint32_t rounds) {
     constexpr bool kWide = kWideBvh && !kAlpha;
     const uint32_t tt = e->cfg.traversal_threads, st = e->cfg.shade_threads;
     // persistent launches: as many blocks as stay resident, for the block shape of the configuration
+    // (the uploaded nodes, a rare form, are traversed in one shape)
     const auto extend = [&](int cur) {
-        if (tt == 64u) return launch_persistent(extend_kernel<kAlpha, kWide, 64>, e, 64, scenes, e->wb, cur, e->cfg.steps_per_refill);
-        if (tt == 256u) return launch_persistent(extend_kernel<kAlpha, kWide, 256>, e, 256, scenes, e->wb, cur, e->cfg.steps_per_refill);
-        return launch_persistent(extend_kernel<kAlpha, kWide, 128>, e, 128, scenes, e->wb, cur, e->cfg.steps_per_refill);
+        if constexpr (kWide || kPacked) {
+            if (tt == 64u) return launch_persistent(extend_kernel<kAlpha, kWide, kPacked, 64>, e, 64, scenes, e->wb, cur, e->cfg.steps_per_refill);
+            if (tt == 256u) return launch_persistent(extend_kernel<kAlpha, kWide, kPacked, 256>, e, 256, scenes, e->wb, cur, e->cfg.steps_per_refill);
+        }
+        return launch_persistent(extend_kernel<kAlpha, kWide, kPacked, 128>, e, 128, scenes, e->wb, cur, e->cfg.steps_per_refill);
     };
     const auto shade = [&](int cur, uint32_t bounce) {
         if (st == 128u) return launch_persistent(shade_kernel<kAlpha, 128>, e, 128, scenes, jobs, e->wb, cur, bounce);
@@ -716,9 +724,11 @@ cudaError_t issue_wave(pt_engine* e, uint32_t rounds) {
         return launch_persistent(shade_kernel<kAlpha, 1024>, e, 1024, scenes, jobs, e->wb, cur, bounce);
     };
     const auto shadow = [&]() {
-        if (tt == 64u) return launch_persistent(shadow_kernel<kWide, 64>, e, 64, scenes, e->wb, e->cfg.steps_per_refill);
-        if (tt == 256u) return launch_persistent(shadow_kernel<kWide, 256>, e, 256, scenes, e->wb, e->cfg.steps_per_refill);
-        return launch_persistent(shadow_kernel<kWide, 128>, e, 128, scenes, e->wb, e->cfg.steps_per_refill);
+        if constexpr (kWide || kPacked) {
+            if (tt == 64u) return launch_persistent(shadow_kernel<kWide, kPacked, 64>, e, 64, scenes, e->wb, e->cfg.steps_per_refill);
+            if (tt == 256u) return launch_persistent(shadow_kernel<kWide, kPacked, 256>, e, 256, scenes, e->wb, e->cfg.steps_per_refill);
+        }
+        return launch_persistent(shadow_kernel<kWide, kPacked, 128>, e, 128, scenes, e->wb, e->cfg.steps_per_refill);
     };
     int cur = 0;
     for (uint32_t bounce = 0; bounce < rounds; ++bounce) {
@@ -743,24 +753,24 @@ cudaError_t issue_wave(pt_engine* e, uint32_t rounds) {
     return cudaGetLastError();
 }
 
-cudaError_t issue_any_wave(pt_engine* e, bool alpha, uint32_t rounds) {
-    const bool wide = (e->cfg.precision & PT_PRECISION_WIDE_BVH) != 0;
-    if (alpha) return issue_wave<true, false>(e, rounds);
-    return wide ? issue_wave<false, true>(e, rounds) : issue_wave<false, false>(e, rounds);
+cudaError_t issue_any_wave(pt_engine* e, uint32_t kind, uint32_t rounds) {
+    const bool wide = (e->cfg.precision & PT_PRECISION_WIDE_BVH) != 0, plain = (kind & kWavePlain) != 0;
+    if (kind & kWaveAlpha) return plain ? issue_wave<true, false, false>(e, rounds) : issue_wave<true, false, true>(e, rounds);
+    if (wide) return issue_wave<false, true, false>(e, rounds);
+    return plain ? issue_wave<false, false, false>(e, rounds) : issue_wave<false, false, true>(e, rounds);
 }
 
 // one wave of `rounds` bounce rounds (the deepest job of the wave needs
 // max_bounces + 1; a path never takes more, so shallower waves skip the
 // launches of rounds that would find empty queues)
-int launch_wave(pt_engine* e, bool alpha, uint32_t rounds) {
-    const int gi = alpha ? 1 : 0;
+int launch_wave(pt_engine* e, uint32_t kind, uint32_t rounds) {
     if (rounds < 1 || rounds > kRounds) rounds = kRounds;
-    cudaGraphExec_t& exec = e->graph[gi][rounds - 1];
+    cudaGraphExec_t& exec = e->graph[kind][rounds - 1];
     if (e->cfg.use_graphs && !exec) {
         cudaGraph_t g = nullptr;
         int rc = e->cuda(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal), "graph capture");
         if (rc) return rc;
-        const cudaError_t le = issue_any_wave(e, alpha, rounds);
+        const cudaError_t le = issue_any_wave(e, kind, rounds);
         const cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
         if ((rc = e->cuda(le, "wave capture"))) return rc;
         if ((rc = e->cuda(ce, "graph capture"))) return rc;
@@ -774,7 +784,7 @@ int launch_wave(pt_engine* e, bool alpha, uint32_t rounds) {
     if (e->cfg.use_graphs)
         rc = e->cuda(cudaGraphLaunch(exec, e->stream), "graph launch");
     else
-        rc = e->cuda(issue_any_wave(e, alpha, rounds), "wave launch");
+        rc = e->cuda(issue_any_wave(e, kind, rounds), "wave launch");
     if (rc) return rc;
     cudaEventRecord(f.stop, e->stream);
     e->flights.push_back(f);
@@ -820,6 +830,7 @@ int start_job(pt_engine* e, Job& j) {
         }
     j.rounds = a.max_bounces + 1u;
     j.alpha = sc->any_alpha;
+    j.plain = !sc->packable;
     e->slot_items[a.slot] += count;
     j.items_target = e->slot_items[a.slot];
     e->stats.items += count;
@@ -839,10 +850,10 @@ double feed_key(const Job& j, std::chrono::steady_clock::time_point now) {
 // its pending items in tile order while they fit the wave's path budget and
 // item limit.  Writes them to the ring and the ring's tail, so the wave's
 // planner (which takes every item up to the budget) consumes exactly these.
-// Returns the number of items fed; *alpha and *rounds describe the wave.
-int feed_wave(pt_engine* e, size_t* fed, bool* alpha, uint32_t* rounds) {
+// Returns the number of items fed; *kind and *rounds describe the wave.
+int feed_wave(pt_engine* e, size_t* fed, uint32_t* kind, uint32_t* rounds) {
     *fed = 0;
-    *alpha = false;
+    *kind = 0;
     *rounds = 1;
     const auto now = std::chrono::steady_clock::now();
     std::vector<std::pair<double, Job*>> order;
@@ -862,7 +873,7 @@ int feed_wave(pt_engine* e, size_t* fed, bool* alpha, uint32_t* rounds) {
             paths += np;
             j->pending_paths -= np;
             j->pending.pop_front();
-            *alpha |= j->alpha;
+            *kind |= (j->alpha ? kWaveAlpha : 0u) | (j->plain ? kWavePlain : 0u);
             *rounds = std::max(*rounds, j->rounds);
         }
         if (paths >= budget || wave.size() >= e->max_items) break;
@@ -951,12 +962,11 @@ int harvest(pt_engine* e, bool block) {
 int pump(pt_engine* e) {
     while (e->flights.size() < PT_ENGINE_FLIGHTS) {
         size_t fed = 0;
-        bool alpha = false;
-        uint32_t rounds = 1;
-        int rc = feed_wave(e, &fed, &alpha, &rounds);
+        uint32_t kind = 0, rounds = 1;
+        int rc = feed_wave(e, &fed, &kind, &rounds);
         if (rc) return rc;
         if (fed == 0) break;
-        if ((rc = launch_wave(e, alpha, rounds))) return rc;
+        if ((rc = launch_wave(e, kind, rounds))) return rc;
     }
     return PT_OK;
 }
@@ -1023,10 +1033,10 @@ int upload_scene(pt_engine* e, Scene& s, const pt_world_updates* u) {
         lut[i] = (float)(v <= 0.04045 ? v / 12.92 : std::pow((v + 0.055) / 1.055, 2.4));
     }
     if (!rc) rc = put(s.lut, lut, sizeof lut, "sRGB table");
-    if (!rc) rc = e->cuda(s.pairs.alloc((sc->node_count + 1) * 32 + 256), "BVH layout");
-    if (!rc)
-        rc = e->cuda(cudaMemcpyAsync(static_cast<char*>(s.pairs.p) + 32, s.nodes.p, sc->node_count * 32,
-                                     cudaMemcpyDeviceToDevice, e->stream), "BVH layout");
+    if (!rc && s.packable) {
+        rc = e->cuda(s.packed.alloc(packed_bytes(sc->node_count)), "packed BVH");
+        if (!rc) rc = e->cuda(ptw::pack_bvh(s.nodes.as<pt_bvh_node>(), sc->node_count, s.packed.as<float4>(), e->stream), "packed BVH");
+    }
     if (!rc) rc = e->cuda(s.tri4.alloc(sc->triangle_count * 16 * ptd::kTriStride), "triangle layout");
     if (!rc) {
         pad_triangles_kernel<<<(unsigned)((sc->triangle_count + 255) / 256), 256, 0, e->stream>>>(
@@ -1055,7 +1065,8 @@ int upload_scene(pt_engine* e, Scene& s, const pt_world_updates* u) {
     w.any_alpha = s.any_alpha ? 1 : 0;
     w.attr16 = 1;  // a device allocation
     if (ptd::kTriStride == 4) w.tri64 = s.tri4.as<float4>();  // the shading frame's vertices
-    d.f.pairs = reinterpret_cast<const float4*>(static_cast<const char*>(s.pairs.p) + 32);
+    d.f.pairs = s.nodes.as<float4>();
+    d.f.packed = s.packed.p ? s.packed.as<float4>() : nullptr;
     d.f.tri4 = s.tri4.as<float4>();
     d.f.wide = s.wide.p ? s.wide.as<float4>() : nullptr;
     d.f.parent = s.links.p ? s.links.as<uint32_t>() : nullptr;
@@ -1244,6 +1255,8 @@ int pte_scene_add(pt_engine* e, const pt_world_updates* u, uint64_t* scene_id) t
     for (uint64_t i = 0; i < sc->triangle_count; ++i)
         if (sc->attributes[i].material_index >= sc->material_count)
             return e->fail(PT_ERR_INVALID_ARG, "triangle material index outside the material buffer");
+    uint64_t tree_nodes = 0;
+    uint32_t max_leaf = 0;
     {
         std::vector<uint8_t> seen(sc->node_count, 0);
         std::vector<std::pair<uint64_t, uint32_t>> st{{0, 0}};
@@ -1252,8 +1265,10 @@ int pte_scene_add(pt_engine* e, const pt_world_updates* u, uint64_t* scene_id) t
             st.pop_back();
             if (seen[i]) return e->fail(PT_ERR_INVALID_ARG, "BVH node reached twice (not a tree)");
             seen[i] = 1;
+            tree_nodes += 1;
             const pt_bvh_node& n = sc->bvh_nodes[i];
             if (n.tri_count > 0) {
+                max_leaf = std::max(max_leaf, n.tri_count);
                 if ((uint64_t)n.left_first + n.tri_count > sc->triangle_count)
                     return e->fail(PT_ERR_INVALID_ARG, "BVH leaf triangle range outside the triangle buffer");
             } else {
@@ -1317,7 +1332,7 @@ int pte_scene_add(pt_engine* e, const pt_world_updates* u, uint64_t* scene_id) t
                      (sc->srgb_atlas_count + sc->linear_atlas_count) * layer + sk->alias_count * 12 +
                      u->scene_alias_count * 16 + 1024;
     bytes += form.half ? sc->triangle_count * 64 + texels * 8 : sc->triangle_count * 112 + texels * 16;
-    bytes += sc->node_count * 64 + 256;             // binary nodes + child-pair copy
+    bytes += sc->node_count * 32 + packed_bytes(sc->node_count);  // binary nodes + their packed form
     bytes += form.wide ? sc->node_count * (64 + 4) + sc->triangle_count * 4 : 0;  // wide nodes (at most one per
                                                                                    // two binary nodes) + links
     while (e->used + bytes > e->budget && evict_one(e)) {
@@ -1345,6 +1360,7 @@ int pte_scene_add(pt_engine* e, const pt_world_updates* u, uint64_t* scene_id) t
     s->caller_refs = 1;
     s->last_use = e->use_clock;
     s->any_alpha = any_alpha;
+    s->packable = ptw::packable(sc->node_count, tree_nodes, sc->triangle_count, max_leaf);
     int rc = upload_scene(e, *s, u);
     if (rc) return rc;
     e->scene_slots[slot] = h;

@@ -70,6 +70,7 @@ struct pt_ctx {
     pt_scene_uniforms scene{};
     pt_skybox_uniforms sky_u{};
     std::vector<uint32_t> alpha_modes;
+    bool packable = false;  // the BVH fits the wavefront kernels' packed form
     bool world_ready = false;
 
     // tile (bind group 0)
@@ -183,8 +184,11 @@ int copy_to(pt_ctx* c, DevBuf& buf, const void* src, size_t bytes, const char* w
 // the BVH must be a tree reachable from node 0 whose traversal never needs
 // more than 64 deferred entries (trace.slang:632,786).  Returns PT_OK or an
 // error code with *msg set; touches no context, so it may run on a helper
-// thread.
-int check_bvh(const pt_bvh_node* nodes, uint64_t count, uint64_t tris, const char** msg) {
+// thread.  *reached_nodes: the nodes of the tree; *max_leaf: its largest leaf.
+int check_bvh(const pt_bvh_node* nodes, uint64_t count, uint64_t tris, const char** msg, uint64_t* reached_nodes,
+              uint32_t* max_leaf) {
+    uint64_t in_tree = 0;
+    uint32_t largest = 0;
     if (count == 0) {
         *msg = "BVH has no nodes";
         return PT_ERR_INVALID_ARG;
@@ -200,8 +204,10 @@ int check_bvh(const pt_bvh_node* nodes, uint64_t count, uint64_t tris, const cha
         for (uint64_t i = 0; i < count && ordered; ++i) {
             const uint8_t r = reached[i];
             if (r == 0) continue;  // unreachable from the root: ignored, as by the traversal
+            in_tree += 1;
             const pt_bvh_node& n = nodes[i];
             if (n.tri_count > 0) {
+                largest = n.tri_count > largest ? n.tri_count : largest;
                 if ((uint64_t)n.left_first + n.tri_count > tris) {
                     *msg = "BVH leaf triangle range outside the triangle buffer";
                     return PT_ERR_INVALID_ARG;
@@ -223,8 +229,14 @@ int check_bvh(const pt_bvh_node* nodes, uint64_t count, uint64_t tris, const cha
             }
             reached[l] = reached[l + 1] = (uint8_t)(r + 1);
         }
-        if (ordered) return PT_OK;
+        if (ordered) {
+            *reached_nodes = in_tree;
+            *max_leaf = largest;
+            return PT_OK;
+        }
     }
+    in_tree = 0;
+    largest = 0;
     std::vector<uint8_t> seen(count, 0);
     std::vector<std::pair<uint64_t, uint32_t>> st{{0, 0}};
     while (!st.empty()) {
@@ -235,8 +247,10 @@ int check_bvh(const pt_bvh_node* nodes, uint64_t count, uint64_t tris, const cha
             return PT_ERR_INVALID_ARG;
         }
         seen[i] = 1;
+        in_tree += 1;
         const pt_bvh_node& n = nodes[i];
         if (n.tri_count > 0) {
+            largest = n.tri_count > largest ? n.tri_count : largest;
             if ((uint64_t)n.left_first + n.tri_count > tris) {
                 *msg = "BVH leaf triangle range outside the triangle buffer";
                 return PT_ERR_INVALID_ARG;
@@ -254,6 +268,8 @@ int check_bvh(const pt_bvh_node* nodes, uint64_t count, uint64_t tris, const cha
             st.push_back({(uint64_t)n.left_first + 1, depth + 1});
         }
     }
+    *reached_nodes = in_tree;
+    *max_leaf = largest;
     return PT_OK;
 }
 
@@ -350,6 +366,8 @@ int apply(pt_ctx* c, const pt_world_updates* u, bool initial) {
     pt_skybox_uniforms sky = u->skybox_uniforms ? *u->skybox_uniforms : c->sky_u;
     uint64_t sky_alias_count = c->sky_alias_count;
     uint64_t live = u->scene ? 0 : c->scene_alias_live;
+    uint64_t tree_nodes = 0;  // of the uploaded BVH
+    uint32_t max_leaf = 0;
     bool sky_checked = false, sky_aliases_ok = true;  // the skybox alias scan, when it ran beside the BVH walk
     const auto validate = [&]() -> int {
         if (const pt_scene_upload* s = u->scene) {
@@ -368,7 +386,7 @@ int apply(pt_ctx* c, const pt_world_updates* u, bool initial) {
             int bvh_rc = PT_OK;
             bool sky_ok = true;
             const auto helper = [&] {
-                bvh_rc = check_bvh(s->bvh_nodes, s->node_count, s->triangle_count, &bvh_msg);
+                bvh_rc = check_bvh(s->bvh_nodes, s->node_count, s->triangle_count, &bvh_msg, &tree_nodes, &max_leaf);
                 if (scan_sky) sky_ok = sky_aliases_in_range(k->alias_table, k->alias_count);
             };
             std::thread worker;
@@ -442,7 +460,8 @@ int apply(pt_ctx* c, const pt_world_updates* u, bool initial) {
         c->alpha_modes.resize(s->material_count);
         for (uint64_t i = 0; i < s->material_count; ++i) c->alpha_modes[i] = s->materials[i].alpha_mode;
         c->scene_alias_live = 0;
-        if (c->wavefront) ptw::world_changed(c->wavefront);
+        c->packable = ptw::packable(s->node_count, tree_nodes, s->triangle_count, max_leaf);
+        if (c->wavefront) ptw::world_changed(c->wavefront, c->packable);
     }
     if (const pt_skybox_upload* k = u->skybox) {
         const size_t px = (size_t)k->uniforms.width * k->uniforms.height;
@@ -549,6 +568,7 @@ int trace_impl(pt_ctx* c, uint32_t samples, uint32_t* traced, pt_path_record* ho
         if (!c->wavefront) {
             const int ce = ptw::create(&c->wavefront);
             if (ce) return c->cuda((cudaError_t)ce, "wavefront streams");
+            ptw::world_changed(c->wavefront, c->packable);
         }
         const bool record = rec != nullptr || tot != nullptr;
         const uint32_t form = ptw::effective_precision(w, c->precision, record);
@@ -874,7 +894,10 @@ int pt_debug_intersect(pt_ctx* c, uint64_t n, const float* origins, const float*
     const ptd::World w = c->view();
     const bool wide = (ptw::effective_precision(w, c->precision, records != nullptr) & PT_PRECISION_WIDE_BVH) != 0;
     if (!rc && wide) {
-        if (!c->wavefront) rc = c->cuda((cudaError_t)ptw::create(&c->wavefront), "wavefront streams");
+        if (!c->wavefront) {
+            rc = c->cuda((cudaError_t)ptw::create(&c->wavefront), "wavefront streams");
+            if (!rc) ptw::world_changed(c->wavefront, c->packable);
+        }
         if (!rc) rc = c->cuda(ptw::prepare(c->wavefront, w, c->node_count, c->tri_count, PT_PRECISION_WIDE_BVH, c->stream),
                      "wide BVH");
     }

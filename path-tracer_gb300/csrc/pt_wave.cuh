@@ -11,7 +11,8 @@
 namespace ptd {
 
 struct Fast {
-    const float4* pairs;  // node i at pairs[2i], pairs[2i+1]
+    const float4* pairs;  // the binary nodes: node i at pairs[2i], pairs[2i+1] (32-byte aligned)
+    const float4* packed = nullptr;  // the packed BVH (see PackedRay); null: the scene has none
     const float4* tri4;   // triangle i at tri4[kTriStride i .. kTriStride i + 2] (padded to 48 or 64 bytes)
     const float4* wide = nullptr;  // pt_wide_node i at wide[8i .. 8i+7] (precision form)
     const uint32_t* parent = nullptr;   // binary node -> its parent (root: 0xffffffff)
@@ -130,6 +131,11 @@ constexpr int kShadeThreads = PT_SHADE_THREADS;
 #define PT_SMEM_STACK 8
 #endif
 constexpr uint32_t kSmemStack = PT_SMEM_STACK;
+// the same for the packed traversal (16 bytes an entry)
+#ifndef PT_PACKED_SMEM_STACK
+#define PT_PACKED_SMEM_STACK 8
+#endif
+constexpr uint32_t kPackedSmemStack = PT_PACKED_SMEM_STACK;
 // the same for the 8-wide traversal kernels
 #ifndef PT_WIDE_SMEM_STACK
 #define PT_WIDE_SMEM_STACK 8
@@ -144,13 +150,13 @@ struct LaneStack {
     uint2* col;  // &shared[threadIdx.x]; entry i < kShared at col[i * kThreads]
     uint2 deep[64];
     PTD void put(uint32_t i, uint2 e) {
-        if (kShared > 0u && i < kShared)
+        if (i < kShared)
             col[i * kThreads] = e;
         else
             deep[i & 63u] = e;
     }
     PTD uint2 get(uint32_t i) const {
-        if (kShared > 0u && i < kShared) return col[i * kThreads];
+        if (i < kShared) return col[i * kThreads];
         return deep[i & 63u];
     }
 };
@@ -200,18 +206,20 @@ struct OneScene {
     const Fast& fast;
     PTD const World& w() const { return world; }
     PTD const Fast& f() const { return fast; }
-    PTD const float4* nodes() const { return fast.pairs; }
+    PTD const float4* packed() const { return fast.packed; }
     PTD const float4* wide() const { return fast.wide; }
     PTD const float4* tri4() const { return fast.tri4; }
 };
-// ... or each lane its own, its two hot pointers kept in registers
+// ... or each lane its own: a table of Record { World w; Fast f; } and the
+// lane's index in it, its two hot pointers kept in registers
+template <class Record>
 struct LaneScene {
-    const World* world;
-    const Fast* fast;
+    const Record* table;
+    uint32_t index;
     const float4 *boxes, *tris;
-    PTD const World& w() const { return *world; }
-    PTD const Fast& f() const { return *fast; }
-    PTD const float4* nodes() const { return boxes; }
+    PTD const World& w() const { return table[index].w; }
+    PTD const Fast& f() const { return table[index].f; }
+    PTD const float4* packed() const { return boxes; }
     PTD const float4* wide() const { return boxes; }
     PTD const float4* tri4() const { return tris; }
 };
@@ -224,10 +232,14 @@ struct LaneScene {
 #define PT_VISIT_KEEP 16
 #endif
 #ifndef PT_TEST_LEAVE
-#define PT_TEST_LEAVE 2
+#define PT_TEST_LEAVE 4
 #endif
 #ifndef PT_REFILL_AT
 #define PT_REFILL_AT 20
+#endif
+// two visits between two looks at the warp's lanes: 10.84 against 11.03 ms a 960x540x16 image of 1M triangles
+#ifndef PT_VISIT_TWICE
+#define PT_VISIT_TWICE 1
 #endif
 #ifndef PT_WIDE_VISIT_KEEP
 #define PT_WIDE_VISIT_KEEP 16
@@ -239,7 +251,7 @@ struct LaneScene {
 #define PT_WIDE_REFILL_AT 20
 #endif
 
-// What a traversal lane does next, in `todo`: 0 visit an interior node, > 0
+// What a lane of the two-word traversals does next, in `todo`: 0 visit an interior node, > 0
 // test that many triangles of a leaf, kFinished: the ray's result is there
 // and not filed yet, kIdle: no ray.
 constexpr int32_t kFinished = -2, kIdle = -1;
@@ -249,8 +261,22 @@ constexpr int32_t kFinished = -2, kIdle = -1;
 PTD float below(float t) { return t > 0.0f ? __uint_as_float(__float_as_uint(t) - 1u) : -1.0f; }
 PTD float above(float t) { return __uint_as_float(__float_as_uint(t) + 1u); }
 
+// A box's entry distance, at least 2^-149, and exit distance, at most `limit`
+// (see BinaryRay): the box is accepted when *t_near <= *t_far.
+PTD void slabs(float4 lo, float4 hi, f3 rcp, f3 nod, float limit, float* t_near, float* t_far) {
+    const float t0x = fma_(lo.x, rcp.x, nod.x), t0y = fma_(lo.y, rcp.y, nod.y), t0z = fma_(lo.z, rcp.z, nod.z);
+    const float t1x = fma_(hi.x, rcp.x, nod.x), t1y = fma_(hi.y, rcp.y, nod.y), t1z = fma_(hi.z, rcp.z, nod.z);
+    *t_near = max3f(fmaxf(fminf(t0x, t1x), 0x1p-149f), fminf(t0y, t1y), fminf(t0z, t1z));
+    *t_far = min3f(fminf(fmaxf(t0x, t1x), limit), fmaxf(t0y, t1y), fmaxf(t0z, t1z));
+}
+// no axis of the ray gives a slab distance that is a number (see BinaryRay)
+PTD bool boxless(f3 nod) {
+    const float inf = __int_as_float(0x7f800000);
+    return !(fabsf(nod.x) < inf) && !(fabsf(nod.y) < inf) && !(fabsf(nod.z) < inf);
+}
+
 // One ray's traversal (trace.slang:764-884 closest hit, or 614-717 any hit
-// when kShadow) on the aligned child-pair layout: visit() one interior node,
+// when kShadow) on the binary nodes as uploaded: visit() one interior node,
 // test() one triangle of a leaf; traverse_queue() decides when each runs.
 // The deferred stack holds the (left_first, tri_count) of each node, so a pop
 // needs no memory access.  A ray's visits and tests happen in exactly the
@@ -278,22 +304,26 @@ struct BinaryRay {
     Rec<kRec> rec;
 
     PTD explicit BinaryRay(Scene scene) : sc(scene), todo(kIdle) {}
+    PTD bool busy() const { return todo >= 0; }
+    PTD bool at_node() const { return todo == 0; }
+    PTD bool at_leaf() const { return todo > 0; }
+    PTD bool finished() const { return todo == kFinished; }
+    PTD void set_idle() { todo = kIdle; }
 
-    PTD void init(f3 origin, f3 dir, float t_max, int32_t light) {
+    template <class S>
+    PTD void init(f3 origin, f3 dir, float t_max, int32_t light, S&) {
         o = origin;
         rcp = 1.0f / dir;
         s = make_shear(dir, rcp);
         nod = -o * rcp;
-        const float inf = __int_as_float(0x7f800000);
-        const bool boxless = !(fabsf(nod.x) < inf) && !(fabsf(nod.y) < inf) && !(fabsf(nod.z) < inf);
-        limit = boxless ? -1.0f : below(t_max);
+        limit = boxless(nod) ? -1.0f : below(t_max);
         hv = hw = 0.0f;
         hit = -1;
         light_tri = light;
         sp = 0u;
         idx = 0u;
-        lf = __float_as_uint(__ldg(&sc.nodes()[0].w));
-        todo = __float_as_int(__ldg(&sc.nodes()[1].w));
+        lf = __float_as_uint(__ldg(&sc.f().pairs[0].w));
+        todo = __float_as_int(__ldg(&sc.f().pairs[1].w));
         if constexpr (kRec) {
             rec.c = &c;
             rng.rec.c = &c;
@@ -333,22 +363,15 @@ struct BinaryRay {
         }
     }
 
-    PTD void slabs(float4 lo, float4 hi, float* t_near, float* t_far) const {
-        const float t0x = fma_(lo.x, rcp.x, nod.x), t0y = fma_(lo.y, rcp.y, nod.y), t0z = fma_(lo.z, rcp.z, nod.z);
-        const float t1x = fma_(hi.x, rcp.x, nod.x), t1y = fma_(hi.y, rcp.y, nod.y), t1z = fma_(hi.z, rcp.z, nod.z);
-        *t_near = max3f(fmaxf(fminf(t0x, t1x), 0x1p-149f), fminf(t0y, t1y), fminf(t0z, t1z));
-        *t_far = min3f(fminf(fmaxf(t0x, t1x), limit), fmaxf(t0y, t1y), fmaxf(t0z, t1z));
-    }
-
     template <class S>
     PTD void visit(S& stack, uint32_t* istack) {
-        const float4* p = sc.nodes() + 2 * (size_t)lf;
+        const float4* p = sc.f().pairs + 2 * (size_t)lf;
         float4 l0, l1, r0, r1;
         load_node(p, l0, l1);
         load_node(p + 2, r0, r1);
         float ln, lx, rn, rx;
-        slabs(l0, l1, &ln, &lx);
-        slabs(r0, r1, &rn, &rx);
+        slabs(l0, l1, rcp, nod, limit, &ln, &lx);
+        slabs(r0, r1, rcp, nod, limit, &rn, &rx);
         const bool hl = ln <= lx, hr = rn <= rx;
         if (!hl && !hr) {
             pop(stack, istack);
@@ -399,6 +422,308 @@ struct BinaryRay {
             }
         }
         if (todo == 0) pop(stack, istack);
+    }
+};
+
+// ---------------------------------------------------------------- packed BVH
+//
+// A pair of child boxes in 32 bytes, one load a visit.  The two children of an
+// interior node share its planes: on each side of each axis one child (at
+// least) has the parent's plane, so the pair needs six new planes and six bits
+// that say whose they are.  In a ray's terms a shared plane adds nothing: the
+// children's entry distance is the largest of the parent's entry distance and
+// those of their own new near planes, and likewise the exit, so the traversal
+// carries the node's two distances instead of its box.  The distances are
+// those of the uploaded boxes bit for bit (fma is monotonic in the plane, so
+// the largest over the three axes does not change when an axis is replaced by
+// the parent's smaller or equal value).
+//
+// Record of the interior node whose children are l and l + 1, at l / 2 (a
+// child pair has one parent): three new minima and the left child's
+// reference, three new maxima and the right child's reference.  Reference:
+// index << 7 | count << 3 | owners; count 0: an interior node, index = its
+// record; 1..14: a leaf, index = its first triangle; 15: an interior node
+// whose record holds no planes, only l in its first word (boxes that are not
+// exactly the union of their children's, planes out of order or not finite,
+// even l), visited from the uploaded nodes.  owners, bit a: in the left
+// reference, the new minimum of axis a is the right child's (else the left
+// child's); in the right reference the same of the new maximum.
+// Entry 0 of the array is the root's box and reference; the records follow.
+constexpr uint32_t kPackedMaxLeaf = 14, kPackedPlain = 15;
+constexpr uint64_t kPackedMaxNodes = 1ull << 26, kPackedMaxTris = 1ull << 25;  // exclusive: all ones is no index
+constexpr uint32_t kRefIdle = 0xffffffffu, kRefFinished = 0xfffffffeu;
+
+PTD bool finite3(float4 v) {
+    const float inf = __int_as_float(0x7f800000);
+    return fabsf(v.x) < inf && fabsf(v.y) < inf && fabsf(v.z) < inf;
+}
+
+// node i's children as six new planes and their owners (false: kPackedPlain)
+PTD bool pack_planes(const float4* nodes, uint64_t node_count, uint64_t i, float* plane_lo, float* plane_hi,
+                     uint32_t* own_lo, uint32_t* own_hi) {
+    const float4 p0 = nodes[2 * i], p1 = nodes[2 * i + 1];
+    const uint64_t l = __float_as_uint(p0.w);
+    if ((l & 1u) == 0u || l + 1u >= node_count) return false;
+    const float4 l0 = nodes[2 * l], l1 = nodes[2 * l + 1], r0 = nodes[2 * l + 2], r1 = nodes[2 * l + 3];
+    if (!finite3(l0) || !finite3(l1) || !finite3(r0) || !finite3(r1)) return false;
+    const float plo[3] = {p0.x, p0.y, p0.z}, phi[3] = {p1.x, p1.y, p1.z};
+    const float llo[3] = {l0.x, l0.y, l0.z}, lhi[3] = {l1.x, l1.y, l1.z};
+    const float rlo[3] = {r0.x, r0.y, r0.z}, rhi[3] = {r1.x, r1.y, r1.z};
+    *own_lo = *own_hi = 0u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (!(llo[a] <= lhi[a]) || !(rlo[a] <= rhi[a])) return false;
+        if (plo[a] != fminf(llo[a], rlo[a]) || phi[a] != fmaxf(lhi[a], rhi[a])) return false;
+        const bool lo_right = llo[a] == plo[a], hi_right = lhi[a] == phi[a];
+        plane_lo[a] = lo_right ? rlo[a] : llo[a];
+        plane_hi[a] = hi_right ? rhi[a] : lhi[a];
+        *own_lo |= (lo_right ? 1u : 0u) << a;
+        *own_hi |= (hi_right ? 1u : 0u) << a;
+    }
+    return true;
+}
+
+// reference to node i
+PTD uint32_t pack_ref(const float4* nodes, uint64_t node_count, uint64_t i) {
+    const uint32_t first = __float_as_uint(nodes[2 * i].w), count = __float_as_uint(nodes[2 * i + 1].w);
+    if (count > 0u) return (first << 7) | (count << 3);
+    float lo[3], hi[3];
+    uint32_t a, b;
+    return ((first >> 1) << 7) | (pack_planes(nodes, node_count, i, lo, hi, &a, &b) ? 0u : kPackedPlain << 3);
+}
+
+// One thread per node of a tree in which every node is reachable, with at most
+// kPackedMaxLeaf triangles a leaf.  (A template, so that both translation
+// units may include it.)
+template <int kUnused>
+__global__ void __launch_bounds__(256) pack_bvh_kernel(const float4* nodes, uint64_t node_count, float4* packed) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= node_count) return;
+    if (i == 0u) {
+        const float4 a = nodes[0], b = nodes[1];
+        packed[0] = make_float4(a.x, a.y, a.z, __uint_as_float(pack_ref(nodes, node_count, 0u)));
+        packed[1] = make_float4(b.x, b.y, b.z, 0.0f);
+    }
+    if (__float_as_uint(nodes[2 * i + 1].w) > 0u) return;
+    const uint32_t l = __float_as_uint(nodes[2 * i].w);
+    if ((uint64_t)l + 1u >= node_count) return;
+    float lo[3] = {__uint_as_float(l), 0.0f, 0.0f}, hi[3] = {0.0f, 0.0f, 0.0f};
+    uint32_t own_lo = 0u, own_hi = 0u;
+    if (!pack_planes(nodes, node_count, i, lo, hi, &own_lo, &own_hi)) {
+        lo[0] = __uint_as_float(l);
+        own_lo = own_hi = 0u;
+    }
+    float4* r = packed + 2 + 2 * (size_t)(l >> 1);
+    r[0] = make_float4(lo[0], lo[1], lo[2], __uint_as_float(pack_ref(nodes, node_count, l) | own_lo));
+    r[1] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(pack_ref(nodes, node_count, l + 1u) | own_hi));
+}
+
+// bytes of the packed BVH of a tree
+constexpr size_t packed_bytes(uint64_t nodes) { return 32 + 32 * (nodes / 2 + 1); }
+
+// v into the left child's distance, or the right child's where `right` is not 0
+PTD void route_max(uint32_t right, float v, float& l, float& r) {
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@!p max.f32 %0, %0, %2;\n\t@p max.f32 %1, %1, %2;\n\t}"
+        : "+f"(l), "+f"(r)
+        : "f"(v), "r"(right));
+}
+PTD void route_min(uint32_t right, float v, float& l, float& r) {
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@!p min.f32 %0, %0, %2;\n\t@p min.f32 %1, %1, %2;\n\t}"
+        : "+f"(l), "+f"(r)
+        : "f"(v), "r"(right));
+}
+
+// The deferred stack of a packed traversal, 16 bytes an entry (reference,
+// entry distance, exit distance): the first kShared entries in shared memory,
+// the others in the lane's local memory.  Entry 0 is the end: a popped
+// kRefFinished ends the traversal.  Positions are byte offsets in local
+// memory (16 an entry).  Everything a visit does with the stack is predicated
+// instructions, so that a warp whose lanes push, pop and do neither runs no
+// branch for it.
+template <uint32_t kThreads, uint32_t kShared>
+struct PackedStack {
+    static constexpr uint32_t kLast = 16u * (kShared - 1u);  // position of the last shared entry
+    uint32_t col;   // shared address of this thread's entry 0; entry i at + i * kThreads * 16
+    uint32_t deep;  // local address of entry 0
+    float4 entries[66];  // at most 64 deferred nodes (checked at upload) above entry 0
+    PTD void bind(const float4* top) {
+        // (opaque to the compiler, which otherwise computes the addresses again on every visit)
+        asm volatile("mov.u32 %0, %1;" : "=r"(col) : "r"((uint32_t)__cvta_generic_to_shared(top + threadIdx.x)));
+        asm volatile("{\n\t.reg .u64 a;\n\tcvta.to.local.u64 a, %1;\n\tcvt.u32.u64 %0, a;\n\t}" : "=r"(deep) : "l"(entries) : "memory");
+    }
+    PTD void clear() const {
+        asm volatile("st.shared.b32 [%0], %1;" ::"r"(col), "r"(kRefFinished) : "memory");
+    }
+    PTD void pop(uint32_t& sp, uint32_t& ref, float& t_near, float& t_far) const {
+        asm volatile(
+            "{\n\t.reg .pred s;\n\t.reg .b32 z;\n\tsetp.le.u32 s, %0, %4;\n\t"
+            "@s ld.shared.v4.b32 {%1, %2, %3, z}, [%5];\n\t@!s ld.local.v4.b32 {%1, %2, %3, z}, [%6];\n\t"
+            "sub.u32 %0, %0, 16;\n\t}"
+            : "+r"(sp), "+r"(ref), "+f"(t_near), "+f"(t_far)
+            : "n"(kLast), "r"(col + sp * kThreads), "r"(deep + sp)
+            : "memory");
+    }
+    // the end of a visit: on to the nearer accepted child, deferring the other,
+    // or to the deferred node at the stack's top
+    PTD void descend(uint32_t& sp, uint32_t& ref, float& t_near, float& t_far, uint32_t wl, uint32_t wr, float ln,
+                     float lx, float rn, float rx) const {
+        asm volatile(
+            "{\n\t.reg .pred hl, hr, lt, nr, left, both, any, s, p;\n\t.reg .b32 f0, f1, f2, z;\n\t"
+            "setp.le.f32 hl, %6, %7;\n\tsetp.le.f32 hr, %8, %9;\n\tsetp.lt.f32 lt, %6, %8;\n\t"
+            "not.pred nr, hr;\n\tor.pred left, nr, lt;\n\tand.pred left, left, hl;\n\t"
+            "and.pred both, hl, hr;\n\tor.pred any, hl, hr;\n\t"
+            "selp.b32 f0, %5, %4, left;\n\tselp.b32 f1, %8, %6, left;\n\tselp.b32 f2, %9, %7, left;\n\t"
+            "setp.lt.and.u32 p, %0, %10, both;\n\t@p st.shared.v4.b32 [%11 + %13], {f0, f1, f2, f0};\n\t"
+            "setp.ge.and.u32 p, %0, %10, both;\n\t@p st.local.v4.b32 [%12 + 16], {f0, f1, f2, f0};\n\t"
+            "not.pred nr, any;\n\t"
+            "setp.le.and.u32 s, %0, %10, nr;\n\t@s ld.shared.v4.b32 {%1, %2, %3, z}, [%11];\n\t"
+            "setp.gt.and.u32 s, %0, %10, nr;\n\t@s ld.local.v4.b32 {%1, %2, %3, z}, [%12];\n\t"
+            "@any selp.b32 %1, %4, %5, left;\n\t@any selp.b32 %2, %6, %8, left;\n\t@any selp.b32 %3, %7, %9, left;\n\t"
+            "@both add.u32 %0, %0, 16;\n\t@nr sub.u32 %0, %0, 16;\n\t}"
+            : "+r"(sp), "+r"(ref), "+f"(t_near), "+f"(t_far)
+            : "r"(wl), "r"(wr), "f"(ln), "f"(lx), "f"(rn), "f"(rx), "n"(kLast), "r"(col + sp * kThreads),
+              "r"(deep + sp), "n"(kThreads * 16u)
+            : "memory");
+    }
+};
+
+// The traversal of BinaryRay on the packed BVH: the same visits and tests in
+// the same order.  What it is worth: the uploaded nodes cost two 32-byte loads
+// a visit, and a load of 32 scattered lanes is 32 wavefronts of the L1 data
+// pipe, which was 79 % busy; here it is 62 %, and the kernel is bound by
+// instructions (73 % of the issue slots, ALU pipe 60 %).  The extend launch of
+// bounce 1 (1M triangles, 960x540x8): 1.08 ms at first, 1.01 with turns of
+// visits and tests, 0.87 packed.  2.1M triangles, 1920x1080x16: extend 31.2 ->
+// 25.2 ms, the image 55.2 -> 47.9 ms.  At 56 registers 9 blocks of 128 are
+// resident with 8 stack entries in shared memory (16 KB a block); 8 blocks
+// with 64 registers: 11.3 against 10.8 ms for a 960x540x16 image of 1M
+// triangles, 6 entries: 11.3.  A visit has no branch.  The selection of the near
+// and far plane by the ray's direction is done by the multiplier: rp holds the
+// positive reciprocals, rn the negative ones, 0 elsewhere, and
+// fma(a, rp, fma(b, rn, nod)) is the distance of a or b, with one rounding
+// (the other product is an exact 0), which spares the ALU pipe, the busiest
+// one (half rate), a select.
+template <bool kAlpha, bool kShadow, class Scene>
+struct PackedRay {
+    static constexpr int kVisitKeep = PT_VISIT_KEEP, kTestLeave = PT_TEST_LEAVE, kRefillAt = PT_REFILL_AT;
+    Scene sc;
+    f3 o, rp, rn, nod;
+    float limit, hv, hw, tn, tf;  // limit: below(hit_t); tn, tf: the node's entry and exit distances
+    int32_t hit, light_tri;
+    uint32_t ref, sp;  // sp: position of the stack's top entry
+    uint32_t oct;      // bit a: rcp[a] < 0; bits 3..6: visits read the uploaded nodes
+    uint32_t axes;     // kx, ky, kz of the shear, two bits each
+    float sx, sy, sz;
+    Rng<false> rng;
+
+    PTD explicit PackedRay(Scene scene) : sc(scene), ref(kRefIdle) {}
+    PTD bool busy() const { return ref < kRefFinished; }
+    PTD bool at_node() const { return ((ref | oct) & 0x78u) == 0u; }
+    PTD bool at_leaf() const { return ((ref | oct) & 0x78u) != 0u && ref < kRefFinished; }
+    PTD bool finished() const { return ref == kRefFinished; }
+    PTD void set_idle() { ref = kRefIdle; }
+    PTD float hit_t() const { return above(limit); }
+
+    template <class S>
+    PTD void init(f3 origin, f3 dir, float t_max, int32_t light, S& stack) {
+        o = origin;
+        const f3 rcp = 1.0f / dir;
+        const Shear s = make_shear(dir, rcp);
+        axes = (uint32_t)s.kx | ((uint32_t)s.ky << 2) | ((uint32_t)s.kz << 4);
+        sx = s.sx;
+        sy = s.sy;
+        sz = s.sz;
+        nod = -o * rcp;
+        rp = mk(rcp.x < 0.0f ? 0.0f : rcp.x, rcp.y < 0.0f ? 0.0f : rcp.y, rcp.z < 0.0f ? 0.0f : rcp.z);
+        rn = mk(rcp.x < 0.0f ? rcp.x : 0.0f, rcp.y < 0.0f ? rcp.y : 0.0f, rcp.z < 0.0f ? rcp.z : 0.0f);
+        oct = (rcp.x < 0.0f ? 1u : 0u) | (rcp.y < 0.0f ? 2u : 0u) | (rcp.z < 0.0f ? 4u : 0u);
+        limit = boxless(nod) ? -1.0f : below(t_max);
+        hv = hw = 0.0f;
+        hit = -1;
+        light_tri = light;
+        stack.clear();
+        sp = 0u;
+        float4 a, b;
+        load_node(sc.packed(), a, b);
+        ref = __float_as_uint(a.w);
+        slabs(a, b, rcp, nod, __int_as_float(0x7f800000), &tn, &tf);
+        // an axis without a finite reciprocal (a zero direction component) has no
+        // distances that could be carried: such a ray visits the uploaded nodes
+        const float inf = __int_as_float(0x7f800000);
+        if (!(fabsf(nod.x) < inf && fabsf(nod.y) < inf && fabsf(nod.z) < inf)) oct |= 0x78u;
+    }
+
+    template <class S>
+    PTD void visit(S& stack, uint32_t*) {
+        float4 a, b;
+        load_node(sc.packed() + 2 + 2 * (size_t)(ref >> 7), a, b);
+        const uint32_t wl = __float_as_uint(a.w), wr = __float_as_uint(b.w);
+        // owners of the near and of the far planes
+        const uint32_t near_own = (wl & ~oct) | (wr & oct), far_own = (wr & ~oct) | (wl & oct);
+        float ln = tn, rn_ = tn, lx = fminf(tf, limit), rx = lx;
+        route_max(near_own & 1u, fma_(a.x, rp.x, fma_(b.x, rn.x, nod.x)), ln, rn_);
+        route_max(near_own & 2u, fma_(a.y, rp.y, fma_(b.y, rn.y, nod.y)), ln, rn_);
+        route_max(near_own & 4u, fma_(a.z, rp.z, fma_(b.z, rn.z, nod.z)), ln, rn_);
+        route_min(far_own & 1u, fma_(b.x, rp.x, fma_(a.x, rn.x, nod.x)), lx, rx);
+        route_min(far_own & 2u, fma_(b.y, rp.y, fma_(a.y, rn.y, nod.y)), lx, rx);
+        route_min(far_own & 4u, fma_(b.z, rp.z, fma_(a.z, rn.z, nod.z)), lx, rx);
+        stack.descend(sp, ref, tn, tf, wl, wr, ln, lx, rn_, rx);
+    }
+
+    // a visit from the uploaded boxes of the two children
+    template <class S>
+    PTD void visit_plain(S& stack) {
+        const float4* r = sc.packed() + 2 + 2 * (size_t)(ref >> 7);
+        uint32_t l = 2u * (ref >> 7) + 1u;
+        if ((ref & 0x78u) != 0u) l = __float_as_uint(__ldg(&r[0].x));
+        const uint32_t wl = __float_as_uint(__ldg(&r[0].w)), wr = __float_as_uint(__ldg(&r[1].w));
+        const float4* p = sc.f().pairs + 2 * (size_t)l;
+        float4 l0, l1, r0, r1;
+        load_node(p, l0, l1);
+        load_node(p + 2, r0, r1);
+        const f3 rcp = rp + rn;
+        float ln, lx, rn_, rx;
+        slabs(l0, l1, rcp, nod, limit, &ln, &lx);
+        slabs(r0, r1, rcp, nod, limit, &rn_, &rx);
+        stack.descend(sp, ref, tn, tf, wl, wr, ln, lx, rn_, rx);
+    }
+
+    // One triangle of the leaf, or a plain visit.  A ray whose every visit is
+    // plain runs to its end here: such a ray (an axis-parallel one) can meet
+    // thousands of boxes, because its zero axis rejects none, and would hold up
+    // the launch's end if each visit waited for a turn of the warp (2.1M
+    // triangles, 1344x756x16, camera rays: extend 14.0 ms in turns).
+    template <class S>
+    PTD void test(S& stack, uint32_t*) {
+        do {
+            const uint32_t count = (ref >> 3) & 15u;
+            if (count == 0u || count == kPackedPlain) {
+                visit_plain(stack);
+                continue;
+            }
+            const uint32_t tri = ref >> 7;
+            ref += (1u << 7) - (1u << 3);  // the next triangle, one fewer left
+            const Shear s{(int)(axes & 3u), (int)((axes >> 2) & 3u), (int)(axes >> 4), sx, sy, sz};
+            float t, v, wb;
+            if (!(kShadow && (int32_t)tri == light_tri) &&
+                triangle_test(load_tri4(sc.tri4(), tri), o, s, &t, &v, &wb) && t > 0.0f && t <= limit) {
+                bool counts = true;
+                if constexpr (kAlpha) counts = !passes_through(sc.w(), tri, v, wb, rng);
+                if (counts) {
+                    if constexpr (kShadow) {
+                        hit = 1;
+                        ref = kRefFinished;
+                        return;
+                    } else {
+                        limit = below(t);
+                        hit = (int32_t)tri;
+                        hv = v;
+                        hw = wb;
+                    }
+                }
+            }
+            if (count == 1u) stack.pop(sp, ref, tn, tf);
+        } while ((oct & 0x78u) != 0u && busy());
     }
 };
 
@@ -539,9 +864,15 @@ struct WideRay {
     Rng<false> rng;  // carried through (no alpha draws in the wide form)
 
     PTD explicit WideRay(Scene scene) : sc(scene), todo(kIdle) {}
+    PTD bool busy() const { return todo >= 0; }
+    PTD bool at_node() const { return todo == 0; }
+    PTD bool at_leaf() const { return todo > 0; }
+    PTD bool finished() const { return todo == kFinished; }
+    PTD void set_idle() { todo = kIdle; }
     PTD float hit_t() const { return limit; }
 
-    PTD void init(f3 origin, f3 dir, float t_max, int32_t light) {
+    template <class S>
+    PTD void init(f3 origin, f3 dir, float t_max, int32_t light, S&) {
         o = origin;
         d = dir;
         rcp = 1.0f / d;
@@ -751,7 +1082,7 @@ constexpr uint32_t kSortPerThread = kSortBuckets / 1024;
 template <class Ray>
 PTD uint32_t file_and_fetch(const Queues& q, const Ray& ray, uint32_t slot, uint32_t want) {
     const unsigned lane = lane_id();
-    const bool fin = ray.todo == kFinished, hit = fin && ray.hit != -1;
+    const bool fin = ray.finished(), hit = fin && ray.hit != -1;
     const unsigned hits = __ballot_sync(0xffffffffu, hit), done = __ballot_sync(0xffffffffu, fin);
     const unsigned misses = done & ~hits;
     uint32_t base = 0;
@@ -778,6 +1109,29 @@ PTD uint32_t fetch_entries(uint32_t* fetch, uint32_t want) {
     if (lane_id() == 0u && want) base = atomicAdd(fetch, want);
     return __shfl_sync(0xffffffffu, base, 0);
 }
+
+// The traversal of a kernel: the 8-wide BVH of the precision form, the packed
+// BVH, or the uploaded nodes (recording kernels, pt_trace_noalloc, and scenes
+// that the packed form cannot hold).
+template <bool kRec, bool kAlpha, bool kShadow, bool kTri36, bool kWide, bool kPacked, class Scene>
+using RayOf = typename std::conditional<
+    kWide, WideRay<kShadow, Scene>,
+    typename std::conditional<kPacked, PackedRay<kAlpha, kShadow, Scene>,
+                              BinaryRay<kRec, kAlpha, kShadow, kTri36, Scene>>::type>::type;
+
+// its stack, with the shared memory of one block
+template <uint32_t kThreads, bool kWide, bool kPacked>
+struct BlockStack {
+    static constexpr uint32_t kShared = kWide ? kWideSmemStack : kPacked ? kPackedSmemStack : kSmemStack;
+    using Lane = typename std::conditional<kPacked, PackedStack<kThreads, kShared>, LaneStack<kThreads, kShared>>::type;
+    typename std::conditional<kPacked, float4, uint2>::type top[kShared * kThreads];
+    PTD void bind(Lane& lane) {
+        if constexpr (kPacked)
+            lane.bind(top);
+        else
+            lane.col = top + threadIdx.x;
+    }
+};
 
 // 1: in opaque scenes a shading step adds exactly one radiance term to its
 // path's colour (the sky at a miss, trace.slang:925; emission at a hit,
@@ -1018,32 +1372,35 @@ PTD void traverse_queue(uint32_t count, uint32_t max_visits, Ray& ray, S& stack,
     const unsigned lane = lane_id();
     bool exhausted = false;
     for (;;) {
-        unsigned busy = __ballot_sync(0xffffffffu, ray.todo >= 0);
+        unsigned busy = __ballot_sync(0xffffffffu, ray.busy());
         if (busy == 0u || (!exhausted && __popc(busy) <= Ray::kRefillAt)) {
             const unsigned idle = ~busy;
             const uint32_t want = exhausted ? 0u : (uint32_t)__popc(idle);
             const uint32_t base = turn(want);
-            if (ray.todo == kFinished) ray.todo = kIdle;
+            if (ray.finished()) ray.set_idle();
             if (exhausted) break;  // nobody is busy, nothing is left
-            if (ray.todo == kIdle) {
+            if (!ray.busy()) {
                 const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
                 if (i < count) start(i);
             }
             exhausted = base + want >= count;
-            busy = __ballot_sync(0xffffffffu, ray.todo >= 0);
+            busy = __ballot_sync(0xffffffffu, ray.busy());
             if (busy == 0u) break;
         }
         const int keep = max(1, (__popc(busy) * Ray::kVisitKeep) >> 5);
         uint32_t visits = 0;
         unsigned m;
         do {
-            if (ray.todo == 0) ray.visit(stack, istack);
-            m = __ballot_sync(0xffffffffu, ray.todo == 0);
+            if (ray.at_node()) ray.visit(stack, istack);
+#if PT_VISIT_TWICE
+            if (ray.at_node()) ray.visit(stack, istack);
+#endif
+            m = __ballot_sync(0xffffffffu, ray.at_node());
         } while (__popc(m) >= keep && ++visits < max_visits);
-        m = __ballot_sync(0xffffffffu, ray.todo > 0);
+        m = __ballot_sync(0xffffffffu, ray.at_leaf());
         while (m != 0u) {
-            if (ray.todo > 0) ray.test(stack, istack);
-            m = __ballot_sync(0xffffffffu, ray.todo > 0);
+            if (ray.at_leaf()) ray.test(stack, istack);
+            m = __ballot_sync(0xffffffffu, ray.at_leaf());
             if (__popc(m) <= Ray::kTestLeave) break;
         }
     }

@@ -23,8 +23,16 @@ struct Wavefront;
 
 int create(Wavefront** out);
 void destroy(Wavefront* wf);
-// the world buffers changed: derived layouts are rebuilt on the next trace
-void world_changed(Wavefront* wf);
+// the world buffers changed: derived layouts are rebuilt on the next trace;
+// packable: every node of the BVH is reachable and it fits the packed form
+// (ptw::packable)
+void world_changed(Wavefront* wf, bool packable);
+
+// whether a BVH whose `reached` nodes hang off the root, with at most
+// max_leaf triangles in a leaf, can be packed
+bool packable(uint64_t nodes, uint64_t reached, uint64_t tris, uint32_t max_leaf);
+// the packed BVH of a packable tree, on `stream` (ptd::packed_bytes bytes)
+cudaError_t pack_bvh(const pt_bvh_node* nodes, uint64_t n, float4* packed, cudaStream_t stream);
 
 // wraps each kernel launch (class id from PT_KC_*, the stream it is queued
 // on) so the caller can time it
@@ -33,8 +41,8 @@ using Timer = std::function<cudaError_t(int cls, cudaStream_t stream, const std:
 // the skybox texels changed (its BF16 copy is rebuilt on the next trace)
 void sky_changed(Wavefront* wf);
 
-// (re)build the derived layouts after world_changed: the child-pair BVH and
-// padded triangles always; for the precision form (PT_PRECISION_* bits of
+// (re)build the derived layouts after world_changed: the packed BVH (of a
+// packable tree) and padded triangles always; for the precision form (PT_PRECISION_* bits of
 // include/pt_precision.h) the 8-wide BVH (collapsed on the host from the
 // device's binary nodes) and the FP16 attributes / BF16 skybox.
 // *queued (if given): whether work was queued on `stream`.

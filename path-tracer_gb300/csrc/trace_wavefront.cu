@@ -8,9 +8,8 @@
 //   colour per path id:                  (final_color xyz, unused)
 //   shadow queue (slot order):           (origin xyz, path id), (direction xyz, distance),
 //                                        (contribution xyz, light triangle bits)
-//   BVH nodes copied 32 bytes past a 256-byte boundary, so the two children
-//   of every interior node (indices 2k+1, 2k+2) fill one aligned 64-byte
-//   block read with four 16-byte loads; triangles padded to 3 x float4.
+//   BVH packed to 32 bytes a child pair (PackedRay, pt_wave.cuh); triangles
+//   padded to 4 x float4.
 // Every path runs exactly the arithmetic of the plain kernel (pt_path.cuh),
 // in the same order, so results are bit-identical.
 #include <cmath>
@@ -120,18 +119,17 @@ __global__ void shadow_reset_kernel(uint32_t* cnt) {
 // finishes, so long and short rays do not leave lanes idle.  Finished rays
 // are filed under hits or misses for the shading kernel.  kWide traverses the
 // 8-wide BVH of the precision form instead of the binary one.
-template <bool kRec, bool kAlpha, bool kTri36 = false, bool kWide = false>
+template <bool kRec, bool kAlpha, bool kTri36, bool kWide, bool kPacked>
 __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS) extend_kernel(World w, Fast f, Queues q, int cur, uint32_t bounce) {
     static_assert(!(kWide && (kRec || kAlpha)), "the wide form keeps no records and runs opaque scenes only");
+    static_assert(!(kPacked && (kRec || kTri36 || kWide)), "the packed form keeps no records");
     const Stage st = stage_of(q, cur);
     const uint32_t count = *st.count;
-    using Ray = typename std::conditional<kWide, WideRay<false, OneScene>,
-                                          BinaryRay<kRec, kAlpha, false, kTri36, OneScene>>::type;
-    Ray ray(OneScene{w, f});
-    constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
-    __shared__ uint2 stack_top[kShared > 0u ? kShared * kExtendThreads : 1u];
-    LaneStack<kExtendThreads, kShared> stack;
-    stack.col = stack_top + threadIdx.x;
+    RayOf<kRec, kAlpha, false, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
+    using Stacks = BlockStack<kExtendThreads, kWide, kPacked>;
+    __shared__ Stacks stacks;
+    typename Stacks::Lane stack;
+    stacks.bind(stack);
     uint32_t istack[kRec ? 64 : 1];
     uint32_t slot = 0, path = 0;
     traverse_queue(
@@ -142,10 +140,10 @@ __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : P
             path = __float_as_uint(o4.w);
             ray.rng.s = __float_as_uint(d4.w);
             if constexpr (kRec) ray.c = q.rec[path];
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1);
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1, stack);
         },
         [&](uint32_t want) {
-            if (ray.todo == kFinished) {
+            if (ray.finished()) {
                 if constexpr (kAlpha) st.d[slot].w = __uint_as_float(ray.rng.s);
                 if constexpr (kRec) {
                     q.rec[path] = ray.c;
@@ -226,17 +224,15 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS) shade_kern
 
 // Persistent shadow kernel (opaque scenes): any-hit traversal of every queued
 // shadow ray with the same lane refill; unoccluded rays add their light.
-template <bool kRec, bool kTri36 = false, bool kWide = false>
+template <bool kRec, bool kTri36, bool kWide, bool kPacked>
 __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS) shadow_kernel(World w, Fast f, Queues q) {
     static_assert(!(kWide && kRec), "the wide form keeps no records");
     const uint32_t count = q.cnt[2];
-    using Ray = typename std::conditional<kWide, WideRay<true, OneScene>,
-                                          BinaryRay<kRec, false, true, kTri36, OneScene>>::type;
-    Ray ray(OneScene{w, f});
-    constexpr uint32_t kShared = kWide ? kWideSmemStack : kSmemStack;
-    __shared__ uint2 stack_top[kShared > 0u ? kShared * kExtendThreads : 1u];
-    LaneStack<kExtendThreads, kShared> stack;
-    stack.col = stack_top + threadIdx.x;
+    RayOf<kRec, false, true, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
+    using Stacks = BlockStack<kExtendThreads, kWide, kPacked>;
+    __shared__ Stacks stacks;
+    typename Stacks::Lane stack;
+    stacks.bind(stack);
     uint32_t istack[kRec ? 64 : 1];
     uint32_t path = 0;
     f3 contribution = mk(0.0f, 0.0f, 0.0f);
@@ -247,10 +243,10 @@ __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : P
             contribution = mk(c4.x, c4.y, c4.z);
             path = __float_as_uint(o4.w);
             if constexpr (kRec) ray.c = q.rec[path];
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w));
+            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w), stack);
         },
         [&](uint32_t want) {
-            if (ray.todo == kFinished) {
+            if (ray.finished()) {
                 if (ray.hit != 1) {
                     const float4 col = q.color[path];
                     const f3 sum = mk(col.x, col.y, col.z) + contribution;
@@ -383,9 +379,9 @@ __global__ void debug_intersect_wide_kernel(World w, Fast f, uint64_t n, const f
     WideRay<false, OneScene> ray(OneScene{w, f});
     LocalStack stack;
     ray.init(mk(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2]),
-             mk(directions[3 * i], directions[3 * i + 1], directions[3 * i + 2]), t_max ? t_max[i] : kFltMax, -1);
-    while (ray.todo >= 0) {
-        if (ray.todo == 0)
+             mk(directions[3 * i], directions[3 * i + 1], directions[3 * i + 2]), t_max ? t_max[i] : kFltMax, -1, stack);
+    while (ray.busy()) {
+        if (ray.at_node())
             ray.visit(stack, nullptr);
         else
             ray.test(stack, nullptr);
@@ -468,7 +464,8 @@ struct Wavefront {
     int next_lane = 0;
     cudaEvent_t start = nullptr;  // the caller's stream before the last group began
     bool have_start = false;
-    Buf pairs, tri4;
+    Buf packed, tri4;
+    bool packable = false;  // the world's BVH fits the packed form
     Buf wide, links, attr_h, sky_h;  // precision form copies (links: parent per node, leaf per triangle)
     bool stale = true;
     bool wide_ready = false, attr_h_ready = false, sky_h_ready = false;
@@ -517,14 +514,15 @@ void destroy(Wavefront* wf) {
         if (l.stream) cudaStreamDestroy(l.stream);
     }
     if (wf->start) cudaEventDestroy(wf->start);
-    for (Buf* b : {&wf->rec, &wf->rec_hits, &wf->pairs, &wf->tri4, &wf->wide, &wf->links, &wf->attr_h, &wf->sky_h})
+    for (Buf* b : {&wf->rec, &wf->rec_hits, &wf->packed, &wf->tri4, &wf->wide, &wf->links, &wf->attr_h, &wf->sky_h})
         b->release();
     delete wf;
 }
 
-void world_changed(Wavefront* wf) {
+void world_changed(Wavefront* wf, bool packable) {
     if (wf) {
         wf->stale = true;
+        wf->packable = packable;
         wf->wide_ready = wf->attr_h_ready = false;
     }
 }
@@ -536,8 +534,10 @@ void sky_changed(Wavefront* wf) {
 namespace {
 
 cudaError_t build_layouts(Wavefront* wf, const ptd::World& w, uint64_t nodes, uint64_t tris, cudaStream_t stream) {
-    PTW_TRY(wf->pairs.reserve((nodes + 1) * 32 + 256));
-    PTW_TRY(cudaMemcpyAsync(static_cast<char*>(wf->pairs.p) + 32, w.nodes, nodes * 32, cudaMemcpyDeviceToDevice, stream));
+    if (wf->packable) {
+        PTW_TRY(wf->packed.reserve(ptd::packed_bytes(nodes)));
+        PTW_TRY(pack_bvh(w.nodes, nodes, static_cast<float4*>(wf->packed.p), stream));
+    }
     PTW_TRY(wf->tri4.reserve(tris * 16 * ptd::kTriStride));
     ptd::pad_triangles_kernel<<<(unsigned)((tris + 255) / 256), 256, 0, stream>>>(w.geo, tris, static_cast<float4*>(wf->tri4.p));
     PTW_TRY(cudaGetLastError());
@@ -623,15 +623,15 @@ struct SortCfg {
 // 36-byte triangles instead of the padded copy
 // One group of paths through every bounce on `stream`; the accumulation runs
 // on `acc_stream` (null: `stream`) after `done` marks the group's end there.
-template <bool kRec, bool kAlpha, bool kTri36, bool kWide = false, class TimerF>
+template <bool kRec, bool kAlpha, bool kTri36, bool kWide, bool kPacked, class TimerF>
 cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const ptd::Queues& q,
                       const ptk::Tile& tile, const ptd::Group& g, ptk::Sinks sinks, cudaStream_t stream,
                       TimerF&& timer, const SortCfg& sort = SortCfg(), cudaStream_t acc_stream = nullptr,
                       cudaEvent_t done = nullptr, const ShadowSide* side = nullptr) {
     using namespace ptd;
-    const int ext_blocks = sms * occupancy(extend_kernel<kRec, kAlpha, kTri36, kWide>, kExtendThreads);
+    const int ext_blocks = sms * occupancy(extend_kernel<kRec, kAlpha, kTri36, kWide, kPacked>, kExtendThreads);
     const int sha_blocks = sms * occupancy(shade_kernel<kRec, kAlpha>, kShadeThreads);
-    const int shd_blocks = sms * occupancy(shadow_kernel<kRec, kTri36, kWide>, kExtendThreads);
+    const int shd_blocks = sms * occupancy(shadow_kernel<kRec, kTri36, kWide, kPacked>, kExtendThreads);
     PTW_TRY(timer(PT_KC_RAYGEN, stream, [&] {
         raygen_kernel<kRec><<<(g.paths + 255u) / 256u, 256, 0, stream>>>(w, tile, g, q);
         return cudaGetLastError();
@@ -659,7 +659,7 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
             PTW_TRY(timer(PT_KC_SORT, stream, [&] { return order_rays(cur ? q.d[1] : q.d[0], q.cnt + cur, 8u); }));
         }
         PTW_TRY(timer(PT_KC_EXTEND, stream, [&] {
-            extend_kernel<kRec, kAlpha, kTri36, kWide><<<ext_blocks, kExtendThreads, 0, stream>>>(w, f, q, cur, bounce);
+            extend_kernel<kRec, kAlpha, kTri36, kWide, kPacked><<<ext_blocks, kExtendThreads, 0, stream>>>(w, f, q, cur, bounce);
             return cudaGetLastError();
         }));
         if (sort.counts && sort.min_hits != 0xffffffffu) {
@@ -691,7 +691,7 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
                 PTW_TRY(cudaStreamWaitEvent(ss, side->shaded, 0));
             }
             PTW_TRY(timer(PT_KC_SHADOW, ss, [&] {
-                shadow_kernel<kRec, kTri36, kWide><<<shd_blocks, kExtendThreads, 0, ss>>>(w, f, q);
+                shadow_kernel<kRec, kTri36, kWide, kPacked><<<shd_blocks, kExtendThreads, 0, ss>>>(w, f, q);
                 return cudaGetLastError();
             }));
             if (split) PTW_TRY(cudaEventRecord(side->traced, ss));
@@ -745,7 +745,8 @@ cudaError_t trace(Wavefront* wf, const ptd::World& w_in, const ptk::Tile& tile, 
         wf->have_start = false;
     }
     ptd::Fast f;
-    f.pairs = reinterpret_cast<const float4*>(static_cast<const char*>(wf->pairs.p) + 32);
+    f.pairs = reinterpret_cast<const float4*>(w.nodes);
+    f.packed = wf->packable ? static_cast<const float4*>(wf->packed.p) : nullptr;
     f.tri4 = static_cast<const float4*>(wf->tri4.p);
     f.wide = static_cast<const float4*>(wf->wide.p);
     f.parent = static_cast<const uint32_t*>(wf->links.p);
@@ -806,15 +807,23 @@ cudaError_t trace(Wavefront* wf, const ptd::World& w_in, const ptk::Tile& tile, 
         const cudaStream_t as = record ? nullptr : stream;
         const ShadowSide* side = (!record && !serial && PT_SHADOW_SIDE) ? &l.side : nullptr;
         cudaError_t e;
+        const auto group_of = [&](auto alpha, auto wide_form, auto packed) {
+            return run_group<false, decltype(alpha)::value, false, decltype(wide_form)::value, decltype(packed)::value>(
+                wf->sms, w, f, q, tile, g, sinks, gs, timer, sort, as, l.done, w.any_alpha ? nullptr : side);
+        };
+        using std::false_type;
+        using std::true_type;
         if (record)
-            e = w.any_alpha ? run_group<true, true, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer)
-                            : run_group<true, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer);
+            e = w.any_alpha ? run_group<true, true, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer)
+                            : run_group<true, false, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer);
         else if (wide)
-            e = run_group<false, false, false, true>(wf->sms, w, f, q, tile, g, sinks, gs, timer, sort, as, l.done, side);
+            e = group_of(false_type(), true_type(), false_type());
+        else if (f.packed)
+            e = w.any_alpha ? group_of(true_type(), false_type(), true_type())
+                            : group_of(false_type(), false_type(), true_type());
         else
-            e = w.any_alpha ? run_group<false, true, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, sort, as, l.done)
-                            : run_group<false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, sort, as, l.done,
-                                                             side);
+            e = w.any_alpha ? group_of(true_type(), false_type(), false_type())
+                            : group_of(false_type(), false_type(), false_type());
         PTW_TRY(e);
         if (!record) {
             PTW_TRY(cudaEventRecord(l.freed, stream));
@@ -860,6 +869,15 @@ cudaError_t convert_half_attributes(const pt_triangle_attribute* in, uint64_t n,
     return cudaGetLastError();
 }
 
+bool packable(uint64_t nodes, uint64_t reached, uint64_t tris, uint32_t max_leaf) {
+    return reached == nodes && nodes < ptd::kPackedMaxNodes && tris < ptd::kPackedMaxTris && max_leaf <= ptd::kPackedMaxLeaf;
+}
+
+cudaError_t pack_bvh(const pt_bvh_node* nodes, uint64_t n, float4* packed, cudaStream_t stream) {
+    ptd::pack_bvh_kernel<0><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(reinterpret_cast<const float4*>(nodes), n, packed);
+    return cudaGetLastError();
+}
+
 cudaError_t convert_bf16_sky(const float4* in, uint64_t n, uint2* out, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
     ptd::bf16_sky_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(in, n, out);
@@ -876,7 +894,7 @@ cudaError_t debug_intersect_wide(Wavefront* wf, const ptd::World& w, uint64_t n,
                                  cudaStream_t stream) {
     if (!wf->wide_ready) return cudaErrorNotReady;
     ptd::Fast f;
-    f.pairs = reinterpret_cast<const float4*>(static_cast<const char*>(wf->pairs.p) + 32);
+    f.pairs = reinterpret_cast<const float4*>(w.nodes);
     f.tri4 = static_cast<const float4*>(wf->tri4.p);
     f.wide = static_cast<const float4*>(wf->wide.p);
     f.parent = static_cast<const uint32_t*>(wf->links.p);
@@ -1057,8 +1075,8 @@ extern "C" int pt_trace_noalloc(const pt_device_world* world, const pt_trace_par
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto untimed = [](int, cudaStream_t, auto&& launch) { return launch(); };
     const cudaError_t e = w.any_alpha
-                              ? ptw::run_group<false, true, true>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed)
-                              : ptw::run_group<false, false, true>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed);
+                              ? ptw::run_group<false, true, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed)
+                              : ptw::run_group<false, false, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed);
     return noalloc_cuda(error, error_size, e, "trace launch");
 } catch (...) {
     std::string message;
