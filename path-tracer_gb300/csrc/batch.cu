@@ -54,11 +54,12 @@ struct ItemDev {
     uint32_t x0, y0, w, h;
     uint32_t first_sample;  // 1-based sample index n of the first sample
     uint32_t samples;
-    uint32_t pad;
+    uint32_t offset;  // its first path in its wave
 };
 
 struct Ctrl {
-    unsigned long long head, tail;  // ring positions (items)
+    unsigned long long head;  // ring position of the next wave's first item
+    uint32_t feed_items, feed_paths;  // what the host fed for the next wave
     uint32_t wave_items, wave_paths;
     unsigned long long waves;
 };
@@ -77,29 +78,24 @@ constexpr uint32_t kEngineSortShift = 10;  // sort bucket = triangle index / 102
 
 // ---------------------------------------------------------------- kernels
 
-__global__ void plan_kernel(Ctrl* ctrl, const ItemDev* ring, uint64_t ring_cap, uint32_t budget, uint32_t max_items,
-                            WaveBufs b) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    unsigned long long head = ctrl->head;
-    const unsigned long long tail = ctrl->tail;
-    uint32_t n = 0, paths = 0;
-    while (head < tail && n < max_items) {
-        const ItemDev it = ring[head % ring_cap];
-        const uint32_t np = it.w * it.h * it.samples;
-        if (n > 0 && paths + np > budget) break;
-        b.wave_item[n] = (uint32_t)(head % ring_cap);
-        b.wave_off[n] = paths;
-        paths += np;
-        ++n;
-        ++head;
+// takes the fed items off the ring and clears the rounds' counters (one block)
+__global__ void __launch_bounds__(1024) plan_kernel(Ctrl* ctrl, const ItemDev* ring, uint64_t ring_cap, WaveBufs b) {
+    const unsigned long long head = ctrl->head;
+    const uint32_t n = ctrl->feed_items, paths = ctrl->feed_paths;
+    for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
+        const uint32_t at = (uint32_t)((head + k) % ring_cap);
+        b.wave_item[k] = at;
+        b.wave_off[k] = ring[at].offset;
     }
-    b.wave_off[n] = paths;
-    ctrl->head = head;
-    ctrl->wave_items = n;
-    ctrl->wave_paths = paths;
-    ctrl->waves += 1;
-    b.q.cnt[0] = paths;
-    b.q.cnt[1] = 0u;
+    for (uint32_t k = threadIdx.x; k < kCounterWords; k += blockDim.x) b.q.cnt[k] = k == kCntRays ? paths : 0u;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        b.wave_off[n] = paths;
+        ctrl->head = head + n;
+        ctrl->wave_items = n;
+        ctrl->wave_paths = paths;
+        ctrl->waves += 1;
+    }
 }
 
 // one block per item (grid-stride over the wave's items)
@@ -114,6 +110,7 @@ PTD uint32_t item_path(uint32_t s, uint32_t pix, uint32_t px_count, uint32_t sam
 
 __global__ void __launch_bounds__(256) raygen_kernel(const Ctrl* ctrl, const ItemDev* ring, const JobDev* jobs,
                                                      WaveBufs b) {
+    after_previous();
     const uint32_t n_items = ctrl->wave_items;
     for (uint32_t k = blockIdx.x; k < n_items; k += gridDim.x) {
         const ItemDev it = ring[b.wave_item[k]];
@@ -144,16 +141,6 @@ __global__ void __launch_bounds__(256) raygen_kernel(const Ctrl* ctrl, const Ite
     }
 }
 
-__global__ void reset_kernel(uint32_t* cnt, int next) {
-    cnt[next] = 0u;
-    cnt[2] = 0u;
-    cnt[3] = 0u;
-    cnt[4] = 0u;
-    cnt[5] = 0u;
-    cnt[6] = 0u;
-    cnt[7] = 0u;  // set again by the sort when it runs
-}
-
 // resident blocks per SM a kernel of kThreads threads is compiled for: the
 // same registers per thread as kMinBlocks blocks of kBaseThreads threads
 static_assert((kExtendThreads == 64 || kExtendThreads == 128 || kExtendThreads == 256) &&
@@ -169,47 +156,79 @@ PTD LaneScene<SceneDev> lane_scene(const SceneDev* scenes, uint32_t index) {
     return LaneScene<SceneDev>{scenes, index, kWide ? f.wide : f.packed, f.tri4};
 }
 
+// The rays of a round and the shadow rays of the round before (see trace_kernel
+// of trace_wavefront.cu)
 template <bool kAlpha, bool kWide, bool kPacked, int kThreads>
 __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS, kExtendThreads, kThreads))
-    extend_kernel(const SceneDev* scenes, WaveBufs b, int cur, uint32_t steps_per_refill) {
+    trace_kernel(const SceneDev* scenes, WaveBufs b, uint32_t round, uint32_t steps_per_refill) {
     static_assert(!(kAlpha && kWide), "the wide form runs opaque scenes only");
     static_assert(!(kPacked && kWide), "one form of the BVH");
-    const Stage st = stage_of(b.q, cur);
-    const uint32_t count = *st.count;
-    RayOf<false, kAlpha, false, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
     using Stacks = BlockStack<kThreads, kWide, kPacked>;
     __shared__ Stacks stacks;
     typename Stacks::Lane stack;
     stacks.bind(stack);
     uint32_t istack[1];
-    uint32_t slot = 0;
-    traverse_queue(
-        count, kWide ? kWideStepsPerRefill : steps_per_refill, ray, stack, istack,
-        [&](uint32_t i) {
-            slot = i;
-            const float4 o4 = st.o[i], d4 = st.d[i];
-            ray.sc = lane_scene<kWide>(scenes, b.tag[__float_as_uint(o4.w)] & 0xffu);
-            ray.rng.s = __float_as_uint(d4.w);
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1, stack);
-        },
-        [&](uint32_t want) {
-            if constexpr (kAlpha) {
-                if (ray.finished()) st.d[slot].w = __uint_as_float(ray.rng.s);
-            }
-            return file_and_fetch(b.q, ray, slot, want);
-        });
+    const uint32_t visits = kWide ? kWideStepsPerRefill : steps_per_refill;
+    after_previous();
+    uint32_t* const cnt = round_counters(b.q, round);
+    const uint32_t rays = cnt[kCntRays], shadows = kAlpha ? 0u : cnt[kCntShadows];
+    {
+        const Stage st = stage_of(b.q, round);
+        RayOf<false, kAlpha, false, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
+        uint32_t slot = 0;
+        traverse_queue(
+            QueueShare(0u, rays, rays + shadows), visits, ray, stack, istack,
+            [&](uint32_t i) {
+                slot = i;
+                const float4 o4 = st.o[i], d4 = st.d[i];
+                ray.sc = lane_scene<kWide>(scenes, b.tag[__float_as_uint(o4.w)] & 0xffu);
+                ray.rng.s = __float_as_uint(d4.w);
+                ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1, stack);
+            },
+            [&](uint32_t want) {
+                if constexpr (kAlpha) {
+                    if (ray.finished()) st.d[slot].w = __uint_as_float(ray.rng.s);
+                }
+                return file_and_fetch(b.q, cnt, ray, slot, want);
+            });
+    }
+    if constexpr (!kAlpha) {
+        if (shadows == 0u) return;
+        RayOf<false, false, true, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
+        uint32_t path = 0;
+        f3 contribution = mk(0.0f, 0.0f, 0.0f);
+        traverse_queue(
+            QueueShare(rays, shadows, rays + shadows), visits, ray, stack, istack,
+            [&](uint32_t i) {
+                const float4 o4 = b.q.so[i], d4 = b.q.sd[i], c4 = b.q.sc[i];
+                contribution = mk(c4.x, c4.y, c4.z);
+                path = __float_as_uint(o4.w);
+                ray.sc = lane_scene<kWide>(scenes, b.tag[path] & 0xffu);
+                ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w), stack);
+            },
+            [&](uint32_t want) {
+                if (ray.finished() && ray.hit != 1) {
+                    const float4 col = b.q.color[path];
+                    const f3 sum = mk(col.x, col.y, col.z) + contribution;
+                    b.q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
+                }
+                return fetch_entries(cnt + kCntShadowFetch, want);
+            });
+    }
 }
 
 template <bool kAlpha, int kThreads = kShadeThreads>
 __global__ void __launch_bounds__(kThreads, blocks_for(PT_SHADE_MIN_BLOCKS, kShadeThreads, kThreads))
-    shade_kernel(const SceneDev* scenes, const JobDev* jobs, WaveBufs b, int cur, uint32_t bounce) {
-    const Stage st = stage_of(b.q, cur);
-    const ShadeRange range(b.q);
-    const uint32_t count = range.count();
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    shade_kernel(const SceneDev* scenes, const JobDev* jobs, WaveBufs b, uint32_t bounce) {
+    after_previous();
+    const Stage st = stage_of(b.q, bounce);
+    uint32_t* const cnt = round_counters(b.q, bounce);
+    const ShadeRange range = ShadeRange::of<false>(b.q, cnt);
+    const BlockTurns turns(range.count());
+    const uint32_t wi = threadIdx.x >> 5;
     const unsigned lane = lane_id();
-    for (uint32_t base = warp * 32u; base < count; base += warps * 32u) {
+    for (uint32_t at = turns.first; at < turns.last && turns.mine(at, wi); at += turns.step) {
+        const uint32_t base = (at + wi) * 32u;
         const uint32_t i = range.slot(b.q, base + lane);
         bool cont = false;
         ShadowRay sr;
@@ -249,58 +268,27 @@ __global__ void __launch_bounds__(kThreads, blocks_for(PT_SHADE_MIN_BLOCKS, kSha
             store_color<kAlpha>(b.q.color, p, ps.color);
             rs = rng.s;
         }
-        const uint32_t slot = warp_append(cont, st.next_count, 0xffffffffu);
+        const Places to = append_warp(cnt + kRoundCounters, cont, sr.valid);
         if (cont) {
-            st.no[slot] = make_float4(ps.o.x, ps.o.y, ps.o.z, __uint_as_float(p));
-            st.nd[slot] = make_float4(ps.d.x, ps.d.y, ps.d.z, __uint_as_float(rs));
-            st.nT[slot] = make_float4(ps.throughput.x, ps.throughput.y, ps.throughput.z, ps.prev_pdf);
+            st.no[to.ray] = make_float4(ps.o.x, ps.o.y, ps.o.z, __uint_as_float(p));
+            st.nd[to.ray] = make_float4(ps.d.x, ps.d.y, ps.d.z, __uint_as_float(rs));
+            st.nT[to.ray] = make_float4(ps.throughput.x, ps.throughput.y, ps.throughput.z, ps.prev_pdf);
         }
         if constexpr (!kAlpha) {
-            const uint32_t sslot = warp_append(sr.valid, &b.q.cnt[2], 0xffffffffu);
             if (sr.valid) {
-                b.q.so[sslot] = make_float4(sr.o.x, sr.o.y, sr.o.z, __uint_as_float(p));
-                b.q.sd[sslot] = make_float4(sr.d.x, sr.d.y, sr.d.z, sr.dist);
-                b.q.sc[sslot] = make_float4(sr.contribution.x, sr.contribution.y, sr.contribution.z, __int_as_float(sr.light_tri));
+                b.q.so[to.shadow] = make_float4(sr.o.x, sr.o.y, sr.o.z, __uint_as_float(p));
+                b.q.sd[to.shadow] = make_float4(sr.d.x, sr.d.y, sr.d.z, sr.dist);
+                b.q.sc[to.shadow] = make_float4(sr.contribution.x, sr.contribution.y, sr.contribution.z, __int_as_float(sr.light_tri));
             }
         }
     }
-}
-
-template <bool kWide, bool kPacked, int kThreads>
-__global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS, kExtendThreads, kThreads))
-    shadow_kernel(const SceneDev* scenes, WaveBufs b, uint32_t steps_per_refill) {
-    const uint32_t count = b.q.cnt[2];
-    RayOf<false, false, true, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
-    using Stacks = BlockStack<kThreads, kWide, kPacked>;
-    __shared__ Stacks stacks;
-    typename Stacks::Lane stack;
-    stacks.bind(stack);
-    uint32_t istack[1];
-    uint32_t path = 0;
-    f3 contribution = mk(0.0f, 0.0f, 0.0f);
-    traverse_queue(
-        count, kWide ? kWideStepsPerRefill : steps_per_refill, ray, stack, istack,
-        [&](uint32_t i) {
-            const float4 o4 = b.q.so[i], d4 = b.q.sd[i], c4 = b.q.sc[i];
-            contribution = mk(c4.x, c4.y, c4.z);
-            path = __float_as_uint(o4.w);
-            ray.sc = lane_scene<kWide>(scenes, b.tag[path] & 0xffu);
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w), stack);
-        },
-        [&](uint32_t want) {
-            if (ray.finished() && ray.hit != 1) {
-                const float4 col = b.q.color[path];
-                const f3 sum = mk(col.x, col.y, col.z) + contribution;
-                b.q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
-            }
-            return fetch_entries(&b.q.cnt[4], want);
-        });
 }
 
 // accumulate, trace.slang:1299-1308: one block per item, samples in order;
 // then count the item as finished for its job slot
 __global__ void __launch_bounds__(256) accumulate_kernel(const Ctrl* ctrl, const ItemDev* ring, const JobDev* jobs,
                                                          WaveBufs b, uint32_t* items_done) {
+    after_previous();
     const uint32_t n_items = ctrl->wave_items;
     for (uint32_t k = blockIdx.x; k < n_items; k += gridDim.x) {
         const ItemDev it = ring[b.wave_item[k]];
@@ -648,7 +636,7 @@ int setup_wave(pt_engine* e) {
     e->max_items = W / 64 + 1;
     int rc = PT_OK;
     for (int k = 0; k < 11 && !rc; ++k) rc = e->cuda(e->wave[k].alloc((size_t)W * 16), "wave buffers");
-    if (!rc) rc = e->cuda(e->wave[11].alloc(64), "wave counters");
+    if (!rc) rc = e->cuda(e->wave[11].alloc(kCounterWords * 4), "wave counters");
     if (!rc) rc = e->cuda(e->wave[12].alloc((size_t)W * 12 + 2 * kSortBuckets * 4), "wave hit lists");
     if (!rc) rc = e->cuda(cudaMemset(e->wave[12].as<uint32_t>() + 3 * (size_t)W, 0, kSortBuckets * 4), "sort counts");
     if (!rc) rc = e->cuda(e->d_tag.alloc((size_t)W * 4), "wave buffers");
@@ -682,17 +670,10 @@ int setup_wave(pt_engine* e) {
     return PT_OK;
 }
 
-template <class K>
-int occupancy(K kernel, int threads) {
-    int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, 0);
-    return blocks > 0 ? blocks : 1;
-}
-
 // one launch of a persistent stage kernel: the blocks that stay resident on every SM
 template <class... P, class... A>
-void launch_persistent(void (*kernel)(P...), pt_engine* e, int threads, A&&... args) {
-    kernel<<<e->sms * occupancy(kernel, threads), threads, 0, e->stream>>>(std::forward<A>(args)...);
+void launch_persistent(void (*kernel)(P...), pt_engine* e, uint32_t threads, A&&... args) {
+    launch_after(kernel, (uint32_t)e->sms * resident_blocks(kernel, (int)threads), threads, e->stream, std::forward<A>(args)...);
 }
 
 // the launches of one wave (captured into a graph, or issued directly)
@@ -703,51 +684,41 @@ cudaError_t issue_wave(pt_engine* e, uint32_t rounds) {
     Ctrl* ctrl = e->d_ctrl.as<Ctrl>();
     const SceneDev* scenes = e->d_scenes.as<const SceneDev>();
     const JobDev* jobs = e->d_jobs.as<const JobDev>();
-    const int per_wave_blocks = e->sms * 8;
-    plan_kernel<<<1, 32, 0, s>>>(ctrl, ring, e->ring_cap, e->cfg.wave_paths, e->max_items, e->wb);
-    raygen_kernel<<<per_wave_blocks, 256, 0, s>>>(ctrl, ring, jobs, e->wb);
+    const uint32_t per_wave_blocks = (uint32_t)e->sms * 8u;
+    plan_kernel<<<1, 1024, 0, s>>>(ctrl, ring, e->ring_cap, e->wb);
+    launch_after(raygen_kernel, per_wave_blocks, 256u, s, ctrl, ring, jobs, e->wb);
     constexpr bool kWide = kWideBvh && !kAlpha;
     const uint32_t tt = e->cfg.traversal_threads, st = e->cfg.shade_threads;
     // persistent launches: as many blocks as stay resident, for the block shape of the configuration
     // (the uploaded nodes, a rare form, are traversed in one shape)
-    const auto extend = [&](int cur) {
+    const auto trace = [&](uint32_t round) {
         if constexpr (kWide || kPacked) {
-            if (tt == 64u) return launch_persistent(extend_kernel<kAlpha, kWide, kPacked, 64>, e, 64, scenes, e->wb, cur, e->cfg.steps_per_refill);
-            if (tt == 256u) return launch_persistent(extend_kernel<kAlpha, kWide, kPacked, 256>, e, 256, scenes, e->wb, cur, e->cfg.steps_per_refill);
+            if (tt == 64u) return launch_persistent(trace_kernel<kAlpha, kWide, kPacked, 64>, e, 64, scenes, e->wb, round, e->cfg.steps_per_refill);
+            if (tt == 256u) return launch_persistent(trace_kernel<kAlpha, kWide, kPacked, 256>, e, 256, scenes, e->wb, round, e->cfg.steps_per_refill);
         }
-        return launch_persistent(extend_kernel<kAlpha, kWide, kPacked, 128>, e, 128, scenes, e->wb, cur, e->cfg.steps_per_refill);
+        return launch_persistent(trace_kernel<kAlpha, kWide, kPacked, 128>, e, 128, scenes, e->wb, round, e->cfg.steps_per_refill);
     };
-    const auto shade = [&](int cur, uint32_t bounce) {
-        if (st == 128u) return launch_persistent(shade_kernel<kAlpha, 128>, e, 128, scenes, jobs, e->wb, cur, bounce);
-        if (st == 256u) return launch_persistent(shade_kernel<kAlpha, 256>, e, 256, scenes, jobs, e->wb, cur, bounce);
-        if (st == 512u) return launch_persistent(shade_kernel<kAlpha, 512>, e, 512, scenes, jobs, e->wb, cur, bounce);
-        return launch_persistent(shade_kernel<kAlpha, 1024>, e, 1024, scenes, jobs, e->wb, cur, bounce);
+    const auto shade = [&](uint32_t round) {
+        if (st == 128u) return launch_persistent(shade_kernel<kAlpha, 128>, e, 128, scenes, jobs, e->wb, round);
+        if (st == 256u) return launch_persistent(shade_kernel<kAlpha, 256>, e, 256, scenes, jobs, e->wb, round);
+        if (st == 512u) return launch_persistent(shade_kernel<kAlpha, 512>, e, 512, scenes, jobs, e->wb, round);
+        return launch_persistent(shade_kernel<kAlpha, 1024>, e, 1024, scenes, jobs, e->wb, round);
     };
-    const auto shadow = [&]() {
-        if constexpr (kWide || kPacked) {
-            if (tt == 64u) return launch_persistent(shadow_kernel<kWide, kPacked, 64>, e, 64, scenes, e->wb, e->cfg.steps_per_refill);
-            if (tt == 256u) return launch_persistent(shadow_kernel<kWide, kPacked, 256>, e, 256, scenes, e->wb, e->cfg.steps_per_refill);
-        }
-        return launch_persistent(shadow_kernel<kWide, kPacked, 128>, e, 128, scenes, e->wb, e->cfg.steps_per_refill);
-    };
-    int cur = 0;
-    for (uint32_t bounce = 0; bounce < rounds; ++bounce) {
-        reset_kernel<<<1, 1, 0, s>>>(e->wb.q.cnt, cur ^ 1);
-        extend(cur);
+    for (uint32_t round = 0; round < rounds; ++round) {
+        trace(round);
         if (e->cfg.sort_min_hits != 0xffffffffu) {
             // hits of all jobs by triangle bucket (1024 triangles per bucket)
-            sort_count_kernel<1><<<e->sms * 4, kSortThreads, 0, s>>>(World{}, e->wb.q, e->sort_counts,
-                                                                   e->cfg.sort_min_hits, kEngineSortShift);
-            sort_scan_kernel<0><<<1, 1024, 0, s>>>(e->wb.q, e->sort_counts, e->sort_counts + kSortBuckets,
-                                                   e->cfg.sort_min_hits);
-            sort_scatter_kernel<1><<<e->sms * 4, kSortThreads, 0, s>>>(World{}, e->wb.q, e->sort_counts + kSortBuckets,
-                                                                     e->cfg.sort_min_hits, kEngineSortShift);
+            launch_after(sort_count_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round, e->sort_counts,
+                         e->cfg.sort_min_hits, kEngineSortShift);
+            launch_after(sort_scan_kernel<0>, 1u, 1024u, s, e->wb.q, round, e->sort_counts, e->sort_counts + kSortBuckets,
+                         e->cfg.sort_min_hits);
+            launch_after(sort_scatter_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round,
+                         e->sort_counts + kSortBuckets, e->cfg.sort_min_hits, kEngineSortShift);
         }
-        shade(cur, bounce);
-        if constexpr (!kAlpha) shadow();
-        cur ^= 1;
+        shade(round);
     }
-    accumulate_kernel<<<per_wave_blocks, 256, 0, s>>>(ctrl, ring, jobs, e->wb, e->d_done.as<uint32_t>());
+    if constexpr (!kAlpha) trace(rounds);  // the last round's shadow rays
+    launch_after(accumulate_kernel, per_wave_blocks, 256u, s, ctrl, ring, jobs, e->wb, e->d_done.as<uint32_t>());
     cudaMemcpyAsync(e->h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(e->h_done, e->d_done.p, kMaxSlots * 4, cudaMemcpyDeviceToHost, s);
     return cudaGetLastError();
@@ -823,7 +794,7 @@ int start_job(pt_engine* e, Job& j) {
             it.h = std::min(T, a.height - y);
             it.first_sample = a.samples_done + 1u;
             it.samples = j.samples;
-            it.pad = 0;
+            it.offset = 0;
             j.pending.push_back(it);
             j.pending_paths += (uint64_t)it.w * it.h * it.samples;
             ++count;
@@ -870,6 +841,7 @@ int feed_wave(pt_engine* e, size_t* fed, uint32_t* kind, uint32_t* rounds) {
             const uint64_t np = (uint64_t)it.w * it.h * it.samples;
             if (!wave.empty() && paths + np > budget) break;
             wave.push_back(it);
+            wave.back().offset = (uint32_t)paths;
             paths += np;
             j->pending_paths -= np;
             j->pending.pop_front();
@@ -891,9 +863,9 @@ int feed_wave(pt_engine* e, size_t* fed, uint32_t* kind, uint32_t* rounds) {
         done += n;
     }
     e->tail += wave.size();
-    const unsigned long long t = e->tail;
-    int rc = e->cuda(cudaMemcpyAsync(&e->d_ctrl.as<Ctrl>()->tail, &t, sizeof t, cudaMemcpyHostToDevice, e->stream),
-                     "ring tail");
+    const uint32_t feed[2] = {(uint32_t)wave.size(), (uint32_t)paths};
+    int rc = e->cuda(cudaMemcpyAsync(&e->d_ctrl.as<Ctrl>()->feed_items, feed, sizeof feed, cudaMemcpyHostToDevice, e->stream),
+                     "wave feed");
     if (rc) return rc;
     *fed = wave.size();
     return PT_OK;

@@ -812,60 +812,92 @@ PTD Lobes evaluate_lobes_t(f3 wo, f3 wi, const Bsdf& b, const LobeTerms& t) {
     return {f_total, b.p_ggx * pdf_ggx + b.p_diffuse * pdf_eon};
 }
 
-// estimate_e_dielectric, trace.slang:396-411.  With PT_HOIST_INVARIANTS the
-// parts of sample_VNDF, fresnel_exact and ggx_lambda that do not change
-// between the 16 samples (the stretched view vector, ior^2, the squared
-// roughnesses) are evaluated once before the loop, by the same operations in
-// the same order, so every sample's bits are those of the plain loop
-// (1920x1080x64 on the 2.1M-triangle scene: 1817 against 1797 Mrays/s, shade
-// 199.5 against 207.8 ms over three images).
-#ifndef PT_HOIST_INVARIANTS
-#define PT_HOIST_INVARIANTS 1
-#endif
-// unroll factor of that loop (1: a rolled loop; 2 and 4 measured slower on
-// the 2.1M-triangle scene, 1798 and 1789 against 1818 Mrays/s)
-#ifndef PT_EDIEL_UNROLL
-#define PT_EDIEL_UNROLL 1
-#endif
-#define PT_STRINGIFY(x) #x
-#define PT_PRAGMA(x) _Pragma(PT_STRINGIFY(x))
+// The lanes among which a hit's dielectric estimate is spread: 2^log2
+// neighbouring lanes that all shade the same hit, this one being the
+// `index`th, `mask` their lanes.
+struct Spread {
+    uint32_t log2 = 0u, index = 0u;
+    unsigned mask = 0u;
+};
+
+// s after 2 n draws of rand_next, n <= 16: s -> a s + c
+struct RngJump {
+    uint32_t a[17], c[17];
+};
+constexpr RngJump rng_jumps() {
+    RngJump j{};
+    uint32_t a = 1u, c = 0u;
+    for (int n = 0; n <= 16; ++n) {
+        j.a[n] = a;
+        j.c[n] = c;
+        for (int k = 0; k < 2; ++k) {
+            a = a * 747796405u;
+            c = c * 747796405u + 2891336453u;
+        }
+    }
+    return j;
+}
+static __constant__ RngJump kRngJump = rng_jumps();
+
+// One of the 16 samples of estimate_e_dielectric, trace.slang:399-409: its
+// term of the sum, 0 where the sample adds none (the sum is never -0, so adding
+// +0 changes nothing).  The parts of sample_VNDF, fresnel_exact and
+// ggx_lambda that are the same for all 16 are given.
+struct DielectricTerms {
+    f3 wo, ww;
+    float ww1, opl, ior, ior2, ax2, ay2;
+    f2 alpha;
+};
 template <bool kRec>
-PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_color, Rng<kRec>& rng) {
+PTD float dielectric_sample(const DielectricTerms& t, Rng<kRec>& rng) {
+    const float r1 = rng();
+    const float tpr = kTwoPi * rng();
+    float sn, cs;
+    ptm::sincosf_(tpr, &sn, &cs);
+    const f3 h = sample_vndf_ww(t.ww, t.ww1, t.alpha, r1, sn, cs);
+    const f3 wi = reflect(-t.wo, h);
+    if (wi.z <= 0.0f) return 0.0f;
+    const float f = fresnel_exact_sq(t.ior, t.ior2, dot(h, t.wo));
+    return f * t.opl / (t.opl + ggx_lambda_sq(wi, t.ax2, t.ay2));
+}
+
+// estimate_e_dielectric, trace.slang:396-411.  A rolled loop (unrolled by 2
+// and 4 it measured slower).  With kSpread a launch of few hits has 2^log2
+// lanes shade each hit; sample i is then taken by lane i mod 2^log2, from the
+// random state skipped ahead to it, and every lane adds the terms in the
+// order of the samples: the same bits, in a 16th of the time of the longest
+// serial chain of a shading step.
+template <bool kRec, bool kSpread>
+PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_color, Rng<kRec>& rng,
+                             const Spread& spread) {
+    DielectricTerms t;
+    t.wo = wo;
+    t.ww = vndf_view(wo, alpha);
+    t.ww1 = 1.0f + t.ww.z;
+    t.opl = opl;
+    t.ior = ior_m;
+    t.ior2 = ior_m * ior_m;
+    t.alpha = alpha;
+    t.ax2 = alpha.x * alpha.x;
+    t.ay2 = alpha.y * alpha.y;
     float sum = 0.0f;
-#if PT_HOIST_INVARIANTS
-    const f3 ww = vndf_view(wo, alpha);
-    const float ww1 = 1.0f + ww.z;
-    const float ior2 = ior_m * ior_m;
-    const float ax2 = alpha.x * alpha.x, ay2 = alpha.y * alpha.y;
-    PT_PRAGMA(unroll PT_EDIEL_UNROLL)
-    for (int i = 0; i < 16; ++i) {
-        const float r1 = rng();
-        const float tpr = kTwoPi * rng();
-        float sn, cs;
-#if PT_SHARED_SINCOS
-        ptm::sincosf_(tpr, &sn, &cs);
-#else
-        sn = ptm::sinf_(tpr);
-        cs = ptm::cosf_(tpr);
-#endif
-        const f3 h = sample_vndf_ww(ww, ww1, alpha, r1, sn, cs);
-        const f3 wi = reflect(-wo, h);
-        if (wi.z <= 0.0f) continue;
-        const float f = fresnel_exact_sq(ior_m, ior2, dot(h, wo));
-        sum += f * opl / (opl + ggx_lambda_sq(wi, ax2, ay2));
-    }
-#else
+    if (kSpread && !kRec && spread.log2 > 0u) {
+        const uint32_t start = rng.s, lanes = 1u << spread.log2;
+        const uint32_t first = (uint32_t)__ffs(spread.mask) - 1u;
+        rng.s = kRngJump.a[spread.index] * start + kRngJump.c[spread.index];
+        const uint32_t ja = kRngJump.a[lanes], jc = kRngJump.c[lanes];
 #pragma unroll 1
-    for (int i = 0; i < 16; ++i) {
-        const float r1 = rng();
-        const float tpr = kTwoPi * rng();
-        const f3 h = sample_vndf(wo, alpha, r1, tpr);
-        const f3 wi = reflect(-wo, h);
-        if (wi.z <= 0.0f) continue;
-        const float f = fresnel_exact(ior_m, dot(h, wo));
-        sum += f * opl / (opl + ggx_lambda(wi, alpha));
+        for (uint32_t i = 0; i < 16u; i += lanes) {
+            Rng<kRec> own = rng;
+            const float term = dielectric_sample(t, own);
+            for (uint32_t k = 0; k < lanes; ++k) sum += __shfl_sync(spread.mask, term, first + k);
+            rng.s = ja * rng.s + jc;
+        }
+        rng.s = kRngJump.a[16] * start + kRngJump.c[16];
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < 16; ++i) sum += dielectric_sample(t, rng);
     }
-#endif
     return spec_color * sum / 16.0f;
 }
 

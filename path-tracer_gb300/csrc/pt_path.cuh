@@ -198,10 +198,12 @@ struct ShadowRay {
 // here (required when some material is not opaque: its any-hit test draws
 // random numbers before the BSDF sample does); otherwise it is returned in
 // *shadow for a later shadow kernel.  Returns true if the path continues
-// with ps.o / ps.d set to the next ray.
-template <bool kRec, bool kInlineShadow>
+// with ps.o / ps.d set to the next ray.  kSpread: the lanes of `spread` shade
+// this hit together (every one of them computes all of it but the dielectric
+// estimate's samples).
+template <bool kRec, bool kInlineShadow, bool kSpread = false>
 PTD bool shade_hit(const World& w, uint32_t bounce, uint32_t max_bounces, PathState& ps, float hit_t, uint32_t h,
-                   float hv, float hw, Rng<kRec>& rng, Counters* c, ShadowRay* shadow) {
+                   float hv, float hw, Rng<kRec>& rng, Counters* c, ShadowRay* shadow, const Spread& spread = Spread()) {
     const float hu = 1.0f - hv - hw;
     const f2 iuv = interp_uv(w, h, hu, hv, hw);
     const pt_material& m = w.mat[attr_material(w, h)];
@@ -292,7 +294,7 @@ PTD bool shade_hit(const World& w, uint32_t bounce, uint32_t max_bounces, PathSt
     if (ls > 0.0f) bx = mk(wo.x, wo.y, 0.0f) * rsqrt_(ls);
     b.bx = bx;
     b.by = mk(-bx.y, bx.x, 0.0f);
-    b.e_dielectric = estimate_e_dielectric(wo, b.opl, b.alpha, b.ior_m, specular_color, rng);
+    b.e_dielectric = estimate_e_dielectric<kRec, kSpread>(wo, b.opl, b.alpha, b.ior_m, specular_color, rng, spread);
     const f3 luma = mk(0.2126f, 0.7152f, 0.0722f);
     const float albedo_gloss = dot(b.e_dielectric, luma);
     const float albedo_diffuse = (1.0f - albedo_gloss) * base_weight * dot(base_color, luma);

@@ -4,7 +4,10 @@
 // warp-aggregated queue appends.
 #pragma once
 
+#include <map>
+#include <mutex>
 #include <type_traits>
+#include <utility>
 
 #include "pt_path.cuh"
 
@@ -31,21 +34,33 @@ struct Queues {
     float4* sc;
     uint32_t* hit_list;   // slots of the current queue whose ray hit a triangle
     uint32_t* miss_list;  // slots whose ray left the scene
-    uint32_t* hit_sorted = nullptr;  // the hit list sorted by key (when cnt[7] != 0)
+    uint32_t* hit_sorted = nullptr;  // the hit list sorted by key (when the round's kCntSorted != 0)
     // beside the hit list, each filed hit's triangle-bucket sort key (triangle
     // >> key_shift, at most the last bucket), written by the extend kernel so
     // that the sort reads its keys in order instead of gathering the hit
     // records; null: the sort computes the keys itself
     uint32_t* hit_keys = nullptr;
     uint32_t key_shift = 0;
-    uint32_t* cnt;  // [0], [1] ray queue lengths, [2] shadow length, [3] extend fetch, [4] shadow fetch,
-                    // [5] hit list length, [6] miss list length, [7] 1 if hit_sorted holds this bounce's hits,
-                    // [8] 1 if hit_sorted holds the order of the current ray queue, [9] of the shadow queue
+    uint32_t* cnt;  // the counters of every round: kRoundCounters words each, all zeroed before the first
     Counters* rec;  // per path (recording variants)
     int32_t* rec_hits;
 };
 
-// the queues one stage reads and writes, with the ping-pong already resolved
+// The counters of one round (bounce).  Each round has its own, so that no
+// launch is needed to clear them between rounds.
+constexpr uint32_t kRoundCounters = 8;
+constexpr uint32_t kCntRays = 0;         // rays of the round
+constexpr uint32_t kCntShadows = 1;      // shadow rays that the shading of the round before queued
+constexpr uint32_t kCntFetch = 2;        // rays taken; the next two are filed with the same atomic instruction
+constexpr uint32_t kCntHits = 3;         // hit list length
+constexpr uint32_t kCntMisses = 4;       // miss list length
+constexpr uint32_t kCntShadowFetch = 5;  // shadow rays taken
+constexpr uint32_t kCntSorted = 6;       // 1: hit_sorted holds the round's hits
+// rounds 0 .. max_bounces, and the empty one after the last
+constexpr uint32_t kCounterWords = kRoundCounters * (PT_MAX_BOUNCES_LIMIT + 2u);
+PTD uint32_t* round_counters(const Queues& q, uint32_t round) { return q.cnt + kRoundCounters * round; }
+
+// the ray queues a round reads and writes (they alternate)
 struct Stage {
     float4* o;  // current ray queue
     float4* d;
@@ -53,22 +68,23 @@ struct Stage {
     float4* no;  // next ray queue
     float4* nd;
     float4* nT;
-    uint32_t* count;       // length of the current queue
-    uint32_t* next_count;  // length of the next queue
 };
 
-PTD Stage stage_of(const Queues& q, int cur) {
+PTD Stage stage_of(const Queues& q, uint32_t round) {
+    const bool odd = (round & 1u) != 0u;
     Stage s;
-    s.o = cur ? q.o[1] : q.o[0];
-    s.d = cur ? q.d[1] : q.d[0];
-    s.T = cur ? q.T[1] : q.T[0];
-    s.no = cur ? q.o[0] : q.o[1];
-    s.nd = cur ? q.d[0] : q.d[1];
-    s.nT = cur ? q.T[0] : q.T[1];
-    s.count = cur ? q.cnt + 1 : q.cnt;
-    s.next_count = cur ? q.cnt : q.cnt + 1;
+    s.o = odd ? q.o[1] : q.o[0];
+    s.d = odd ? q.d[1] : q.d[0];
+    s.T = odd ? q.T[1] : q.T[0];
+    s.no = odd ? q.o[0] : q.o[1];
+    s.nd = odd ? q.d[0] : q.d[1];
+    s.nT = odd ? q.T[0] : q.T[1];
     return s;
 }
+
+// Waits until the launch before this one in its stream has finished, when it
+// was launched with programmatic stream serialization (else it has already).
+PTD void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // launch shapes (overridable at build time for tuning sweeps)
 #ifndef PT_EXTEND_THREADS
@@ -108,16 +124,6 @@ constexpr uint32_t kWideLeafMerge = PT_WIDE_LEAF_MERGE;
 // resident blocks per SM the 8-wide traversal kernels are compiled for
 #ifndef PT_WIDE_MIN_BLOCKS
 #define PT_WIDE_MIN_BLOCKS 8
-#endif
-// order the next bounce's rays / the shadow rays by direction octant before
-// their traversal (when the hit sort is on and a queue holds at least its
-// threshold); measured slower: the octant split breaks up the origin
-// coherence the hit sort gives the next rays, so off by default
-#ifndef PT_RAY_ORDER
-#define PT_RAY_ORDER 0
-#endif
-#ifndef PT_SHADOW_ORDER
-#define PT_SHADOW_ORDER 0
 #endif
 // 1: a pixel's samples are consecutive paths of a group / work item
 // (camera rays of a warp share their first nodes); 0: sample-major
@@ -1053,16 +1059,54 @@ struct WideRay {
 constexpr uint32_t kStepsPerRefill = PT_STEPS_PER_REFILL;
 constexpr uint32_t kWideStepsPerRefill = PT_WIDE_STEPS_PER_REFILL;
 
-// warp-aggregated append: one atomic per warp, slots in lane order
-PTD uint32_t warp_append(bool want, uint32_t* counter, unsigned mask) {
-    const unsigned ballot = __ballot_sync(mask, want);
-    if (ballot == 0u) return 0xffffffffu;
+// The places of a shading step's next ray and shadow ray in their queues, in
+// lane order.
+struct Places {
+    uint32_t ray, shadow;
+};
+// One atomic instruction per warp (two lanes, neighbouring words `cnt` and
+// `cnt + 1`): atomics on one address leave an L2 slice every 0.65 ns, whatever
+// the number of warps.  All 32 lanes.
+PTD Places append_warp(uint32_t* cnt, bool ray, bool shadow) {
     const unsigned lane = lane_id();
-    const unsigned leader = (unsigned)(__ffs(ballot) - 1);
+    const unsigned rays = __ballot_sync(0xffffffffu, ray), shadows = __ballot_sync(0xffffffffu, shadow);
     uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(ballot));
-    base = __shfl_sync(mask, base, leader);
-    return want ? base + (uint32_t)__popc(ballot & ((1u << lane) - 1u)) : 0xffffffffu;
+    const uint32_t n = (uint32_t)__popc(lane == 0u ? rays : shadows);
+    if (lane < 2u && n) base = atomicAdd(cnt + lane, n);
+    const unsigned before = (1u << lane) - 1u;
+    return Places{__shfl_sync(0xffffffffu, base, 0) + (uint32_t)__popc(rays & before),
+                  __shfl_sync(0xffffffffu, base, 1) + (uint32_t)__popc(shadows & before)};
+}
+// The same with one atomic instruction per block, for launches whose many
+// warps each append little (a hit spread over 16 lanes leaves two per warp).
+// All threads of the block; shared: 2 + 2 per warp words.
+template <int kThreads>
+PTD Places append_block(uint32_t* cnt, bool ray, bool shadow, uint32_t* shared) {
+    constexpr uint32_t kWarps = kThreads / 32;
+    static_assert(kWarps <= 32, "one lane per warp");
+    const unsigned lane = lane_id(), wi = threadIdx.x >> 5;
+    const unsigned rays = __ballot_sync(0xffffffffu, ray), shadows = __ballot_sync(0xffffffffu, shadow);
+    __syncthreads();  // the last step's places have been read
+    if (lane < 2u) shared[2u + 2u * wi + lane] = (uint32_t)__popc(lane == 0u ? rays : shadows);
+    __syncthreads();
+    uint32_t at_ray = 0, at_shadow = 0, all_rays = 0, all_shadows = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kWarps; ++k) {
+        if (k == wi) {
+            at_ray = all_rays;
+            at_shadow = all_shadows;
+        }
+        all_rays += shared[2u + 2u * k];
+        all_shadows += shared[3u + 2u * k];
+    }
+    if (threadIdx.x < 2u) {
+        const uint32_t n = threadIdx.x == 0u ? all_rays : all_shadows;
+        shared[threadIdx.x] = n ? atomicAdd(cnt + threadIdx.x, n) : 0u;
+    }
+    __syncthreads();
+    const unsigned before = (1u << lane) - 1u;
+    return Places{shared[0] + at_ray + (uint32_t)__popc(rays & before),
+                  shared[1] + at_shadow + (uint32_t)__popc(shadows & before)};
 }
 
 // sort keys of the hit sort (see sort_count_kernel)
@@ -1080,7 +1124,7 @@ constexpr uint32_t kSortPerThread = kSortBuckets / 1024;
 // so a warp waits for memory once.  All 32 lanes, converged; `want` lanes ask
 // for entries.  Returns the first entry taken.
 template <class Ray>
-PTD uint32_t file_and_fetch(const Queues& q, const Ray& ray, uint32_t slot, uint32_t want) {
+PTD uint32_t file_and_fetch(const Queues& q, uint32_t* cnt, const Ray& ray, uint32_t slot, uint32_t want) {
     const unsigned lane = lane_id();
     const bool fin = ray.finished(), hit = fin && ray.hit != -1;
     const unsigned hits = __ballot_sync(0xffffffffu, hit), done = __ballot_sync(0xffffffffu, fin);
@@ -1088,7 +1132,7 @@ PTD uint32_t file_and_fetch(const Queues& q, const Ray& ray, uint32_t slot, uint
     uint32_t base = 0;
     if (lane < 3u) {
         const uint32_t n = lane == 0u ? want : (uint32_t)__popc(lane == 1u ? hits : misses);
-        if (n) base = atomicAdd(q.cnt + (lane == 0u ? 3 : 4 + (int)lane), n);
+        if (n) base = atomicAdd(cnt + kCntFetch + lane, n);
     }
     const unsigned below_me = (1u << lane) - 1u;
     const uint32_t bh = __shfl_sync(0xffffffffu, base, 1), bm = __shfl_sync(0xffffffffu, base, 2);
@@ -1162,21 +1206,57 @@ PTD void store_color(float4* color, uint32_t p, f3 c) {
     }
 }
 
-// The shading kernels' view of the filed results: misses first, padded to
-// whole warps, then hits.  Entry j of that range maps to a queue slot.
+// The shading kernels' view of a round's filed results: misses first, padded to
+// whole warps, then hits, each hit on 2^spread neighbouring lanes (see
+// estimate_e_dielectric).  Entry j of that range maps to a queue slot; the
+// first lane of a hit is the one that writes.
 struct ShadeRange {
-    uint32_t n_hit, n_miss, miss_span;
+    uint32_t n_hit, n_miss, miss_span, spread;
     const uint32_t* hits;
-    PTD ShadeRange(const Queues& q)
-        : n_hit(q.cnt[5]), n_miss(q.cnt[6]), miss_span((q.cnt[6] + 31u) & ~31u),
-          hits(q.cnt[7] ? q.hit_sorted : q.hit_list) {}
-    PTD uint32_t count() const { return miss_span + n_hit; }
+    // kSpread: hits are spread while the launch's threads allow it
+    template <bool kSpread>
+    PTD static ShadeRange of(const Queues& q, const uint32_t* cnt) {
+        ShadeRange r;
+        r.n_hit = cnt[kCntHits];
+        r.n_miss = cnt[kCntMisses];
+        r.miss_span = (r.n_miss + 31u) & ~31u;
+        r.hits = cnt[kCntSorted] ? q.hit_sorted : q.hit_list;
+        r.spread = 0u;
+        if constexpr (kSpread) {
+            const uint32_t threads = gridDim.x * blockDim.x;
+            while (r.spread < 4u && r.miss_span + (r.n_hit << (r.spread + 1u)) <= threads) r.spread += 1u;
+        }
+        return r;
+    }
+    PTD uint32_t count() const { return miss_span + (n_hit << spread); }
     // queue slot of entry j, or 0xffffffff for the padding after the misses and past the end
     PTD uint32_t slot(const Queues& q, uint32_t j) const {
         if (j < miss_span) return j < n_miss ? q.miss_list[j] : 0xffffffffu;
-        const uint32_t k = j - miss_span;
+        const uint32_t k = (j - miss_span) >> spread;
         return k < n_hit ? hits[k] : 0xffffffffu;
     }
+    PTD bool leads(uint32_t j) const { return j < miss_span || ((j - miss_span) & ((1u << spread) - 1u)) == 0u; }
+};
+
+// The blocks' share of `count` entries, 32 per warp: with more than one turn
+// per warp, consecutive blocks take consecutive entries (a block's neighbouring
+// hits share its L1); otherwise each block takes an equal run, so that every SM
+// gets some.  for (at = first; at < last; at += step): the block's warp wi has
+// the entries of turn at + wi when mine(at, wi).
+struct BlockTurns {
+    uint32_t first, last, step, run;  // in warps of entries
+    PTD explicit BlockTurns(uint32_t count) {
+        const uint32_t per_block = blockDim.x >> 5;
+        last = (count + 31u) >> 5;
+        run = per_block;
+        step = gridDim.x * per_block;
+        if (last <= step) {
+            run = (last + gridDim.x - 1u) / gridDim.x;
+            step = last;
+        }
+        first = blockIdx.x * run;
+    }
+    PTD bool mine(uint32_t at, uint32_t wi) const { return wi < run && at + wi < last; }
 };
 
 // ---- hit sorting before shading: a counting sort of the hit list into
@@ -1186,8 +1266,8 @@ struct ShadeRange {
 // and mostly of one mesh).  Three passes: block histograms into global
 // counts; one block scans the counts into bucket offsets (and clears the
 // counts for the next bounce); blocks recount their chunk, reserve each
-// key's range with one global atomic and scatter.  Skipped (cnt[7] = 0)
-// below min_hits.
+// key's range with one global atomic and scatter.  Skipped (kCntSorted stays
+// 0) below min_hits.
 constexpr int kSortThreads = 256, kSortItems = 8;
 
 template <int kMode>
@@ -1199,10 +1279,11 @@ PTD uint32_t hit_key(const World& w, const Queues& q, uint32_t slot, uint32_t tr
 }
 
 template <int kMode>
-__global__ void __launch_bounds__(kSortThreads) sort_count_kernel(World w, Queues q, uint32_t* counts,
+__global__ void __launch_bounds__(kSortThreads) sort_count_kernel(World w, Queues q, uint32_t round, uint32_t* counts,
                                                                    uint32_t min_hits, uint32_t tri_shift) {
     __shared__ uint32_t hist[kSortBuckets];
-    const uint32_t n = q.cnt[5];
+    after_previous();
+    const uint32_t n = round_counters(q, round)[kCntHits];
     if (n < min_hits) return;
     for (uint32_t i = threadIdx.x; i < kSortBuckets; i += blockDim.x) hist[i] = 0u;
     __syncthreads();
@@ -1214,86 +1295,15 @@ __global__ void __launch_bounds__(kSortThreads) sort_count_kernel(World w, Queue
         if (hist[i]) atomicAdd(&counts[i], hist[i]);
 }
 
-// Ray ordering: the slots of a ray queue (the next bounce's rays, or the
-// shadow rays) grouped by direction octant, written to `order`; within an
-// octant, slots keep roughly their queue order (which follows the sorted
-// hits, so origins stay close).  A warp of the traversal then holds rays
-// whose near-child choices agree more often.  Only the processing order
-// changes.  `flag` (a counter slot) is 1 when `order` is valid.
-PTD uint32_t octant(float4 d) { return (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u); }
-
-// (templates, as the other sort kernels, so that both translation units may include them)
-template <int kUnused>
-__global__ void __launch_bounds__(kSortThreads) ray_count_kernel(const float4* d, const uint32_t* count,
-                                                                 uint32_t* counts, uint32_t min_rays) {
-    __shared__ uint32_t hist[8];
-    const uint32_t n = *count;
-    if (n < min_rays) return;
-    if (threadIdx.x < 8) hist[threadIdx.x] = 0u;
-    __syncthreads();
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x)
-        atomicAdd(&hist[octant(d[j])], 1u);
-    __syncthreads();
-    if (threadIdx.x < 8 && hist[threadIdx.x]) atomicAdd(&counts[threadIdx.x], hist[threadIdx.x]);
-}
-
-template <int kUnused>
-__global__ void ray_scan_kernel(const uint32_t* count, uint32_t* counts, uint32_t* offsets, uint32_t* flag,
-                                uint32_t min_rays) {
-    if (*count < min_rays) {
-        *flag = 0u;
-        return;
-    }
-    uint32_t base = 0;
-    for (int k = 0; k < 8; ++k) {
-        offsets[k] = base;
-        base += counts[k];
-        counts[k] = 0u;
-    }
-    *flag = 1u;
-}
-
-template <int kUnused>
-__global__ void __launch_bounds__(kSortThreads) ray_scatter_kernel(const float4* d, const uint32_t* count,
-                                                                   uint32_t* offsets, uint32_t* order,
-                                                                   uint32_t min_rays) {
-    __shared__ uint32_t hist[8];
-    const uint32_t n = *count;
-    if (n < min_rays) return;
-    const uint32_t chunk = kSortThreads * kSortItems;
-    for (uint32_t c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
-        if (threadIdx.x < 8) hist[threadIdx.x] = 0u;
-        __syncthreads();
-        uint32_t keys[kSortItems];
-#pragma unroll
-        for (int k = 0; k < kSortItems; ++k) {
-            const uint32_t j = c0 + (uint32_t)k * kSortThreads + threadIdx.x;
-            keys[k] = 0xffffffffu;
-            if (j < n) {
-                keys[k] = octant(d[j]);
-                atomicAdd(&hist[keys[k]], 1u);
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x < 8 && hist[threadIdx.x]) hist[threadIdx.x] = atomicAdd(&offsets[threadIdx.x], hist[threadIdx.x]);
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kSortItems; ++k)
-            if (keys[k] != 0xffffffffu) order[atomicAdd(&hist[keys[k]], 1u)] = c0 + (uint32_t)k * kSortThreads + threadIdx.x;
-        __syncthreads();
-    }
-}
-
 // one block of 1024 threads, kSortPerThread buckets each
 template <int kUnused>
-__global__ void __launch_bounds__(1024) sort_scan_kernel(Queues q, uint32_t* counts, uint32_t* offsets,
-                                                          uint32_t min_hits) {
+__global__ void __launch_bounds__(1024) sort_scan_kernel(Queues q, uint32_t round, uint32_t* counts,
+                                                          uint32_t* offsets, uint32_t min_hits) {
     __shared__ uint32_t part[1024];
+    after_previous();
     const uint32_t t = threadIdx.x;
-    if (q.cnt[5] < min_hits) {
-        if (t == 0) q.cnt[7] = 0u;
-        return;
-    }
+    uint32_t* cnt = round_counters(q, round);
+    if (cnt[kCntHits] < min_hits) return;  // kCntSorted stays 0
     uint32_t c[kSortPerThread], sum = 0;
 #pragma unroll
     for (uint32_t k = 0; k < kSortPerThread; ++k) {
@@ -1315,14 +1325,16 @@ __global__ void __launch_bounds__(1024) sort_scan_kernel(Queues q, uint32_t* cou
         offsets[kSortPerThread * t + k] = base;
         base += c[k];
     }
-    if (t == 0) q.cnt[7] = 1u;
+    if (t == 0) cnt[kCntSorted] = 1u;
 }
 
 template <int kMode>
-__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(World w, Queues q, uint32_t* offsets,
-                                                                     uint32_t min_hits, uint32_t tri_shift) {
+__global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(World w, Queues q, uint32_t round,
+                                                                     uint32_t* offsets, uint32_t min_hits,
+                                                                     uint32_t tri_shift) {
     __shared__ uint32_t hist[kSortBuckets];
-    const uint32_t n = q.cnt[5];
+    after_previous();
+    const uint32_t n = round_counters(q, round)[kCntHits];
     if (n < min_hits) return;
     const uint32_t chunk = kSortThreads * kSortItems;
     for (uint32_t c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
@@ -1350,6 +1362,35 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(World w, Que
     }
 }
 
+// How a launch's warps share a queue: every warp begins with `lanes` entries
+// of its own (no atomic; a launch of few rays then takes none at all), the
+// rest are taken as lanes fall idle.  All 32 lanes when there are enough rays,
+// else as few as share them out, at least 8: a warp of few rays diverges less,
+// but each warp costs an atomic when it files them.
+#ifndef PT_MIN_SHARE
+#define PT_MIN_SHARE 8
+#endif
+struct QueueShare {
+    uint32_t count, first, dealt;  // entries; this warp's first; entries dealt to the warps
+    unsigned usable;               // the lanes that take entries
+    // a launch drains two queues, the first of `before` entries, this one of
+    // `entries`, of `all`: the second begins with the warps that the first's
+    // entries leave over
+    PTD QueueShare(uint32_t before, uint32_t entries, uint32_t all) : count(entries) {
+        const uint32_t per_block = blockDim.x >> 5, warps = gridDim.x * per_block;
+        const uint32_t share = min(max((all + warps - 1u) / warps, (uint32_t)PT_MIN_SHARE), 32u);
+        usable = share >= 32u ? 0xffffffffu : (1u << share) - 1u;
+        // with fewer entries than lanes the warps of a block are far apart in the
+        // queue, so that every SM gets some
+        const uint32_t wi = threadIdx.x >> 5;
+        uint32_t warp = share >= 32u ? blockIdx.x * per_block + wi : wi * gridDim.x + blockIdx.x;
+        const uint32_t taken = min((before + share - 1u) / share, warps);
+        warp = warp >= taken ? warp - taken : warp + warps - taken;
+        first = warp * share;
+        dealt = warps * share;
+    }
+};
+
 // The persistent traversal loop of one warp; every lane holds at most one ray.
 // Node visits and triangle tests run in turns: the warp visits nodes while
 // enough of its busy lanes are at one, then the lanes that reached a leaf test
@@ -1367,23 +1408,25 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(World w, Que
 // queue entries.  A warp leaves only when the queue is exhausted and none of
 // its lanes is busy, so every entry below `count` is traced once.
 template <class Ray, class S, class Start, class Turn>
-PTD void traverse_queue(uint32_t count, uint32_t max_visits, Ray& ray, S& stack, uint32_t* istack, Start&& start,
-                        Turn&& turn) {
+PTD void traverse_queue(const QueueShare& share, uint32_t max_visits, Ray& ray, S& stack, uint32_t* istack,
+                        Start&& start, Turn&& turn) {
     const unsigned lane = lane_id();
-    bool exhausted = false;
+    if (share.first >= share.count) return;
+    bool exhausted = share.dealt >= share.count;
+    if (((share.usable >> lane) & 1u) != 0u && share.first + lane < share.count) start(share.first + lane);
     for (;;) {
         unsigned busy = __ballot_sync(0xffffffffu, ray.busy());
         if (busy == 0u || (!exhausted && __popc(busy) <= Ray::kRefillAt)) {
-            const unsigned idle = ~busy;
+            const unsigned idle = ~busy & share.usable;
             const uint32_t want = exhausted ? 0u : (uint32_t)__popc(idle);
-            const uint32_t base = turn(want);
+            const uint32_t base = share.dealt + turn(want);
             if (ray.finished()) ray.set_idle();
             if (exhausted) break;  // nobody is busy, nothing is left
-            if (!ray.busy()) {
+            if ((idle >> lane) & 1u) {
                 const uint32_t i = base + (uint32_t)__popc(idle & ((1u << lane) - 1u));
-                if (i < count) start(i);
+                if (i < share.count) start(i);
             }
-            exhausted = base + want >= count;
+            exhausted = base + want >= share.count;
             busy = __ballot_sync(0xffffffffu, ray.busy());
             if (busy == 0u) break;
         }
@@ -1404,6 +1447,40 @@ PTD void traverse_queue(uint32_t count, uint32_t max_visits, Ray& ray, S& stack,
             if (__popc(m) <= Ray::kTestLeave) break;
         }
     }
+}
+
+// A launch that may start while the launch before it in its stream ends (the
+// kernel waits for it with after_previous()): 1.4 us from launch to launch
+// against 4.1 us for a grid of 1368 blocks.
+template <class... P, class... A>
+cudaError_t launch_after(void (*kernel)(P...), uint32_t grid, uint32_t block, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute serial{};
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = stream;
+    cfg.attrs = &serial;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+// blocks of a kernel that stay resident on an SM of the current device (asked once per kernel and device)
+template <class K>
+uint32_t resident_blocks(K kernel, int threads) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    static std::mutex mutex;
+    static std::map<std::pair<int, std::pair<const void*, int>>, uint32_t> known;
+    std::lock_guard<std::mutex> lock(mutex);
+    uint32_t& blocks = known[{dev, {reinterpret_cast<const void*>(kernel), threads}}];
+    if (blocks == 0u) {
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, 0);
+        blocks = n > 0 ? (uint32_t)n : 1u;
+    }
+    return blocks;
 }
 
 }  // namespace ptd

@@ -55,14 +55,14 @@ cudaError_t prepare(Wavefront* wf, const ptd::World& w, uint64_t nodes, uint64_t
 uint32_t effective_precision(const ptd::World& w, uint32_t precision, bool record);
 
 // Traces samples first_sample.. of the tile in groups of at most 2^25 paths.
-// Each group runs on one of two internal streams with its own queues, so
+// Each group runs on one of a few internal streams with its own queues, so
 // consecutive groups overlap (the next group's first bounces beside the last
 // bounces of the previous one); its accumulation is queued on `stream`, so
 // any later work there sees the finished samples in order.  `overlap`: no
 // work was queued on `stream` since the previous call's groups began, so this
 // call's groups may start where those did (otherwise they wait for `stream`).
-// Within a group, a bounce's shadow rays are traced on a second stream beside
-// the next bounce's extend stage.  `serial`: no overlap at all (each group
+// Within a group, a bounce's shadow rays are traced by the launch that traces
+// the next bounce's rays.  `serial`: no overlap at all (each group
 // starts after the previous one's accumulation, each stage after the one
 // before), so that the timer sees every kernel alone.
 cudaError_t trace(Wavefront* wf, const ptd::World& w, const ptk::Tile& tile, uint32_t first_sample,

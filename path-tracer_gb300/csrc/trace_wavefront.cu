@@ -12,6 +12,7 @@
 //   padded to 4 x float4.
 // Every path runs exactly the arithmetic of the plain kernel (pt_path.cuh),
 // in the same order, so results are bit-identical.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <mutex>
@@ -59,11 +60,9 @@ PTD size_t path_of(uint32_t s, uint32_t pix, const Group& g) {
 
 template <bool kRec>
 __global__ void __launch_bounds__(256) raygen_kernel(World w, ptk::Tile t, Group g, Queues q) {
+    after_previous();
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) {
-        q.cnt[0] = g.paths;
-        q.cnt[1] = 0u;
-    }
+    if (p < kCounterWords) q.cnt[p] = p == kCntRays ? g.paths : 0u;
     if (p >= g.paths) return;
     uint32_t s, pix;
     split_path(p, g, &s, &pix);
@@ -91,80 +90,111 @@ __global__ void __launch_bounds__(256) raygen_kernel(World w, ptk::Tile t, Group
     }
 }
 
-// counters of one bounce: the next ray queue, the extend fetch, the hit and
-// miss lists, the sort and order flags (shadow: true also the shadow queue,
-// its fetch counter and order flag)
-__global__ void bounce_reset_kernel(uint32_t* cnt, int next, bool shadow) {
-    cnt[next] = 0u;
-    cnt[3] = 0u;
-    cnt[5] = 0u;
-    cnt[6] = 0u;
-    cnt[7] = 0u;
-    cnt[8] = 0u;
-    if (shadow) {
-        cnt[2] = 0u;
-        cnt[4] = 0u;
-        cnt[9] = 0u;
-    }
-}
-// the shadow queue's counters alone (before the shading kernel appends to it)
-__global__ void shadow_reset_kernel(uint32_t* cnt) {
-    cnt[2] = 0u;
-    cnt[4] = 0u;
-    cnt[9] = 0u;
-}
+// What a launch of trace_kernel traces: the rays of its round, the shadow rays
+// of the round before, or both.
+constexpr uint32_t kTraceRays = 1, kTraceShadows = 2;
 
-// Persistent extend kernel: every lane traverses its own ray and takes a new
-// one from the queue (one atomic per warp for all idle lanes) as soon as it
-// finishes, so long and short rays do not leave lanes idle.  Finished rays
-// are filed under hits or misses for the shading kernel.  kWide traverses the
-// 8-wide BVH of the precision form instead of the binary one.
+// Persistent traversal kernel: every lane traverses its own ray and takes a
+// new one from the queue when its warp runs low, so long and short rays do not
+// leave lanes idle.  Closest hits of the round's rays are filed under hits or
+// misses for the shading kernel; unoccluded shadow rays of the round before
+// (opaque scenes) add their light to their path's colour.  The two touch
+// nothing of each other's, so one launch drains both queues: a warp that finds
+// no more rays goes on to the shadow rays, which fill the tail of the rays.
 template <bool kRec, bool kAlpha, bool kTri36, bool kWide, bool kPacked>
-__global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS) extend_kernel(World w, Fast f, Queues q, int cur, uint32_t bounce) {
+__global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS)
+    trace_kernel(World w, Fast f, Queues q, uint32_t round, uint32_t what) {
     static_assert(!(kWide && (kRec || kAlpha)), "the wide form keeps no records and runs opaque scenes only");
     static_assert(!(kPacked && (kRec || kTri36 || kWide)), "the packed form keeps no records");
-    const Stage st = stage_of(q, cur);
-    const uint32_t count = *st.count;
-    RayOf<kRec, kAlpha, false, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
     using Stacks = BlockStack<kExtendThreads, kWide, kPacked>;
     __shared__ Stacks stacks;
     typename Stacks::Lane stack;
     stacks.bind(stack);
     uint32_t istack[kRec ? 64 : 1];
-    uint32_t slot = 0, path = 0;
-    traverse_queue(
-        count, kWide ? kWideStepsPerRefill : kStepsPerRefill, ray, stack, istack,
-        [&](uint32_t i) {
-            slot = i;
-            const float4 o4 = st.o[slot], d4 = st.d[slot];
-            path = __float_as_uint(o4.w);
-            ray.rng.s = __float_as_uint(d4.w);
-            if constexpr (kRec) ray.c = q.rec[path];
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1, stack);
-        },
-        [&](uint32_t want) {
-            if (ray.finished()) {
-                if constexpr (kAlpha) st.d[slot].w = __uint_as_float(ray.rng.s);
-                if constexpr (kRec) {
-                    q.rec[path] = ray.c;
-                    if (bounce < PT_RECORD_MAX_BOUNCES) q.rec_hits[(size_t)path * PT_RECORD_MAX_BOUNCES + bounce] = ray.hit;
+    constexpr uint32_t kVisits = kWide ? kWideStepsPerRefill : kStepsPerRefill;
+    after_previous();
+    uint32_t* const cnt = round_counters(q, round);
+    const uint32_t rays = (what & kTraceRays) ? cnt[kCntRays] : 0u;
+    uint32_t shadows = 0u;
+    if constexpr (!kAlpha) shadows = (what & kTraceShadows) ? cnt[kCntShadows] : 0u;
+    if (rays != 0u) {
+        const Stage st = stage_of(q, round);
+        RayOf<kRec, kAlpha, false, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
+        uint32_t slot = 0, path = 0;
+        traverse_queue(
+            QueueShare(0u, rays, rays + shadows), kVisits, ray, stack, istack,
+            [&](uint32_t i) {
+                slot = i;
+                const float4 o4 = st.o[slot], d4 = st.d[slot];
+                path = __float_as_uint(o4.w);
+                ray.rng.s = __float_as_uint(d4.w);
+                if constexpr (kRec) ray.c = q.rec[path];
+                ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), kFltMax, -1, stack);
+            },
+            [&](uint32_t want) {
+                if (ray.finished()) {
+                    if constexpr (kAlpha) st.d[slot].w = __uint_as_float(ray.rng.s);
+                    if constexpr (kRec) {
+                        q.rec[path] = ray.c;
+                        if (round < PT_RECORD_MAX_BOUNCES) q.rec_hits[(size_t)path * PT_RECORD_MAX_BOUNCES + round] = ray.hit;
+                    }
                 }
-            }
-            return file_and_fetch(q, ray, slot, want);
-        });
+                return file_and_fetch(q, cnt, ray, slot, want);
+            });
+    }
+    if constexpr (!kAlpha) {
+        if (shadows == 0u) return;
+        RayOf<kRec, false, true, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
+        uint32_t path = 0;
+        f3 contribution = mk(0.0f, 0.0f, 0.0f);
+        traverse_queue(
+            QueueShare(rays, shadows, rays + shadows), kVisits, ray, stack, istack,
+            [&](uint32_t i) {
+                const float4 o4 = q.so[i], d4 = q.sd[i], c4 = q.sc[i];
+                contribution = mk(c4.x, c4.y, c4.z);
+                path = __float_as_uint(o4.w);
+                if constexpr (kRec) ray.c = q.rec[path];
+                ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w), stack);
+            },
+            [&](uint32_t want) {
+                if (ray.finished()) {
+                    if (ray.hit != 1) {
+                        const float4 col = q.color[path];
+                        const f3 sum = mk(col.x, col.y, col.z) + contribution;
+                        q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
+                    }
+                    if constexpr (kRec) q.rec[path] = ray.c;
+                }
+                return fetch_entries(cnt + kCntShadowFetch, want);
+            });
+    }
 }
 
-template <bool kRec, bool kAlpha>
-__global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS) shade_kernel(World w, Fast f, Queues q, int cur, uint32_t bounce,
-                                                              uint32_t max_bounces) {
-    const Stage st = stage_of(q, cur);
-    const ShadeRange range(q);
-    const uint32_t count = range.count();
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+// kSpread: hits may be spread over several lanes (launches of few paths)
+template <bool kRec, bool kAlpha, bool kSpread, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads == kShadeThreads ? PT_SHADE_MIN_BLOCKS
+                                                                      : PT_SHADE_MIN_BLOCKS * kShadeThreads / kThreads)
+    shade_kernel(World w, Queues q, uint32_t round, uint32_t max_bounces) {
+    after_previous();
+    const Stage st = stage_of(q, round);
+    uint32_t* const cnt = round_counters(q, round);
+    const ShadeRange range = ShadeRange::of<kSpread>(q, cnt);
+    const BlockTurns turns(range.count());
+    const uint32_t wi = threadIdx.x >> 5;
     const unsigned lane = lane_id();
-    for (uint32_t base = warp * 32u; base < count; base += warps * 32u) {
-        const uint32_t i = range.slot(q, base + lane);
+    __shared__ uint32_t places[kSpread ? 2 + 2 * (kThreads / 32) : 1];
+    Spread spread;
+    if constexpr (kSpread) {
+        spread.log2 = range.spread;
+        spread.index = lane & ((1u << range.spread) - 1u);
+        spread.mask = ((1u << (1u << range.spread)) - 1u) << (lane - spread.index);
+    }
+    for (uint32_t at = turns.first; at < turns.last; at += turns.step) {
+        const bool mine = turns.mine(at, wi);
+        if (!kSpread && !mine) break;  // kSpread: the block's warps append together
+        const uint32_t base = (at + wi) * 32u;
+        const uint32_t i = mine ? range.slot(q, base + lane) : 0xffffffffu;
+        const bool leads = !kSpread || range.leads(base + lane);
         bool cont = false;
         ShadowRay sr;
         sr.valid = false;
@@ -196,70 +226,41 @@ __global__ void __launch_bounds__(kShadeThreads, PT_SHADE_MIN_BLOCKS) shade_kern
             const int32_t hit = __float_as_int(h4.y);
             if (hit == -1) {
                 if constexpr (kRec) c.sky_misses += 1;
-                shade_miss(w, bounce, ps);
+                shade_miss(w, round, ps);
             } else {
                 if constexpr (kRec) c.hits += 1;
-                cont = shade_hit<kRec, kAlpha>(w, bounce, max_bounces, ps, h4.x, (uint32_t)hit, h4.z, h4.w, rng, &c, &sr);
+                cont = shade_hit<kRec, kAlpha, kSpread>(w, round, max_bounces, ps, h4.x, (uint32_t)hit, h4.z, h4.w, rng,
+                                                        &c, &sr, spread);
             }
-            store_color<kAlpha>(q.color, p, ps.color);
+            if (leads) store_color<kAlpha>(q.color, p, ps.color);
+            cont = cont && leads;
+            sr.valid = sr.valid && leads;
             rs = rng.s;
             if constexpr (kRec) q.rec[p] = c;
         }
-        const uint32_t slot = warp_append(cont, st.next_count, 0xffffffffu);
+        Places to;
+        if constexpr (kSpread)
+            to = append_block<kThreads>(cnt + kRoundCounters, cont, sr.valid, places);
+        else
+            to = append_warp(cnt + kRoundCounters, cont, sr.valid);
         if (cont) {
-            st.no[slot] = make_float4(ps.o.x, ps.o.y, ps.o.z, __uint_as_float(p));
-            st.nd[slot] = make_float4(ps.d.x, ps.d.y, ps.d.z, __uint_as_float(rs));
-            st.nT[slot] = make_float4(ps.throughput.x, ps.throughput.y, ps.throughput.z, ps.prev_pdf);
+            st.no[to.ray] = make_float4(ps.o.x, ps.o.y, ps.o.z, __uint_as_float(p));
+            st.nd[to.ray] = make_float4(ps.d.x, ps.d.y, ps.d.z, __uint_as_float(rs));
+            st.nT[to.ray] = make_float4(ps.throughput.x, ps.throughput.y, ps.throughput.z, ps.prev_pdf);
         }
         if constexpr (!kAlpha) {
-            const uint32_t sslot = warp_append(sr.valid, &q.cnt[2], 0xffffffffu);
             if (sr.valid) {
-                q.so[sslot] = make_float4(sr.o.x, sr.o.y, sr.o.z, __uint_as_float(p));
-                q.sd[sslot] = make_float4(sr.d.x, sr.d.y, sr.d.z, sr.dist);
-                q.sc[sslot] = make_float4(sr.contribution.x, sr.contribution.y, sr.contribution.z, __int_as_float(sr.light_tri));
+                q.so[to.shadow] = make_float4(sr.o.x, sr.o.y, sr.o.z, __uint_as_float(p));
+                q.sd[to.shadow] = make_float4(sr.d.x, sr.d.y, sr.d.z, sr.dist);
+                q.sc[to.shadow] = make_float4(sr.contribution.x, sr.contribution.y, sr.contribution.z, __int_as_float(sr.light_tri));
             }
         }
     }
 }
 
-// Persistent shadow kernel (opaque scenes): any-hit traversal of every queued
-// shadow ray with the same lane refill; unoccluded rays add their light.
-template <bool kRec, bool kTri36, bool kWide, bool kPacked>
-__global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : PT_EXTEND_MIN_BLOCKS) shadow_kernel(World w, Fast f, Queues q) {
-    static_assert(!(kWide && kRec), "the wide form keeps no records");
-    const uint32_t count = q.cnt[2];
-    RayOf<kRec, false, true, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
-    using Stacks = BlockStack<kExtendThreads, kWide, kPacked>;
-    __shared__ Stacks stacks;
-    typename Stacks::Lane stack;
-    stacks.bind(stack);
-    uint32_t istack[kRec ? 64 : 1];
-    uint32_t path = 0;
-    f3 contribution = mk(0.0f, 0.0f, 0.0f);
-    traverse_queue(
-        count, kWide ? kWideStepsPerRefill : kStepsPerRefill, ray, stack, istack,
-        [&](uint32_t i) {
-            const float4 o4 = q.so[i], d4 = q.sd[i], c4 = q.sc[i];
-            contribution = mk(c4.x, c4.y, c4.z);
-            path = __float_as_uint(o4.w);
-            if constexpr (kRec) ray.c = q.rec[path];
-            ray.init(mk(o4.x, o4.y, o4.z), mk(d4.x, d4.y, d4.z), d4.w, __float_as_int(c4.w), stack);
-        },
-        [&](uint32_t want) {
-            if (ray.finished()) {
-                if (ray.hit != 1) {
-                    const float4 col = q.color[path];
-                    const f3 sum = mk(col.x, col.y, col.z) + contribution;
-                    q.color[path] = make_float4(sum.x, sum.y, sum.z, 0.0f);
-                }
-                if constexpr (kRec) q.rec[path] = ray.c;
-            }
-            return fetch_entries(&q.cnt[4], want);
-        });
-}
-
 // accumulate, trace.slang:1299-1308, samples of the group in order
 __global__ void accumulate_kernel(ptk::Tile t, Group g, const float4* color) {
+    after_previous();
     const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
     if (pix >= g.pixels) return;
     const uint32_t gy = pix / g.vis_w, gx = pix - gy * g.vis_w;
@@ -417,12 +418,6 @@ struct Buf {
 
 constexpr uint64_t kMaxPaths = 1ull << 25;  // paths in flight per group
 
-// 1: a group's shadow stage runs on a second stream of its lane, beside the
-// next bounce's extend stage
-#ifndef PT_SHADOW_SIDE
-#define PT_SHADOW_SIDE 1
-#endif
-
 #define PTW_TRY(x)                          \
     do {                                    \
         const cudaError_t e_ = (x);         \
@@ -430,13 +425,6 @@ constexpr uint64_t kMaxPaths = 1ull << 25;  // paths in flight per group
     } while (0)
 
 }  // namespace
-
-// the second stream of a lane for the shadow stage, with its two events
-struct ShadowSide {
-    cudaStream_t stream;
-    cudaEvent_t shaded;  // a bounce's shading finished (recorded on the group's stream)
-    cudaEvent_t traced;  // its shadow rays finished (recorded on `stream`)
-};
 
 // The queues of one group of paths and the stream it runs on.  Several lanes
 // let consecutive groups overlap: one group's last bounces (few, long rays
@@ -452,7 +440,6 @@ struct Lane {
     Buf o[2], d[2], T[2], hit, color, so, sd, sc, cnt;
     Buf lists;  // hit list, miss list, sorted hit list (capacity entries each), sort counts and offsets
     cudaStream_t stream = nullptr;
-    ShadowSide side{};            // the stream the lane's shadow stage runs on (PT_SHADOW_SIDE)
     cudaEvent_t done = nullptr;   // the lane's group finished (recorded on the lane)
     cudaEvent_t freed = nullptr;  // its accumulation consumed the colours (recorded on the caller's stream)
     bool pending = false;         // `freed` was recorded and not yet waited for
@@ -476,8 +463,6 @@ struct Wavefront {
     const void* layout_geo = nullptr;
     uint64_t capacity = 0;
     int sms = 0;
-    int extend_blocks[2][2] = {{0, 0}, {0, 0}};
-    int shade_blocks = 0;
 };
 
 int create(Wavefront** out) {
@@ -490,9 +475,6 @@ int create(Wavefront** out) {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.freed, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&l.side.stream, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.side.shaded, cudaEventDisableTiming);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&l.side.traced, cudaEventDisableTiming);
     }
     *out = wf;
     return e == cudaSuccess ? 0 : (int)e;
@@ -505,12 +487,8 @@ void destroy(Wavefront* wf) {
         for (Buf* b : {&l.o[0], &l.o[1], &l.d[0], &l.d[1], &l.T[0], &l.T[1], &l.hit, &l.color, &l.so, &l.sd, &l.sc,
                        &l.cnt, &l.lists})
             b->release();
-        if (l.side.stream) cudaStreamSynchronize(l.side.stream);
         if (l.done) cudaEventDestroy(l.done);
         if (l.freed) cudaEventDestroy(l.freed);
-        if (l.side.shaded) cudaEventDestroy(l.side.shaded);
-        if (l.side.traced) cudaEventDestroy(l.side.traced);
-        if (l.side.stream) cudaStreamDestroy(l.side.stream);
         if (l.stream) cudaStreamDestroy(l.stream);
     }
     if (wf->start) cudaEventDestroy(wf->start);
@@ -581,7 +559,7 @@ cudaError_t reserve_paths(Wavefront* wf, uint64_t paths, bool record) {
     for (Lane& l : wf->lane) {
         for (Buf* x : {&l.o[0], &l.o[1], &l.d[0], &l.d[1], &l.T[0], &l.T[1], &l.hit, &l.color, &l.so, &l.sd, &l.sc})
             PTW_TRY(x->reserve(b));
-        PTW_TRY(l.cnt.reserve(64));
+        PTW_TRY(l.cnt.reserve(ptd::kCounterWords * 4));
         // hit list, miss list, sorted hit list, sort counts and offsets, hit sort keys
         PTW_TRY(l.lists.reserve(paths * 16 + 2 * ptd::kSortBuckets * 4));
         PTW_TRY(cudaMemset(static_cast<uint32_t*>(l.lists.p) + 3 * paths, 0, ptd::kSortBuckets * 4));  // sort counts
@@ -592,13 +570,6 @@ cudaError_t reserve_paths(Wavefront* wf, uint64_t paths, bool record) {
     }
     wf->capacity = paths;
     return cudaSuccess;
-}
-
-template <class K>
-int occupancy(K kernel, int threads) {
-    int blocks = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, threads, 0);
-    return blocks > 0 ? blocks : 1;
 }
 
 // hit sorting of one trace: counts[kSortBuckets] then offsets[kSortBuckets];
@@ -618,95 +589,81 @@ struct SortCfg {
 #define PT_SORT_KEY 1
 #endif
 
-// one group of paths through raygen, max_bounces + 1 rounds of extend /
-// (hit sort) / shade / shadow, and accumulate; kTri36 reads the reference's
-// 36-byte triangles instead of the padded copy
-// One group of paths through every bounce on `stream`; the accumulation runs
-// on `acc_stream` (null: `stream`) after `done` marks the group's end there.
+// A group of at most this many paths is launched for latency: grids of the
+// paths' size instead of resident ones, shading blocks of 128 threads on every
+// SM, and hits spread over the lanes that are left over.  The line: shading
+// 0.60 against 0.69 ms at 0.92 M paths (100k triangles, 640x360x4), 1.05
+// against 1.10 at 1.8 M, 1.95 against 1.81 at 4.2 M (512x512x16, where a
+// block's neighbouring hits share an L1), and no gain in the image from 1 M on.
+#ifndef PT_SMALL_PATHS
+#define PT_SMALL_PATHS (1u << 20)
+#endif
+constexpr int kSmallShadeThreads = 128;
+
+// One group of paths through raygen, max_bounces + 1 rounds of trace / (hit
+// sort) / shade, and accumulate on `stream`; the accumulation runs on
+// `acc_stream` (null: `stream`) after `done` marks the group's end there.
+// kTri36 reads the reference's 36-byte triangles instead of the padded copy.
+// `serial`: a round's shadow rays are traced right after its shading, by a
+// launch of their own (the recording kernels, whose records follow the path's
+// order, and profiling).
 template <bool kRec, bool kAlpha, bool kTri36, bool kWide, bool kPacked, class TimerF>
 cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const ptd::Queues& q,
                       const ptk::Tile& tile, const ptd::Group& g, ptk::Sinks sinks, cudaStream_t stream,
-                      TimerF&& timer, const SortCfg& sort = SortCfg(), cudaStream_t acc_stream = nullptr,
-                      cudaEvent_t done = nullptr, const ShadowSide* side = nullptr) {
+                      TimerF&& timer, bool serial, const SortCfg& sort = SortCfg(), cudaStream_t acc_stream = nullptr,
+                      cudaEvent_t done = nullptr) {
     using namespace ptd;
-    const int ext_blocks = sms * occupancy(extend_kernel<kRec, kAlpha, kTri36, kWide, kPacked>, kExtendThreads);
-    const int sha_blocks = sms * occupancy(shade_kernel<kRec, kAlpha>, kShadeThreads);
-    const int shd_blocks = sms * occupancy(shadow_kernel<kRec, kTri36, kWide, kPacked>, kExtendThreads);
+    const bool small = !kRec && g.paths <= PT_SMALL_PATHS;
+    const auto tracer = trace_kernel<kRec, kAlpha, kTri36, kWide, kPacked>;
+    const auto shader = shade_kernel<kRec, kAlpha, false, kShadeThreads>;
+    uint32_t trace_blocks = (uint32_t)sms * resident_blocks(tracer, kExtendThreads);
+    // 8 rays a warp at least (usable_lanes)
+    if (small) trace_blocks = std::min(trace_blocks, (g.paths + kExtendThreads / 4 - 1) / (kExtendThreads / 4));
     PTW_TRY(timer(PT_KC_RAYGEN, stream, [&] {
-        raygen_kernel<kRec><<<(g.paths + 255u) / 256u, 256, 0, stream>>>(w, tile, g, q);
-        return cudaGetLastError();
+        const uint32_t blocks = (std::max(g.paths, kCounterWords) + 255u) / 256u;
+        return launch_after(raygen_kernel<kRec>, blocks, 256, stream, w, tile, g, q);
     }));
-    int cur = 0;
-    const bool sorting = sort.counts && sort.min_hits != 0xffffffffu;
-    // octant order of a ray queue (current rays: flag 8, shadow rays: flag 9) into hit_sorted
-    const auto order_rays = [&](const float4* dirs, const uint32_t* count, uint32_t flag) {
-        ray_count_kernel<0><<<sms * 2, kSortThreads, 0, stream>>>(dirs, count, sort.counts, sort.min_hits);
-        ray_scan_kernel<0><<<1, 1, 0, stream>>>(count, sort.counts, sort.counts + kSortBuckets, q.cnt + flag,
-                                             sort.min_hits);
-        ray_scatter_kernel<0><<<sms * 4, kSortThreads, 0, stream>>>(dirs, count, sort.counts + kSortBuckets,
-                                                                  q.hit_sorted, sort.min_hits);
-        return cudaGetLastError();
+    const auto trace = [&](int cls, uint32_t round, uint32_t what) {
+        return timer(cls, stream, [&] { return launch_after(tracer, trace_blocks, kExtendThreads, stream, w, f, q, round, what); });
     };
-    // With `side`, bounce k's shadow rays are traced on side->stream while
-    // bounce k + 1's extend (and hit sort) run: neither touches what the other
-    // reads or writes.  Bounce k + 1's shading waits for them (it adds to the
-    // same path colours, in the reference's order, and refills the shadow queue).
-    const bool split = side != nullptr && !kAlpha;
-    for (uint32_t bounce = 0; bounce <= tile.max_bounces; ++bounce) {
-        bounce_reset_kernel<<<1, 1, 0, stream>>>(q.cnt, cur ^ 1, !split);
-        PTW_TRY(cudaGetLastError());
-        if (PT_RAY_ORDER && sorting && bounce > 0) {  // camera rays are coherent already (pixel-major)
-            PTW_TRY(timer(PT_KC_SORT, stream, [&] { return order_rays(cur ? q.d[1] : q.d[0], q.cnt + cur, 8u); }));
-        }
-        PTW_TRY(timer(PT_KC_EXTEND, stream, [&] {
-            extend_kernel<kRec, kAlpha, kTri36, kWide, kPacked><<<ext_blocks, kExtendThreads, 0, stream>>>(w, f, q, cur, bounce);
-            return cudaGetLastError();
-        }));
-        if (sort.counts && sort.min_hits != 0xffffffffu) {
+    const bool shadows = !kAlpha;
+    for (uint32_t round = 0; round <= tile.max_bounces; ++round) {
+        const bool both = shadows && !serial && round > 0;
+        PTW_TRY(trace(PT_KC_EXTEND, round, kTraceRays | (both ? kTraceShadows : 0u)));
+        if (sort.counts && sort.min_hits <= g.paths) {
             PTW_TRY(timer(PT_KC_SORT, stream, [&] {
-                sort_count_kernel<PT_SORT_KEY><<<sms * 4, kSortThreads, 0, stream>>>(w, q, sort.counts, sort.min_hits,
-                                                                                    sort.tri_shift);
-                sort_scan_kernel<0><<<1, 1024, 0, stream>>>(q, sort.counts, sort.counts + kSortBuckets, sort.min_hits);
-                sort_scatter_kernel<PT_SORT_KEY><<<sms * 4, kSortThreads, 0, stream>>>(
-                    w, q, sort.counts + kSortBuckets, sort.min_hits, sort.tri_shift);
-                return cudaGetLastError();
+                cudaError_t e = launch_after(sort_count_kernel<PT_SORT_KEY>, (uint32_t)sms * 4u, kSortThreads, stream, w,
+                                             q, round, sort.counts, sort.min_hits, sort.tri_shift);
+                if (e == cudaSuccess)
+                    e = launch_after(sort_scan_kernel<0>, 1u, 1024u, stream, q, round, sort.counts,
+                                     sort.counts + kSortBuckets, sort.min_hits);
+                if (e == cudaSuccess)
+                    e = launch_after(sort_scatter_kernel<PT_SORT_KEY>, (uint32_t)sms * 4u, kSortThreads, stream, w, q,
+                                     round, sort.counts + kSortBuckets, sort.min_hits, sort.tri_shift);
+                return e;
             }));
-        }
-        if (split) {
-            if (bounce > 0) PTW_TRY(cudaStreamWaitEvent(stream, side->traced, 0));
-            shadow_reset_kernel<<<1, 1, 0, stream>>>(q.cnt);
-            PTW_TRY(cudaGetLastError());
         }
         PTW_TRY(timer(PT_KC_SHADE, stream, [&] {
-            shade_kernel<kRec, kAlpha><<<sha_blocks, kShadeThreads, 0, stream>>>(w, f, q, cur, bounce, tile.max_bounces);
-            return cudaGetLastError();
+            if constexpr (!kRec) {
+                if (small) {
+                    const auto spread = shade_kernel<kRec, kAlpha, true, kSmallShadeThreads>;
+                    return launch_after(spread, (uint32_t)sms * resident_blocks(spread, kSmallShadeThreads),
+                                        kSmallShadeThreads, stream, w, q, round, tile.max_bounces);
+                }
+            }
+            return launch_after(shader, (uint32_t)sms * resident_blocks(shader, kShadeThreads), kShadeThreads, stream, w,
+                                q, round, tile.max_bounces);
         }));
-        if constexpr (!kAlpha) {
-            if (PT_SHADOW_ORDER && sorting) {
-                PTW_TRY(timer(PT_KC_SORT, stream, [&] { return order_rays(q.sd, q.cnt + 2, 9u); }));
-            }
-            const cudaStream_t ss = split ? side->stream : stream;
-            if (split) {
-                PTW_TRY(cudaEventRecord(side->shaded, stream));
-                PTW_TRY(cudaStreamWaitEvent(ss, side->shaded, 0));
-            }
-            PTW_TRY(timer(PT_KC_SHADOW, ss, [&] {
-                shadow_kernel<kRec, kTri36, kWide, kPacked><<<shd_blocks, kExtendThreads, 0, ss>>>(w, f, q);
-                return cudaGetLastError();
-            }));
-            if (split) PTW_TRY(cudaEventRecord(side->traced, ss));
-        }
-        cur ^= 1;
+        // the last round's shadow rays, or every round's
+        if (shadows && (serial || round == tile.max_bounces)) PTW_TRY(trace(PT_KC_SHADOW, round + 1u, kTraceShadows));
     }
-    if (split) PTW_TRY(cudaStreamWaitEvent(stream, side->traced, 0));  // the last bounce's shadow rays
     const cudaStream_t as = acc_stream ? acc_stream : stream;
     if (as != stream) {
         PTW_TRY(cudaEventRecord(done, stream));
         PTW_TRY(cudaStreamWaitEvent(as, done, 0));
     }
     PTW_TRY(timer(PT_KC_ACCUMULATE, as, [&] {
-        accumulate_kernel<<<(g.pixels + 255u) / 256u, 256, 0, as>>>(tile, g, q.color);
-        return cudaGetLastError();
+        return launch_after(accumulate_kernel, (g.pixels + 255u) / 256u, 256u, as, tile, g, q.color);
     }));
     if constexpr (kRec) {
         finalize_records_kernel<<<(g.paths + 255u) / 256u, 256, 0, stream>>>(tile, g, q, sinks);
@@ -805,17 +762,16 @@ cudaError_t trace(Wavefront* wf, const ptd::World& w_in, const ptk::Tile& tile, 
             q.key_shift = sort.tri_shift;
         }
         const cudaStream_t as = record ? nullptr : stream;
-        const ShadowSide* side = (!record && !serial && PT_SHADOW_SIDE) ? &l.side : nullptr;
         cudaError_t e;
         const auto group_of = [&](auto alpha, auto wide_form, auto packed) {
             return run_group<false, decltype(alpha)::value, false, decltype(wide_form)::value, decltype(packed)::value>(
-                wf->sms, w, f, q, tile, g, sinks, gs, timer, sort, as, l.done, w.any_alpha ? nullptr : side);
+                wf->sms, w, f, q, tile, g, sinks, gs, timer, serial, sort, as, l.done);
         };
         using std::false_type;
         using std::true_type;
         if (record)
-            e = w.any_alpha ? run_group<true, true, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer)
-                            : run_group<true, false, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer);
+            e = w.any_alpha ? run_group<true, true, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, true)
+                            : run_group<true, false, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, true);
         else if (wide)
             e = group_of(false_type(), true_type(), false_type());
         else if (f.packed)
@@ -917,7 +873,8 @@ namespace {
 constexpr uint64_t kNoAllocPaths = PT_NOALLOC_MAX_PATHS;
 constexpr size_t kNoAllocQueueBytes = 11ull * 16ull * kNoAllocPaths;  // o, d, T (x2), hit, colour, shadow o/d/c
 constexpr size_t kNoAllocCountersOffset = kNoAllocQueueBytes;
-constexpr size_t kNoAllocLutOffset = kNoAllocCountersOffset + 256;
+constexpr size_t kNoAllocLutOffset = kNoAllocCountersOffset + 1024;
+static_assert(ptd::kCounterWords * 4 <= 1024, "the rounds' counters");
 constexpr size_t kNoAllocListOffset = kNoAllocLutOffset + 1024;  // hit list, miss list
 static_assert(kNoAllocListOffset + 2 * 4 * kNoAllocPaths <= PT_NOALLOC_SCRATCH_BYTES, "static scratch too small");
 
@@ -1075,8 +1032,8 @@ extern "C" int pt_trace_noalloc(const pt_device_world* world, const pt_trace_par
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto untimed = [](int, cudaStream_t, auto&& launch) { return launch(); };
     const cudaError_t e = w.any_alpha
-                              ? ptw::run_group<false, true, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed)
-                              : ptw::run_group<false, false, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed);
+                              ? ptw::run_group<false, true, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed, false)
+                              : ptw::run_group<false, false, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed, false);
     return noalloc_cuda(error, error_size, e, "trace launch");
 } catch (...) {
     std::string message;
