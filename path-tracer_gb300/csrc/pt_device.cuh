@@ -266,6 +266,44 @@ PTD f3 orthonormal_tangent(f3 tangent, f3 normal) {
     return mk(fma_(s * normal.x * normal.x, a, 1.0f), s * normal.x * normal.y * a, -s * normal.x);
 }
 
+// Correctly rounded reciprocal, quotient and square root without the range
+// checks of the compiler's own (17 issue slots a warp each; these take 3, 6
+// and 5): the hardware's approximation, refined with fused multiply-adds and,
+// for the quotient and the root, corrected once by the exact residual
+// (Markstein, IBM J. Res. Dev. 34 (1990): a quotient within one ulp, corrected
+// with the residual and a correctly rounded reciprocal, is correctly rounded).
+// The same bits as 1 / b, a / b and sqrtf(x) where no step leaves the normal
+// range: |b| in [2^-120, 2^120]; for a quotient b > 0 or a not +0 (the sign of
+// a zero quotient), |b| in [2^-60, 2^60], and a zero or |a| and |a / b| in
+// [2^-100, 2^100]; x in [2^-96, 2^126].  Checked against the operators over
+// every significand (tests/test_gpu_fast_math.py).
+PTD float rcp_in_range(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return fma_(y, fma_(-b, y, 1.0f), y);
+}
+PTD float div_by(float a, float b, float rcp_b) {  // rcp_b = 1 / b
+    const float q = a * rcp_b;
+    return fma_(-fma_(b, q, -a), rcp_b, q);
+}
+PTD float div_in_range(float a, float b) { return div_by(a, b, rcp_in_range(b)); }
+PTD float sqrt_from(float x, float rsq) {  // rsq: the approximation of 1 / sqrt(x)
+    const float g = x * rsq;
+    return fma_(fma_(-g, g, x), 0.5f * rsq, g);
+}
+PTD float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+PTD float sqrt_in_range(float x) { return sqrt_from(x, rsqrt_approx(x)); }
+// 1 / b for any b
+PTD float rcp(float b) {
+    const float m = fabsf(b);
+    if (m >= 0x1p-100f && m <= 0x1p100f) return rcp_in_range(b);
+    return 1.0f / b;
+}
+
 PTD float fifth_power(float x) { return x * x * x * x * x; }
 
 // fresnel_exact, trace.slang:330-341, with ior2 = ior * ior given
@@ -659,7 +697,7 @@ PTD bool triangle_test(const Tri& t, f3 o, const Shear& s, float* t_out, float* 
     if (fminf(U, fminf(V, W)) < 0.0f && fmaxf(U, fmaxf(V, W)) > 0.0f) return false;
     const float det = U + V + W;
     if (det == 0.0f) return false;
-    const float inv_det = 1.0f / det;
+    const float inv_det = rcp(det);
     *t_out = s.sz * fma_(U, akz, fma_(V, bkz, W * ckz)) * inv_det;
     *v_out = V * inv_det;
     *w_out = W * inv_det;
@@ -845,13 +883,10 @@ static __constant__ RngJump kRngJump = rng_jumps();
 // ggx_lambda that are the same for all 16 are given.
 struct DielectricTerms {
     f3 wo, ww;
-    float ww1, opl, ior, ior2, ax2, ay2;
+    float ww1, opl, ior, ior2, rcp_ior2, ax2, ay2;
     f2 alpha;
 };
-template <bool kRec>
-PTD float dielectric_sample(const DielectricTerms& t, Rng<kRec>& rng) {
-    const float r1 = rng();
-    const float tpr = kTwoPi * rng();
+PTD float dielectric_sample(const DielectricTerms& t, float r1, float tpr) {
     float sn, cs;
     ptm::sincosf_(tpr, &sn, &cs);
     const f3 h = sample_vndf_ww(t.ww, t.ww1, t.alpha, r1, sn, cs);
@@ -861,12 +896,74 @@ PTD float dielectric_sample(const DielectricTerms& t, Rng<kRec>& rng) {
     return f * t.opl / (t.opl + ggx_lambda_sq(wi, t.ax2, t.ay2));
 }
 
-// estimate_e_dielectric, trace.slang:396-411.  A rolled loop (unrolled by 2
-// and 4 it measured slower).  With kSpread a launch of few hits has 2^log2
-// lanes shade each hit; sample i is then taken by lane i mod 2^log2, from the
-// random state skipped ahead to it, and every lane adds the terms in the
-// order of the samples: the same bits, in a 16th of the time of the longest
-// serial chain of a shading step.
+// sin and cos of x in [0, 2 pi]: ptm::sincosf_ with the quadrant taken from the
+// bits of a sum rounded down (the same floor, without the conversions)
+PTD void sincos_turn(float x, float* sn, float* cs) {
+    const float u = __fadd_rd(fma_(x, ptm::kTwoOverPi, 0.5f), 8388608.0f);
+    const float k = u - 8388608.0f;
+    float r = fma_(-k, ptm::kPio2C1, x);
+    r = fma_(-k, ptm::kPio2C2, r);
+    r = fma_(-k, ptm::kPio2C3, r);
+    const float s = ptm::sin_kernel(r), c = ptm::cos_kernel(r);
+    const uint32_t q = __float_as_uint(u);
+    const bool odd = (q & 1u) != 0u;
+    *sn = __uint_as_float(__float_as_uint(odd ? c : s) ^ ((q << 30) & 0x80000000u));
+    *cs = __uint_as_float(__float_as_uint(odd ? s : c) ^ (((q + 1u) << 30) & 0x80000000u));
+}
+
+// Whether dielectric_sample_fast may be used: every quantity below in a range
+// that keeps its divisions and roots in theirs (alpha in [1e-5, 16], ior in
+// [1/16, 16], 1 + lambda(wo) in [1/4, 2^20], directions of length about 1)
+PTD bool dielectric_fast(const DielectricTerms& t) {
+    const float lo = fminf(fminf(t.alpha.x, t.alpha.y), fminf(t.opl * 4e-5f, t.ior * 16e-5f));
+    const float hi = fmaxf(fmaxf(t.alpha.x, t.alpha.y), fmaxf(t.opl * 0x1p-16f, t.ior));
+    const float dir = fmaxf(fmaxf(fmaxf(fabsf(t.wo.x), fabsf(t.wo.y)), fmaxf(fabsf(t.wo.z), fabsf(t.ww.x))),
+                            fmaxf(fabsf(t.ww.y), fabsf(t.ww.z)));
+    // (a NaN passes the comparisons above, and makes this sum one)
+    const float all = t.alpha.x + t.alpha.y + t.opl + t.ior + t.wo.x + t.wo.y + t.wo.z + t.ww.x + t.ww.y + t.ww.z;
+    return lo >= 1e-5f && hi <= 16.0f && dir <= 2.0f && all == all;
+}
+// dielectric_sample with divisions and roots in range, the same operations in
+// the same order.  *redo: a quantity left the range, the value is not to be
+// used.
+PTD float dielectric_sample_fast(const DielectricTerms& t, float r1, float tpr, bool* redo) {
+    float sn, cs;
+    sincos_turn(tpr, &sn, &cs);
+    const float z = fma_(1.0f - r1, t.ww1, -t.ww.z);
+    const float st2 = saturate(fma_(-z, z, 1.0f));  // 0, or at least 2^-24
+    const float sin_theta = sqrt_from(st2, rsqrt_approx(fmaxf(st2, 0x1p-40f)));
+    const f3 hh = mk(sin_theta * cs, sin_theta * sn, z) + t.ww;
+    const f3 v = mk(hh.x * t.alpha.x, hh.y * t.alpha.y, hh.z);
+    const float d2 = dot(v, v);
+    const f3 h = v * rcp_in_range(sqrt_in_range(d2));
+    const f3 wi = reflect(-t.wo, h);
+    // fresnel_exact, trace.slang:330-341
+    const float c = dot(h, t.wo);
+    const float s = div_by(fma_(-c, c, 1.0f), t.ior2, t.rcp_ior2);
+    const float cos_t = sqrt_in_range(1.0f - s);
+    const float den_s = fma_(t.ior, cos_t, c), den_p = fma_(t.ior, c, cos_t);
+    const float rs = div_in_range(fma_(-t.ior, cos_t, c), den_s);
+    const float rp = div_in_range(fma_(-t.ior, c, cos_t), den_p);
+    const bool total = s >= 1.0f;
+    const float f = total ? 1.0f : 0.5f * (rs * rs + rp * rp);
+    // ggx_lambda, trace.slang:347-352
+    const float wz2 = wi.z * wi.z;
+    const float tan2 = div_in_range(t.ax2 * wi.x * wi.x + t.ay2 * wi.y * wi.y, wz2);
+    const float a = f * t.opl;
+    const float term = div_in_range(a, t.opl + fma_(0.5f, sqrt_in_range(1.0f + tan2), -0.5f));
+    const bool none = wi.z <= 0.0f;
+    *redo = d2 < 0x1p-60f || (!none && (wz2 < 0x1p-60f || (!total && fminf(fabsf(den_s), fabsf(den_p)) < 0x1p-20f) ||
+                                        (a > 0.0f && a < 0x1p-80f)));
+    return none ? 0.0f : term;
+}
+
+// estimate_e_dielectric, trace.slang:396-411: two thirds of the shading
+// kernel's instructions.  A rolled loop (unrolled by 2 and 4 it measured
+// slower).  With kSpread a launch of few hits has 2^log2 lanes shade each hit;
+// sample i is then taken by lane i mod 2^log2, from the random state skipped
+// ahead to it, and every lane adds the terms in the order of the samples: the
+// same bits, in a 16th of the time of the longest serial chain of a shading
+// step.
 template <bool kRec, bool kSpread>
 PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_color, Rng<kRec>& rng,
                              const Spread& spread) {
@@ -877,9 +974,19 @@ PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_co
     t.opl = opl;
     t.ior = ior_m;
     t.ior2 = ior_m * ior_m;
+    t.rcp_ior2 = 1.0f / t.ior2;
     t.alpha = alpha;
     t.ax2 = alpha.x * alpha.x;
     t.ay2 = alpha.y * alpha.y;
+    const bool fast = dielectric_fast(t);
+    const auto sample = [&](Rng<kRec>& r) {
+        const float r1 = r();
+        const float tpr = kTwoPi * r();
+        bool redo = false;
+        float term = dielectric_sample_fast(t, r1, tpr, &redo);
+        if (redo || !fast) term = dielectric_sample(t, r1, tpr);
+        return term;
+    };
     float sum = 0.0f;
     if (kSpread && !kRec && spread.log2 > 0u) {
         const uint32_t start = rng.s, lanes = 1u << spread.log2;
@@ -889,14 +996,14 @@ PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_co
 #pragma unroll 1
         for (uint32_t i = 0; i < 16u; i += lanes) {
             Rng<kRec> own = rng;
-            const float term = dielectric_sample(t, own);
+            const float term = sample(own);
             for (uint32_t k = 0; k < lanes; ++k) sum += __shfl_sync(spread.mask, term, first + k);
             rng.s = ja * rng.s + jc;
         }
         rng.s = kRngJump.a[16] * start + kRngJump.c[16];
     } else {
 #pragma unroll 1
-        for (int i = 0; i < 16; ++i) sum += dielectric_sample(t, rng);
+        for (int i = 0; i < 16; ++i) sum += sample(rng);
     }
     return spec_color * sum / 16.0f;
 }

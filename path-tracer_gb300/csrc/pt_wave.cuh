@@ -319,7 +319,7 @@ struct BinaryRay {
     template <class S>
     PTD void init(f3 origin, f3 dir, float t_max, int32_t light, S&) {
         o = origin;
-        rcp = 1.0f / dir;
+        rcp = mk(ptd::rcp(dir.x), ptd::rcp(dir.y), ptd::rcp(dir.z));
         s = make_shear(dir, rcp);
         nod = -o * rcp;
         limit = boxless(nod) ? -1.0f : below(t_max);
@@ -633,7 +633,7 @@ struct PackedRay {
     template <class S>
     PTD void init(f3 origin, f3 dir, float t_max, int32_t light, S& stack) {
         o = origin;
-        const f3 rcp = 1.0f / dir;
+        const f3 rcp = mk(ptd::rcp(dir.x), ptd::rcp(dir.y), ptd::rcp(dir.z));
         const Shear s = make_shear(dir, rcp);
         axes = (uint32_t)s.kx | ((uint32_t)s.ky << 2) | ((uint32_t)s.kz << 4);
         sx = s.sx;
