@@ -659,46 +659,79 @@ PTD float intersect_aabb(const float* bmin, const float* bmax, f3 nod, f3 rcp, f
     return (t_near <= t_far && t_far > 0.0f && t_near < hit_t) ? fmaxf(0.0f, t_near) : -1.0f;
 }
 
-// watertight shear setup, trace.slang:769-783
+// watertight shear setup, trace.slang:769-783.  axes: the permutation as six
+// flags, kx == 0, kx == 1, ky == 0, ky == 1, kz == 0, kz == 1 (bits 0..5).
 struct Shear {
-    int kx, ky, kz;
+    uint32_t axes;
     float sx, sy, sz;
 };
+// (v.kx, v.ky, v.kz) of three vectors: selects, because the branches that the
+// compiler makes of the plain conditionals take the lanes of a warp, whose
+// permutations differ, one after the other (a triangle test: about 200 warp
+// instructions with them, 80 without)
+PTD void permute3(uint32_t axes, f3& a, f3& b, f3& c) {
+    f3 p, q, r;
+    asm("{\n\t.reg .pred x0, x1, y0, y1, z0, z1;\n\t.reg .b32 t;\n\t"
+        "and.b32 t, %18, 1;\n\tsetp.ne.u32 x0, t, 0;\n\tand.b32 t, %18, 2;\n\tsetp.ne.u32 x1, t, 0;\n\t"
+        "and.b32 t, %18, 4;\n\tsetp.ne.u32 y0, t, 0;\n\tand.b32 t, %18, 8;\n\tsetp.ne.u32 y1, t, 0;\n\t"
+        "and.b32 t, %18, 16;\n\tsetp.ne.u32 z0, t, 0;\n\tand.b32 t, %18, 32;\n\tsetp.ne.u32 z1, t, 0;\n\t"
+        "selp.f32 %0, %10, %11, x1;\n\tselp.f32 %0, %9, %0, x0;\n\t"
+        "selp.f32 %1, %10, %11, y1;\n\tselp.f32 %1, %9, %1, y0;\n\t"
+        "selp.f32 %2, %10, %11, z1;\n\tselp.f32 %2, %9, %2, z0;\n\t"
+        "selp.f32 %3, %13, %14, x1;\n\tselp.f32 %3, %12, %3, x0;\n\t"
+        "selp.f32 %4, %13, %14, y1;\n\tselp.f32 %4, %12, %4, y0;\n\t"
+        "selp.f32 %5, %13, %14, z1;\n\tselp.f32 %5, %12, %5, z0;\n\t"
+        "selp.f32 %6, %16, %17, x1;\n\tselp.f32 %6, %15, %6, x0;\n\t"
+        "selp.f32 %7, %16, %17, y1;\n\tselp.f32 %7, %15, %7, y0;\n\t"
+        "selp.f32 %8, %16, %17, z1;\n\tselp.f32 %8, %15, %8, z0;\n\t}"
+        : "=&f"(p.x), "=&f"(p.y), "=&f"(p.z), "=&f"(q.x), "=&f"(q.y), "=&f"(q.z), "=&f"(r.x), "=&f"(r.y), "=&f"(r.z)
+        : "f"(a.x), "f"(a.y), "f"(a.z), "f"(b.x), "f"(b.y), "f"(b.z), "f"(c.x), "f"(c.y), "f"(c.z), "r"(axes));
+    a = p;
+    b = q;
+    c = r;
+}
+
 PTD Shear make_shear(f3 d, f3 rcp) {
     const float adx = fabsf(d.x), ady = fabsf(d.y), adz = fabsf(d.z);
-    const int kxy = adx > ady ? 0 : 1;
-    const int kz = (kxy == 0 ? adx : ady) > adz ? kxy : 2;
-    const int kx_val = kz == 2 ? 0 : kz + 1;
-    const int ky_val = kx_val == 2 ? 0 : kx_val + 1;
-    const bool is_neg = comp(d, kz) < 0.0f;
+    const bool x_over_y = adx > ady;
+    const bool z_last = !((x_over_y ? adx : ady) > adz);  // kz == 2
+    // kx, ky = the axes after kz, exchanged when the direction's kz component is negative
+    const bool k0 = !z_last && x_over_y, k1 = !z_last && !x_over_y;  // kz == 0, kz == 1
+    const uint32_t forward = k0 ? 0x12u : (k1 ? 0x24u : 0x09u), backward = k0 ? 0x18u : (k1 ? 0x21u : 0x06u);
+    f3 p = d, r = rcp, unused = d;
     Shear s;
-    s.kz = kz;
-    s.kx = is_neg ? ky_val : kx_val;
-    s.ky = is_neg ? kx_val : ky_val;
-    s.sz = comp(rcp, kz);
-    s.sx = -comp(d, s.kx) * s.sz;
-    s.sy = -comp(d, s.ky) * s.sz;
+    s.axes = forward;
+    permute3(s.axes, p, r, unused);
+    if (p.z < 0.0f) {
+        s.axes = backward;
+        const float t = p.x;
+        p.x = p.y;
+        p.y = t;
+    }
+    s.sz = r.z;
+    s.sx = -p.x * s.sz;
+    s.sy = -p.y * s.sz;
     return s;
 }
 
 // watertight ray-triangle test, trace.slang:807-834 (false = rejected)
 PTD bool triangle_test(const Tri& t, f3 o, const Shear& s, float* t_out, float* v_out, float* w_out) {
-    const f3 A = t.v0 - o, B = t.v1 - o, C = t.v2 - o;
-    const float akz = comp(A, s.kz), bkz = comp(B, s.kz), ckz = comp(C, s.kz);
-    const float ax = fma_(s.sx, akz, comp(A, s.kx));
-    const float ay = fma_(s.sy, akz, comp(A, s.ky));
-    const float bx = fma_(s.sx, bkz, comp(B, s.kx));
-    const float by = fma_(s.sy, bkz, comp(B, s.ky));
-    const float cx = fma_(s.sx, ckz, comp(C, s.kx));
-    const float cy = fma_(s.sy, ckz, comp(C, s.ky));
+    f3 A = t.v0 - o, B = t.v1 - o, C = t.v2 - o;
+    permute3(s.axes, A, B, C);
+    const float ax = fma_(s.sx, A.z, A.x);
+    const float ay = fma_(s.sy, A.z, A.y);
+    const float bx = fma_(s.sx, B.z, B.x);
+    const float by = fma_(s.sy, B.z, B.y);
+    const float cx = fma_(s.sx, C.z, C.x);
+    const float cy = fma_(s.sy, C.z, C.y);
     const float U = fma_(cx, by, -cy * bx);
     const float V = fma_(ax, cy, -ay * cx);
     const float W = fma_(bx, ay, -by * ax);
-    if (fminf(U, fminf(V, W)) < 0.0f && fmaxf(U, fmaxf(V, W)) > 0.0f) return false;
+    if (min3f(U, V, W) < 0.0f && max3f(U, V, W) > 0.0f) return false;
     const float det = U + V + W;
     if (det == 0.0f) return false;
     const float inv_det = rcp(det);
-    *t_out = s.sz * fma_(U, akz, fma_(V, bkz, W * ckz)) * inv_det;
+    *t_out = s.sz * fma_(U, A.z, fma_(V, B.z, W * C.z)) * inv_det;
     *v_out = V * inv_det;
     *w_out = W * inv_det;
     return true;

@@ -618,8 +618,7 @@ struct PackedRay {
     int32_t hit, light_tri;
     uint32_t ref, sp;  // sp: position of the stack's top entry
     uint32_t oct;      // bit a: rcp[a] < 0; bits 3..6: visits read the uploaded nodes
-    uint32_t axes;     // kx, ky, kz of the shear, two bits each
-    float sx, sy, sz;
+    Shear s;
     Rng<false> rng;
 
     PTD explicit PackedRay(Scene scene) : sc(scene), ref(kRefIdle) {}
@@ -634,11 +633,7 @@ struct PackedRay {
     PTD void init(f3 origin, f3 dir, float t_max, int32_t light, S& stack) {
         o = origin;
         const f3 rcp = mk(ptd::rcp(dir.x), ptd::rcp(dir.y), ptd::rcp(dir.z));
-        const Shear s = make_shear(dir, rcp);
-        axes = (uint32_t)s.kx | ((uint32_t)s.ky << 2) | ((uint32_t)s.kz << 4);
-        sx = s.sx;
-        sy = s.sy;
-        sz = s.sz;
+        s = make_shear(dir, rcp);
         nod = -o * rcp;
         rp = mk(rcp.x < 0.0f ? 0.0f : rcp.x, rcp.y < 0.0f ? 0.0f : rcp.y, rcp.z < 0.0f ? 0.0f : rcp.z);
         rn = mk(rcp.x < 0.0f ? rcp.x : 0.0f, rcp.y < 0.0f ? rcp.y : 0.0f, rcp.z < 0.0f ? rcp.z : 0.0f);
@@ -709,7 +704,6 @@ struct PackedRay {
             }
             const uint32_t tri = ref >> 7;
             ref += (1u << 7) - (1u << 3);  // the next triangle, one fewer left
-            const Shear s{(int)(axes & 3u), (int)((axes >> 2) & 3u), (int)(axes >> 4), sx, sy, sz};
             float t, v, wb;
             if (!(kShadow && (int32_t)tri == light_tri) &&
                 triangle_test(load_tri4(sc.tri4(), tri), o, s, &t, &v, &wb) && t > 0.0f && t <= limit) {
