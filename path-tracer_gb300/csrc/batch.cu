@@ -1032,6 +1032,7 @@ int upload_scene(pt_engine* e, Scene& s, const pt_world_updates* u) {
     w.sky_alias = s.sky_alias.as<pt_skybox_alias_entry>();
     w.scene_alias = s.scene_alias.as<pt_scene_alias_entry>();
     w.sky_u = *u->skybox_uniforms;
+    w.sky_k = sky_terms(w.sky_u);
     w.scene = *u->scene_uniforms;
     w.srgb_lut = s.lut.as<float>();
     w.any_alpha = s.any_alpha ? 1 : 0;

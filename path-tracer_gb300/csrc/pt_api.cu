@@ -116,6 +116,7 @@ struct pt_ctx {
         w.sky_alias = sky_alias.as<const pt_skybox_alias_entry>();
         w.scene_alias = scene_alias.as<const pt_scene_alias_entry>();
         w.sky_u = sky_u;
+        w.sky_k = ptd::sky_terms(sky_u);
         w.scene = scene;
         w.camera = camera;
         w.srgb_lut = srgb_lut.as<const float>();

@@ -53,8 +53,55 @@ PTD f3 operator-(float s, f3 a) { return {s - a.x, s - a.y, s - a.z}; }
 PTD f3 operator-(f3 a, float s) { return {a.x - s, a.y - s, a.z - s}; }
 PTD float dot(f3 a, f3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
 PTD f3 cross(f3 a, f3 b) { return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x}; }
-PTD float rsqrt_(float x) { return 1.0f / sqrtf(x); }
-PTD float length(f3 v) { return sqrtf(dot(v, v)); }
+PTD float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+
+// Correctly rounded reciprocal, quotient and square root without the range
+// checks of the compiler's own (17 issue slots a warp each; these take 3, 6
+// and 5): the hardware's approximation, refined with fused multiply-adds and,
+// for the quotient and the root, corrected once by the exact residual
+// (Markstein, IBM J. Res. Dev. 34 (1990): a quotient within one ulp, corrected
+// with the residual and a correctly rounded reciprocal, is correctly rounded).
+// The same bits as 1 / b, a / b and sqrtf(x) where no step leaves the normal
+// range: |b| in [2^-120, 2^120]; for a quotient b > 0 or a not +0 (the sign of
+// a zero quotient), |b| in [2^-60, 2^60], and a zero or |a| and |a / b| in
+// [2^-100, 2^100]; x in [2^-96, 2^126].  Checked against the operators over
+// every significand (tests/test_gpu_fast_math.py).
+PTD float rcp_in_range(float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return fma_(y, fma_(-b, y, 1.0f), y);
+}
+PTD float div_by(float a, float b, float rcp_b) {  // rcp_b = 1 / b
+    const float q = a * rcp_b;
+    return fma_(-fma_(b, q, -a), rcp_b, q);
+}
+PTD float div_in_range(float a, float b) { return div_by(a, b, rcp_in_range(b)); }
+PTD float sqrt_from(float x, float rsq) {  // rsq: the approximation of 1 / sqrt(x)
+    const float g = x * rsq;
+    return fma_(fma_(-g, g, x), 0.5f * rsq, g);
+}
+PTD float rsqrt_approx(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+PTD float sqrt_in_range(float x) { return sqrt_from(x, rsqrt_approx(x)); }
+// 1 / b, sqrtf(x) and 1 / sqrtf(x) for any argument
+PTD float rcp(float b) {
+    const float m = fabsf(b);
+    if (__builtin_expect(m >= 0x1p-100f && m <= 0x1p100f, 1)) return rcp_in_range(b);
+    return 1.0f / b;
+}
+PTD float sqrt_(float x) {
+    if (__builtin_expect(x >= 0x1p-90f && x <= 0x1p90f, 1)) return sqrt_in_range(x);
+    return sqrtf(x);
+}
+PTD float rsqrt_(float x) {
+    if (__builtin_expect(x >= 0x1p-90f && x <= 0x1p90f, 1)) return rcp_in_range(sqrt_in_range(x));
+    return 1.0f / sqrtf(x);
+}
+
+PTD float length(f3 v) { return sqrt_(dot(v, v)); }
 PTD f3 normalize(f3 v) { return v * rsqrt_(dot(v, v)); }
 PTD float mix(float a, float b, float t) { return a * (1.0f - t) + b * t; }
 PTD f3 mix(f3 a, f3 b, float t) { return {mix(a.x, b.x, t), mix(a.y, b.y, t), mix(a.z, b.z, t)}; }
@@ -65,7 +112,6 @@ PTD float fract(float x) { return x - floorf(x); }
 PTD float signf(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : 0.0f); }
 PTD f3 reflect(f3 i, f3 n) { return i - (2.0f * dot(n, i)) * n; }
 PTD bool any_positive(f3 v) { return v.x > 0.0f || v.y > 0.0f || v.z > 0.0f; }
-PTD float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 PTD float comp(f3 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : v.z); }
 
 // WGSL u32(f32): truncation, saturating, NaN -> 0
@@ -84,6 +130,25 @@ PTD uint32_t seed(uint32_t px, uint32_t py, uint32_t sample_count) {
     return s | 1u;
 }
 
+// terms of the sky's solid angles and sampling that depend on its size alone
+// (trace.slang:476-481, 560-580), each by the shader's operations
+struct SkyTerms {
+    float step = 0.0f;           // pi / height
+    float half_step = 0.0f;      // pi / 2 / height
+    float sin_half_step = 0.0f;  // sin(step / 2)
+    float width_term = 0.0f;     // 2 pi / width * 2
+    float rcp_width = 0.0f;      // 1 / width
+};
+inline SkyTerms sky_terms(const pt_skybox_uniforms& sky) {
+    SkyTerms k;
+    k.step = kPi / (float)sky.height;
+    k.half_step = 0.5f * kPi / (float)sky.height;
+    k.sin_half_step = ptm::sinf_(0.5f * k.step);
+    k.width_term = kTwoPi / (float)sky.width * 2.0f;
+    k.rcp_width = 1.0f / (float)sky.width;
+    return k;
+}
+
 // the world bind group (trace.slang:163-190) as device pointers
 struct World {
     const pt_triangle_geometry* geo;
@@ -98,6 +163,7 @@ struct World {
     const pt_skybox_alias_entry* sky_alias;
     const pt_scene_alias_entry* scene_alias;
     pt_skybox_uniforms sky_u;
+    SkyTerms sky_k;  // sky_terms(sky_u)
     pt_scene_uniforms scene;
     pt_camera camera;
     const float* srgb_lut;  // sRGB EOTF per byte (Rgba8UnormSrgb decode), 256 floats
@@ -218,9 +284,9 @@ PTD float4 atlas(const World& w, bool srgb, int32_t layer, f2 uv) {
     const uint32_t ix = fx >= 8191.0f ? 8191u : to_u32(fx);
     const uint32_t iy = fy >= 8191.0f ? 8191u : to_u32(fy);
     const uchar4 p = __ldg(reinterpret_cast<const uchar4*>(base) + ((uint64_t)l * PT_ATLAS_SIZE + iy) * PT_ATLAS_SIZE + ix);
-    if (srgb)
-        return make_float4(__ldg(w.srgb_lut + p.x), __ldg(w.srgb_lut + p.y), __ldg(w.srgb_lut + p.z), (float)p.w / 255.0f);
-    return make_float4((float)p.x / 255.0f, (float)p.y / 255.0f, (float)p.z / 255.0f, (float)p.w / 255.0f);
+    const auto unorm = [](unsigned char v) { return div_by((float)v, 255.0f, 1.0f / 255.0f); };  // v / 255
+    if (srgb) return make_float4(__ldg(w.srgb_lut + p.x), __ldg(w.srgb_lut + p.y), __ldg(w.srgb_lut + p.z), unorm(p.w));
+    return make_float4(unorm(p.x), unorm(p.y), unorm(p.z), unorm(p.w));
 }
 
 PTD f2 atlas_uv(f2 uv, const float* os) { return {fma_(uv.x, os[2], os[0]), fma_(uv.y, os[3], os[1])}; }
@@ -266,51 +332,13 @@ PTD f3 orthonormal_tangent(f3 tangent, f3 normal) {
     return mk(fma_(s * normal.x * normal.x, a, 1.0f), s * normal.x * normal.y * a, -s * normal.x);
 }
 
-// Correctly rounded reciprocal, quotient and square root without the range
-// checks of the compiler's own (17 issue slots a warp each; these take 3, 6
-// and 5): the hardware's approximation, refined with fused multiply-adds and,
-// for the quotient and the root, corrected once by the exact residual
-// (Markstein, IBM J. Res. Dev. 34 (1990): a quotient within one ulp, corrected
-// with the residual and a correctly rounded reciprocal, is correctly rounded).
-// The same bits as 1 / b, a / b and sqrtf(x) where no step leaves the normal
-// range: |b| in [2^-120, 2^120]; for a quotient b > 0 or a not +0 (the sign of
-// a zero quotient), |b| in [2^-60, 2^60], and a zero or |a| and |a / b| in
-// [2^-100, 2^100]; x in [2^-96, 2^126].  Checked against the operators over
-// every significand (tests/test_gpu_fast_math.py).
-PTD float rcp_in_range(float b) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-    return fma_(y, fma_(-b, y, 1.0f), y);
-}
-PTD float div_by(float a, float b, float rcp_b) {  // rcp_b = 1 / b
-    const float q = a * rcp_b;
-    return fma_(-fma_(b, q, -a), rcp_b, q);
-}
-PTD float div_in_range(float a, float b) { return div_by(a, b, rcp_in_range(b)); }
-PTD float sqrt_from(float x, float rsq) {  // rsq: the approximation of 1 / sqrt(x)
-    const float g = x * rsq;
-    return fma_(fma_(-g, g, x), 0.5f * rsq, g);
-}
-PTD float rsqrt_approx(float x) {
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-PTD float sqrt_in_range(float x) { return sqrt_from(x, rsqrt_approx(x)); }
-// 1 / b for any b
-PTD float rcp(float b) {
-    const float m = fabsf(b);
-    if (m >= 0x1p-100f && m <= 0x1p100f) return rcp_in_range(b);
-    return 1.0f / b;
-}
-
 PTD float fifth_power(float x) { return x * x * x * x * x; }
 
 // fresnel_exact, trace.slang:330-341, with ior2 = ior * ior given
 PTD float fresnel_exact_sq(float ior, float ior2, float cos_i) {
     const float s = fma_(-cos_i, cos_i, 1.0f) / ior2;
     if (s >= 1.0f) return 1.0f;
-    const float cos_t = sqrtf(1.0f - s);
+    const float cos_t = sqrt_(1.0f - s);
     const float rs = fma_(-ior, cos_t, cos_i) / fma_(ior, cos_t, cos_i);
     const float rp = fma_(-ior, cos_i, cos_t) / fma_(ior, cos_i, cos_t);
     return 0.5f * (rs * rs + rp * rp);
@@ -319,7 +347,7 @@ PTD float fresnel_exact(float ior, float cos_i) { return fresnel_exact_sq(ior, i
 
 // ggx_lambda, trace.slang:347-352, with the squared roughnesses ax2 = a.x * a.x, ay2 = a.y * a.y given
 PTD float ggx_lambda_sq(f3 v, float ax2, float ay2) {
-    return fma_(0.5f, sqrtf(1.0f + (ax2 * v.x * v.x + ay2 * v.y * v.y) / (v.z * v.z)), -0.5f);
+    return fma_(0.5f, sqrt_(1.0f + (ax2 * v.x * v.x + ay2 * v.y * v.y) / (v.z * v.z)), -0.5f);
 }
 PTD float ggx_lambda(f3 v, f2 a) { return ggx_lambda_sq(v, a.x * a.x, a.y * a.y); }
 
@@ -328,7 +356,7 @@ PTD float ggx_lambda(f3 v, f2 a) { return ggx_lambda_sq(v, a.x * a.x, a.y * a.y)
 // ww1 = 1 + ww.z
 PTD f3 sample_vndf_ww(f3 ww, float ww1, f2 a, float r, float sin_2pr, float cos_2pr) {
     const float z = fma_(1.0f - r, ww1, -ww.z);
-    const float sin_theta = sqrtf(saturate(fma_(-z, z, 1.0f)));
+    const float sin_theta = sqrt_(saturate(fma_(-z, z, 1.0f)));
     const float x = sin_theta * cos_2pr;
     const float y = sin_theta * sin_2pr;
     const f3 h = mk(x, y, z) + ww;
@@ -366,7 +394,7 @@ PTD float specular_ior_modulated(float ior, float weight) {
     const float num = ior - 1.0f;
     const float den = ior + 1.0f;
     const float f0 = num * num / (den * den);
-    const float f0s = signf(ior - 1.0f) * sqrtf(fminf(weight * f0, __uint_as_float(0x3f800000u - 1u)));
+    const float f0s = signf(ior - 1.0f) * sqrt_(fminf(weight * f0, __uint_as_float(0x3f800000u - 1u)));
     return (1.0f + f0s) / (1.0f - f0s);
 }
 
@@ -498,26 +526,60 @@ PTD f3 evaluate_emission(const World& w, const pt_material& m, f2 uv) {
     return m.emission_weight * m.emission_color_and_luminance[3] * color;
 }
 
-// skybox_uv, trace.slang:467-472
-PTD f2 skybox_uv(f3 d) {
-    return {fract(fma_(ptm::atan2f_(d.z, d.x), kInv2Pi, 0.5f)), ptm::atan2f_(sqrtf(d.x * d.x + d.z * d.z), d.y) * kInvPi};
+// ptm::atan2f_ and ptm::acosf_ without their branches, which the lanes of a
+// warp take one after the other: one division, one series and selects (the
+// same bits, tests/test_gpu_fast_math.py; a direction's sky coordinates take
+// two arc tangents)
+PTD float atan2_(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const bool x_neg = (__float_as_uint(x) >> 31) != 0u;
+    const float n = fminf(ax, ay), m = fmaxf(ax, ay);
+    float z;
+    if (__builtin_expect(m >= 0x1p-60f && m <= 0x1p40f && (n >= 0x1p-60f || n == 0.0f), 1))
+        z = div_in_range(n, m);
+    else
+        z = n / m;
+    const bool big = z > 0.26794919f;
+    const float t = big ? div_in_range(fma_(z, ptm::kSqrt3, -1.0f), ptm::kSqrt3 + z) : z;
+    const float k = ptm::atan_kernel(t);
+    float a = big ? ptm::kPi6 + (k + ptm::kPi6Lo) : k;
+    a = ay > ax ? (ptm::kPio2C1 - a) + ptm::kPio2C2 : a;
+    a = x_neg ? (ptm::kPi - a) + ptm::kPiLo : a;
+    a = ax == ay ? (x_neg ? 3.0f * 0.5f * ptm::kPio2C1 : 0.5f * ptm::kPio2C1) : a;
+    a = ax == 0.0f ? ptm::kPio2C1 : a;
+    a = ay == 0.0f ? (x_neg ? ptm::kPi : 0.0f) : a;
+    a = y != y || x != x ? __uint_as_float(0x7fc00000u) : copysignf(a, y);
+    return a;
+}
+PTD float acos_(float x) {
+    const float ax = fabsf(x);
+    const bool big = ax > 0.5f;
+    const float s2 = (1.0f - ax) * 0.5f;  // 0, or at least 2^-25 where it is used
+    const float k = ptm::asin_kernel(big ? sqrt_from(s2, rsqrt_approx(fmaxf(s2, 0x1p-40f))) : x);
+    const float r = 2.0f * k;
+    const float far = x < 0.0f ? (ptm::kPi - r) + ptm::kPiLo : r;
+    const float a = big ? far : (ptm::kPio2C1 - k) + ptm::kPio2C2;
+    return ax <= 1.0f ? a : __uint_as_float(0x7fc00000u);
 }
 
-// evaluate_skybox, trace.slang:473-475
-PTD f3 evaluate_skybox(const World& w, f3 d) { return skybox_bilinear(w, skybox_uv(d)) * w.sky_u.average_luminance; }
+// skybox_uv, trace.slang:467-472
+PTD f2 skybox_uv(f3 d) {
+    return {fract(fma_(atan2_(d.z, d.x), kInv2Pi, 0.5f)), atan2_(sqrt_(d.x * d.x + d.z * d.z), d.y) * kInvPi};
+}
+
+// evaluate_skybox, trace.slang:473-475, at a direction's skybox_uv
+PTD f3 evaluate_skybox(const World& w, f2 uv) { return skybox_bilinear(w, uv) * w.sky_u.average_luminance; }
 
 // skybox_texel_solid_angle, trace.slang:476-481
 PTD float skybox_texel_solid_angle(const World& w, uint32_t row) {
-    const float step = kPi / (float)w.sky_u.height;
     const uint32_t other = w.sky_u.height - 1u - row;
     const uint32_t pole_row = row < other ? row : other;
-    return (kTwoPi / (float)w.sky_u.width) * 2.0f * ptm::sinf_(((float)pole_row + 0.5f) * step) * ptm::sinf_(0.5f * step);
+    return w.sky_k.width_term * ptm::sinf_(((float)pole_row + 0.5f) * w.sky_k.step) * w.sky_k.sin_half_step;
 }
 
-// skybox_light_pdf, trace.slang:482-489
-PTD float skybox_light_pdf(const World& w, f3 d, float prob) {
+// skybox_light_pdf, trace.slang:482-489, at a direction's skybox_uv
+PTD float skybox_light_pdf(const World& w, f2 uv, float prob) {
     if (prob <= 0.0f) return 0.0f;
-    const f2 uv = skybox_uv(d);
     uint32_t px = to_u32(uv.x * (float)w.sky_u.width);
     uint32_t py = to_u32(uv.y * (float)w.sky_u.height);
     if (px > w.sky_u.width - 1u) px = w.sky_u.width - 1u;
@@ -575,14 +637,14 @@ PTD LightSample sample_light(const World& w, f3 origin, Rng<kRec>& rng, Counters
         const pt_scene_alias_entry cand = w.scene_alias[slot];
         const pt_scene_alias_entry entry = w.scene_alias[rng() < cand.threshold ? slot : cand.alias_index];
         const Tri t = load_tri(w, entry.triangle_index);
-        const float root = sqrtf(rng());
+        const float root = sqrt_(rng());
         const float u = 1.0f - root;
         const float v = root * (1.0f - rng());
         const float wb = 1.0f - u - v;
         const f3 delta = u * t.v0 + v * t.v1 + wb * t.v2 - origin;
         const float d2 = dot(delta, delta);
         if (d2 <= 0.0f) return r;
-        r.distance = sqrtf(d2);
+        r.distance = sqrt_(d2);
         r.direction = delta / r.distance;
         r.triangle_index = (int32_t)entry.triangle_index;
         r.pdf = triangle_light_pdf(w, entry.triangle_index, r.direction, d2, p0 * entry.selection_probability);
@@ -598,21 +660,21 @@ PTD LightSample sample_light(const World& w, f3 origin, Rng<kRec>& rng, Counters
         const pt_skybox_alias_entry cand = w.sky_alias[slot];
         const uint32_t index = rng() < cand.threshold ? slot : cand.alias_index;
         const uint32_t row = index / W, column = index % W;
-        const float phi = (((float)column + rng()) / (float)W - 0.5f) * kTwoPi;
+        const float phi = (div_by((float)column + rng(), (float)W, w.sky_k.rcp_width) - 0.5f) * kTwoPi;
         const bool north = row < H / 2u;
         const uint32_t pole_row = north ? row : H - 1u - row;
-        const float half_step = 0.5f * kPi / (float)H;
-        const float a = ptm::sinf_((float)pole_row * half_step);
-        const float b = ptm::sinf_((float)(pole_row + 1u) * half_step);
+        const float a = ptm::sinf_((float)pole_row * w.sky_k.half_step);
+        const float b = ptm::sinf_((float)(pole_row + 1u) * w.sky_k.half_step);
         const float shs = mix(a * a, b * b, rng());
         const float cos_theta = 1.0f - 2.0f * shs;
-        const float sin_theta = 2.0f * sqrtf(fmaxf(0.0f, shs * (1.0f - shs)));
+        const float sin_theta = 2.0f * sqrt_(fmaxf(0.0f, shs * (1.0f - shs)));
         float sin_phi, cos_phi;
         ptm::sincosf_(phi, &sin_phi, &cos_phi);
         r.direction = mk(sin_theta * cos_phi, north ? cos_theta : -cos_theta, sin_theta * sin_phi);
         r.distance = kFltMax;
-        r.pdf = skybox_light_pdf(w, r.direction, p1);
-        r.emission = evaluate_skybox(w, r.direction);
+        const f2 uv = skybox_uv(r.direction);
+        r.pdf = skybox_light_pdf(w, uv, p1);
+        r.emission = evaluate_skybox(w, uv);
     }
     return r;
 }
@@ -740,8 +802,8 @@ PTD bool triangle_test(const Tri& t, f3 o, const Shear& s, float* t_out, float* 
 // E_FON_exact, trace.slang:318-323
 // with af = 1 / (1 + 0.28779340921 r) given
 PTD float e_fon_af(float mu, float r, float af) {
-    const float si = sqrtf(fma_(-mu, mu, 1.0f));
-    const float g = si * (ptm::acosf_(mu) - si * mu) + 0x1.555556p-1f * ((si / mu) * (1.0f - (si * si * si)) - si);
+    const float si = sqrt_(fma_(-mu, mu, 1.0f));
+    const float g = si * (acos_(mu) - si * mu) + 0x1.555556p-1f * ((si / mu) * (1.0f - (si * si * si)) - si);
     return af + r * af * kInvPi * g;
 }
 PTD float e_fon_exact(float mu, float r) { return e_fon_af(mu, r, 1.0f / fma_(0.28779340921f, r, 1.0f)); }
@@ -957,8 +1019,8 @@ PTD bool dielectric_fast(const DielectricTerms& t) {
     return lo >= 1e-5f && hi <= 16.0f && dir <= 2.0f && all == all;
 }
 // dielectric_sample with divisions and roots in range, the same operations in
-// the same order.  *redo: a quantity left the range, the value is not to be
-// used.
+// the same order.  Sets *redo when a quantity left the range: the value is
+// then not to be used.
 PTD float dielectric_sample_fast(const DielectricTerms& t, float r1, float tpr, bool* redo) {
     float sn, cs;
     sincos_turn(tpr, &sn, &cs);
@@ -969,9 +1031,9 @@ PTD float dielectric_sample_fast(const DielectricTerms& t, float r1, float tpr, 
     const f3 v = mk(hh.x * t.alpha.x, hh.y * t.alpha.y, hh.z);
     const float d2 = dot(v, v);
     const f3 h = v * rcp_in_range(sqrt_in_range(d2));
-    const f3 wi = reflect(-t.wo, h);
-    // fresnel_exact, trace.slang:330-341
     const float c = dot(h, t.wo);
+    const f3 wi = 2.0f * c * h - t.wo;  // reflect(-wo, h): its dot product is -c
+    // fresnel_exact, trace.slang:330-341
     const float s = div_by(fma_(-c, c, 1.0f), t.ior2, t.rcp_ior2);
     const float cos_t = sqrt_in_range(1.0f - s);
     const float den_s = fma_(t.ior, cos_t, c), den_p = fma_(t.ior, c, cos_t);
@@ -984,10 +1046,10 @@ PTD float dielectric_sample_fast(const DielectricTerms& t, float r1, float tpr, 
     const float tan2 = div_in_range(t.ax2 * wi.x * wi.x + t.ay2 * wi.y * wi.y, wz2);
     const float a = f * t.opl;
     const float term = div_in_range(a, t.opl + fma_(0.5f, sqrt_in_range(1.0f + tan2), -0.5f));
-    const bool none = wi.z <= 0.0f;
-    *redo = d2 < 0x1p-60f || (!none && (wz2 < 0x1p-60f || (!total && fminf(fabsf(den_s), fabsf(den_p)) < 0x1p-20f) ||
-                                        (a > 0.0f && a < 0x1p-80f)));
-    return none ? 0.0f : term;
+    // (the denominators of a totally reflected sample are NaN and compare false,
+    // its root being negative, or those of a valid one)
+    *redo |= fminf(d2, wz2) < 0x1p-60f || fminf(fabsf(den_s), fabsf(den_p)) < 0x1p-20f || (a > 0.0f && a < 0x1p-80f);
+    return wi.z <= 0.0f ? 0.0f : term;
 }
 
 // estimate_e_dielectric, trace.slang:396-411: two thirds of the shading
@@ -1011,33 +1073,40 @@ PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_co
     t.alpha = alpha;
     t.ax2 = alpha.x * alpha.x;
     t.ay2 = alpha.y * alpha.y;
-    const bool fast = dielectric_fast(t);
-    const auto sample = [&](Rng<kRec>& r) {
-        const float r1 = r();
-        const float tpr = kTwoPi * r();
-        bool redo = false;
-        float term = dielectric_sample_fast(t, r1, tpr, &redo);
-        if (redo || !fast) term = dielectric_sample(t, r1, tpr);
-        return term;
-    };
-    float sum = 0.0f;
-    if (kSpread && !kRec && spread.log2 > 0u) {
-        const uint32_t start = rng.s, lanes = 1u << spread.log2;
-        const uint32_t first = (uint32_t)__ffs(spread.mask) - 1u;
-        rng.s = kRngJump.a[spread.index] * start + kRngJump.c[spread.index];
-        const uint32_t ja = kRngJump.a[lanes], jc = kRngJump.c[lanes];
+    // the samples in order: `sample(r1, tpr)` gives one's term.  The checked
+    // samples are a second loop that an estimate falls back to as a whole: as a
+    // branch inside the one loop they cost 6 % of shading and 12 KB of code.
+    const uint32_t start = rng.s;
+    const auto sum_of = [&](auto&& sample) {
+        float sum = 0.0f;
+        rng.s = start;
+        if (kSpread && !kRec && spread.log2 > 0u) {
+            const uint32_t lanes = 1u << spread.log2, first = (uint32_t)__ffs(spread.mask) - 1u;
+            uint32_t at = kRngJump.a[spread.index] * start + kRngJump.c[spread.index];
+            const uint32_t ja = kRngJump.a[lanes], jc = kRngJump.c[lanes];
 #pragma unroll 1
-        for (uint32_t i = 0; i < 16u; i += lanes) {
-            Rng<kRec> own = rng;
-            const float term = sample(own);
-            for (uint32_t k = 0; k < lanes; ++k) sum += __shfl_sync(spread.mask, term, first + k);
-            rng.s = ja * rng.s + jc;
+            for (uint32_t i = 0; i < 16u; i += lanes) {
+                uint32_t own = at;
+                const float r1 = rand_next(own);
+                const float term = sample(r1, kTwoPi * rand_next(own));
+                for (uint32_t k = 0; k < lanes; ++k) sum += __shfl_sync(spread.mask, term, first + k);
+                at = ja * at + jc;
+            }
+            rng.s = kRngJump.a[16] * start + kRngJump.c[16];
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < 16; ++i) {
+                const float r1 = rng();
+                sum += sample(r1, kTwoPi * rng());
+            }
         }
-        rng.s = kRngJump.a[16] * start + kRngJump.c[16];
-    } else {
-#pragma unroll 1
-        for (int i = 0; i < 16; ++i) sum += sample(rng);
-    }
+        return sum;
+    };
+    bool redo = !dielectric_fast(t);
+    float sum = 0.0f;
+    if (!redo) sum = sum_of([&](float r1, float tpr) { return dielectric_sample_fast(t, r1, tpr, &redo); });
+    if (kSpread && !kRec && spread.log2 > 0u) redo = __any_sync(spread.mask, redo);
+    if (__builtin_expect(redo, 0)) sum = sum_of([&](float r1, float tpr) { return dielectric_sample(t, r1, tpr); });
     return spec_color * sum / 16.0f;
 }
 

@@ -179,8 +179,9 @@ PTD void camera_ray(const World& w, uint32_t px, uint32_t py, uint32_t img_w, ui
 // escaped ray, trace.slang:887-927
 PTD void shade_miss(const World& w, uint32_t bounce, PathState& ps) {
     float mis = 1.0f;
-    if (bounce > 0u) mis = power_heuristic(ps.prev_pdf, skybox_light_pdf(w, ps.d, w.scene.light_probabilities[1]));
-    ps.color = ps.color + ps.throughput * evaluate_skybox(w, ps.d) * mis;
+    const f2 uv = skybox_uv(ps.d);
+    if (bounce > 0u) mis = power_heuristic(ps.prev_pdf, skybox_light_pdf(w, uv, w.scene.light_probabilities[1]));
+    ps.color = ps.color + ps.throughput * evaluate_skybox(w, uv) * mis;
 }
 
 // a shadow ray produced by next-event estimation
@@ -358,15 +359,15 @@ PTD bool shade_hit(const World& w, uint32_t bounce, uint32_t max_bounces, PathSt
         wi = reflect(-wo, sample_vndf_sc(wo, b.alpha, r1, sin_2pr, cos_2pr));
     } else if (r1 < b.p_u) {
         const float u1 = r1 / b.p_u;
-        const float sin_theta = sqrtf(1.0f - u1 * u1);
+        const float sin_theta = sqrt_(1.0f - u1 * u1);
         wi = mk(sin_theta * cos_2pr, sin_theta * sin_2pr, u1);
     } else {
         const float u1 = (r1 - b.p_u) / b.p_c;
-        const float R = sqrtf(u1);
+        const float R = sqrt_(u1);
         const float y = R * sin_2pr;
         const float s = fma_(0.5f, rsqrt_(fma_(b.ld, b.ld, 1.0f)), 0.5f);
-        const float x = -mix(sqrtf(fma_(-y, y, 1.0f)), R * cos_2pr, s);
-        const f3 wh = mk(x, y, sqrtf(fmaxf(1.0f - (x * x + y * y), 0.0f)));
+        const float x = -mix(sqrt_(fma_(-y, y, 1.0f)), R * cos_2pr, s);
+        const f3 wh = mk(x, y, sqrt_(fmaxf(1.0f - (x * x + y * y), 0.0f)));
         const f3 wu = mk(b.la * wh.x + b.lb * wh.z, b.lc * wh.y, b.ld * wh.x + wh.z);
         wi = normalize(wu.x * b.bx + wu.y * b.by + wu.z * mk(0.0f, 0.0f, 1.0f));
     }

@@ -978,6 +978,7 @@ extern "C" int pt_trace_noalloc(const pt_device_world* world, const pt_trace_par
     w.sky_alias = world->skybox_aliases;
     w.scene_alias = world->scene_aliases;
     w.sky_u = world->skybox_uniforms;
+    w.sky_k = ptd::sky_terms(w.sky_u);
     w.scene = world->scene_uniforms;
     w.camera = world->camera;
     w.srgb_lut = reinterpret_cast<const float*>(base + kNoAllocLutOffset);

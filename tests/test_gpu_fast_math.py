@@ -27,22 +27,48 @@ __global__ void one_argument(unsigned long long* bad) {
     for (int e = -120; e <= 120; ++e) {
         const float b = make(e, m);
         if (!same(rcp_in_range(b), 1.0f / b) || !same(rcp_in_range(-b), 1.0f / -b)) atomicAdd(bad, 1ull);
-        if (!same(rcp(b), 1.0f / b) || !same(rcp(-b), 1.0f / -b)) atomicAdd(bad, 1ull);
     }
     for (int e = -96; e <= 126; ++e)
         if (!same(sqrt_in_range(make(e, m)), sqrtf(make(e, m)))) atomicAdd(bad + 1, 1ull);
     for (int e = -96; e <= 100; ++e)
-        if (!same(rcp_in_range(sqrt_in_range(make(e, m))), rsqrt_(make(e, m)))) atomicAdd(bad + 2, 1ull);
+        if (!same(rcp_in_range(sqrt_in_range(make(e, m))), 1.0f / sqrtf(make(e, m)))) atomicAdd(bad + 2, 1ull);
 }
 
-// rcp() takes anything
-__global__ void any_reciprocal(unsigned long long* bad) {
+__device__ bool agree(float a, float b) { return same(a, b) || (a != a && b != b); }
+
+// the functions that take any argument, on every float
+__global__ void any_argument(unsigned long long* bad) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t k = 0; k < 256; ++k) {
         const float b = __uint_as_float(i * 256u + k);
-        const float got = rcp(b), want = 1.0f / b;
-        if (!same(got, want) && !(got != got && want != want)) atomicAdd(bad + 3, 1ull);
+        if (!agree(rcp(b), 1.0f / b)) atomicAdd(bad + 3, 1ull);
+        if (!agree(ptd::sqrt_(b), sqrtf(b)) || !agree(rsqrt_(b), 1.0f / sqrtf(b))) atomicAdd(bad + 3, 1ull);
+        if (!agree(acos_(b), ptm::acosf_(b))) atomicAdd(bad + 3, 1ull);
+        const float turn = fabsf(b);
+        float s, c, s1, c1;
+        if (turn <= kTwoPi) {
+            sincos_turn(turn, &s, &c);
+            ptm::sincosf_(turn, &s1, &c1);
+            if (!same(s, s1) || !same(c, c1)) atomicAdd(bad + 3, 1ull);
+        }
+        // arc tangents: against a second argument of every kind
+        const uint32_t r = mixed(((uint64_t)i << 8) + k);
+        const float others[6] = {__uint_as_float(r), b, 0.0f, -0.0f, __uint_as_float(0x7f800000u), (float)(r >> 8) * 0x1p-23f - 1.0f};
+        for (float o : others) {
+            if (!agree(atan2_(b, o), ptm::atan2f_(b, o)) || !agree(atan2_(o, b), ptm::atan2f_(o, b)) ||
+                !agree(atan2_(b, -o), ptm::atan2f_(b, -o)))
+                atomicAdd(bad + 3, 1ull);
+        }
     }
+}
+
+// bytes as unorm, the sky's column over its width
+__global__ void constants(unsigned long long* bad) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < 256u && !same(div_by((float)i, 255.0f, 1.0f / 255.0f), (float)i / 255.0f)) atomicAdd(bad + 4, 1ull);
+    const uint32_t width = 1u + mixed(i) % 16384u, column = mixed(~i) % width;
+    const float a = (float)column + unit(i), w = (float)width;
+    if (!same(div_by(a, w, 1.0f / w), a / w)) atomicAdd(bad + 4, 1ull);
 }
 
 // quotients: random significands, and the hard ones (divisors of ones, numerators next to the divisor or to 1 or 2)
@@ -89,7 +115,7 @@ __global__ void samples(unsigned long long* bad, unsigned long long* count) {
         const float fast = dielectric_sample_fast(d, r1, tpr, &redo), want = dielectric_sample(d, r1, tpr);
         used += 1u;
         redone += redo;
-        if (!redo && !same(fast, want) && !(fast != fast && want != want)) atomicAdd(bad + 5, 1ull);
+        if (!redo && !agree(fast, want)) atomicAdd(bad + 5, 1ull);
     }
     atomicAdd(count, (unsigned long long)used);
     atomicAdd(count + 1, (unsigned long long)redone);
@@ -99,7 +125,8 @@ int main() {
     unsigned long long *bad, h[8] = {0};
     if (cudaMalloc(&bad, 64) != cudaSuccess || cudaMemset(bad, 0, 64) != cudaSuccess) return 2;
     one_argument<<<(1 << 23) / 256, 256>>>(bad);
-    any_reciprocal<<<(1 << 24) / 256, 256>>>(bad);
+    any_argument<<<(1 << 24) / 256, 256>>>(bad);
+    constants<<<1 << 14, 256>>>(bad);
     quotients<<<1 << 11, 256>>>(bad);
     samples<<<1 << 10, 256>>>(bad, bad + 6);
     if (cudaMemcpy(h, bad, 64, cudaMemcpyDeviceToHost) != cudaSuccess) return 3;
