@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCK
     const uint32_t rays = cnt[kCntRays], shadows = kAlpha ? 0u : cnt[kCntShadows];
     {
         const Stage st = stage_of(b.q, round);
-        RayOf<false, kAlpha, false, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
+        RayOf<false, kAlpha, kFindClosest, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
         uint32_t slot = 0;
         traverse_queue(
             QueueShare(0u, rays, rays + shadows), visits, ray, stack, istack,
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCK
     }
     if constexpr (!kAlpha) {
         if (shadows == 0u) return;
-        RayOf<false, false, true, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
+        RayOf<false, false, kFindAny, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
         uint32_t path = 0;
         f3 contribution = mk(0.0f, 0.0f, 0.0f);
         traverse_queue(

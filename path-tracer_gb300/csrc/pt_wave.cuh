@@ -56,6 +56,7 @@ constexpr uint32_t kCntHits = 3;         // hit list length
 constexpr uint32_t kCntMisses = 4;       // miss list length
 constexpr uint32_t kCntShadowFetch = 5;  // shadow rays taken
 constexpr uint32_t kCntSorted = 6;       // 1: hit_sorted holds the round's hits
+constexpr uint32_t kCntTail = 7;         // hits taken by finish_paths beyond those dealt
 // rounds 0 .. max_bounces, and the empty one after the last
 constexpr uint32_t kCounterWords = kRoundCounters * (PT_MAX_BOUNCES_LIMIT + 2u);
 PTD uint32_t* round_counters(const Queues& q, uint32_t round) { return q.cnt + kRoundCounters * round; }
@@ -132,6 +133,8 @@ constexpr uint32_t kWideLeafMerge = PT_WIDE_LEAF_MERGE;
 #endif
 constexpr int kExtendThreads = PT_EXTEND_THREADS;
 constexpr int kShadeThreads = PT_SHADE_THREADS;
+constexpr int kTailThreads = 512;  // one block per SM, 4 warps a scheduler (see finish_paths)
+constexpr uint32_t kTailSmemStack = 5;  // its packed stacks' shared entries: 40 KB (3 and 8: the same times)
 // entries at the top of each traversal lane's stack kept in shared memory
 #ifndef PT_SMEM_STACK
 #define PT_SMEM_STACK 8
@@ -281,8 +284,13 @@ PTD bool boxless(f3 nod) {
     return !(fabsf(nod.x) < inf) && !(fabsf(nod.y) < inf) && !(fabsf(nod.z) < inf);
 }
 
-// One ray's traversal (trace.slang:764-884 closest hit, or 614-717 any hit
-// when kShadow) on the binary nodes as uploaded: visit() one interior node,
+// What a traversal looks for (the template argument kFind): the closest hit
+// (trace.slang:764-884), any hit (614-717), or either by the ray: a ray whose
+// light_tri is kClosestRay looks for the closest.
+constexpr int kFindClosest = 0, kFindAny = 1, kFindEither = 2;
+constexpr int32_t kClosestRay = -2;
+
+// One ray's traversal (closest hit or any hit) on the binary nodes as uploaded: visit() one interior node,
 // test() one triangle of a leaf; traverse_queue() decides when each runs.
 // The deferred stack holds the (left_first, tri_count) of each node, so a pop
 // needs no memory access.  A ray's visits and tests happen in exactly the
@@ -296,7 +304,7 @@ PTD bool boxless(f3 nod) {
 // triangle can be nearer, whatever is visited).  Only when all three axes are
 // NaN does it differ, so such a ray (never accepted by the reference either:
 // each axis then rejects or is NaN) gets the limit -1, which rejects all.
-template <bool kRec, bool kAlpha, bool kShadow, bool kTri36, class Scene>
+template <bool kRec, bool kAlpha, int kFind, bool kTri36, class Scene>
 struct BinaryRay {
     static constexpr int kVisitKeep = PT_VISIT_KEEP, kTestLeave = PT_TEST_LEAVE, kRefillAt = PT_REFILL_AT;
     Scene sc;
@@ -309,6 +317,7 @@ struct BinaryRay {
     Counters c;
     Rec<kRec> rec;
 
+    PTD bool any_hit() const { return kFind == kFindAny || (kFind == kFindEither && light_tri != kClosestRay); }
     PTD explicit BinaryRay(Scene scene) : sc(scene), todo(kIdle) {}
     PTD bool busy() const { return todo >= 0; }
     PTD bool at_node() const { return todo == 0; }
@@ -333,7 +342,7 @@ struct BinaryRay {
         if constexpr (kRec) {
             rec.c = &c;
             rng.rec.c = &c;
-            if constexpr (kShadow) {
+            if constexpr (kFind == kFindAny) {
                 rec.shadow = true;
                 c.shadow_rays += 1;
             } else {
@@ -401,7 +410,7 @@ struct BinaryRay {
         lf += 1u;
         todo -= 1;
         bool skip = false;
-        if constexpr (kShadow) skip = (int32_t)tri == light_tri;
+        if constexpr (kFind != kFindClosest) skip = (int32_t)tri == light_tri;
         if (!skip) {
             rec.tri();
             Tri tv;
@@ -414,7 +423,7 @@ struct BinaryRay {
                 bool counts = true;
                 if constexpr (kAlpha) counts = !passes_through(sc.w(), tri, v, wb, rng);
                 if (counts) {
-                    if constexpr (kShadow) {
+                    if (any_hit()) {
                         hit = 1;
                         todo = kFinished;
                         return;
@@ -609,7 +618,7 @@ struct PackedStack {
 // fma(a, rp, fma(b, rn, nod)) is the distance of a or b, with one rounding
 // (the other product is an exact 0), which spares the ALU pipe, the busiest
 // one (half rate), a select.
-template <bool kAlpha, bool kShadow, class Scene>
+template <bool kAlpha, int kFind, class Scene>
 struct PackedRay {
     static constexpr int kVisitKeep = PT_VISIT_KEEP, kTestLeave = PT_TEST_LEAVE, kRefillAt = PT_REFILL_AT;
     Scene sc;
@@ -621,6 +630,7 @@ struct PackedRay {
     Shear s;
     Rng<false> rng;
 
+    PTD bool any_hit() const { return kFind == kFindAny || (kFind == kFindEither && light_tri != kClosestRay); }
     PTD explicit PackedRay(Scene scene) : sc(scene), ref(kRefIdle) {}
     PTD bool busy() const { return ref < kRefFinished; }
     PTD bool at_node() const { return ((ref | oct) & 0x78u) == 0u; }
@@ -705,12 +715,12 @@ struct PackedRay {
             const uint32_t tri = ref >> 7;
             ref += (1u << 7) - (1u << 3);  // the next triangle, one fewer left
             float t, v, wb;
-            if (!(kShadow && (int32_t)tri == light_tri) &&
+            if (!(kFind != kFindClosest && (int32_t)tri == light_tri) &&
                 triangle_test(load_tri4(sc.tri4(), tri), o, s, &t, &v, &wb) && t > 0.0f && t <= limit) {
                 bool counts = true;
                 if constexpr (kAlpha) counts = !passes_through(sc.w(), tri, v, wb, rng);
                 if (counts) {
-                    if constexpr (kShadow) {
+                    if (any_hit()) {
                         hit = 1;
                         ref = kRefFinished;
                         return;
@@ -849,7 +859,7 @@ PTD unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned
     return d;
 }
 
-template <bool kShadow, class Scene>
+template <int kFind, class Scene>
 struct WideRay {
     static constexpr int kVisitKeep = PT_WIDE_VISIT_KEEP, kTestLeave = PT_WIDE_TEST_LEAVE, kRefillAt = PT_WIDE_REFILL_AT;
     Scene sc;
@@ -863,6 +873,7 @@ struct WideRay {
     uint32_t node, list, lf, sp;
     Rng<false> rng;  // carried through (no alpha draws in the wide form)
 
+    PTD bool any_hit() const { return kFind == kFindAny || (kFind == kFindEither && light_tri != kClosestRay); }
     PTD explicit WideRay(Scene scene) : sc(scene), todo(kIdle) {}
     PTD bool busy() const { return todo >= 0; }
     PTD bool at_node() const { return todo == 0; }
@@ -1024,11 +1035,11 @@ struct WideRay {
         const uint32_t tri = lf;
         lf += 1u;
         todo -= 1;
-        if (kShadow && (int32_t)tri == light_tri) return;
+        if (kFind != kFindClosest && (int32_t)tri == light_tri) return;
         float t, v, wb;
         if (!triangle_test(load_tri4(sc.tri4(), tri), o, s, &t, &v, &wb)) return;
         if (t > 0.0f && t < limit) {
-            if constexpr (kShadow) {
+            if (any_hit()) {
                 hit = 1;
                 todo = kFinished;
             } else {
@@ -1037,7 +1048,7 @@ struct WideRay {
                 hv = v;
                 hw = wb;
             }
-        } else if (!kShadow && t == limit && hit >= 0 && binary_first(sc.f(), o, d, tri, (uint32_t)hit)) {
+        } else if (!any_hit() && t == limit && hit >= 0 && binary_first(sc.f(), o, d, tri, (uint32_t)hit)) {
             // an exact tie: keep the triangle the binary traversal finds first
             hit = (int32_t)tri;
             hv = v;
@@ -1151,16 +1162,16 @@ PTD uint32_t fetch_entries(uint32_t* fetch, uint32_t want) {
 // The traversal of a kernel: the 8-wide BVH of the precision form, the packed
 // BVH, or the uploaded nodes (recording kernels, pt_trace_noalloc, and scenes
 // that the packed form cannot hold).
-template <bool kRec, bool kAlpha, bool kShadow, bool kTri36, bool kWide, bool kPacked, class Scene>
+template <bool kRec, bool kAlpha, int kFind, bool kTri36, bool kWide, bool kPacked, class Scene>
 using RayOf = typename std::conditional<
-    kWide, WideRay<kShadow, Scene>,
-    typename std::conditional<kPacked, PackedRay<kAlpha, kShadow, Scene>,
-                              BinaryRay<kRec, kAlpha, kShadow, kTri36, Scene>>::type>::type;
+    kWide, WideRay<kFind, Scene>,
+    typename std::conditional<kPacked, PackedRay<kAlpha, kFind, Scene>,
+                              BinaryRay<kRec, kAlpha, kFind, kTri36, Scene>>::type>::type;
 
 // its stack, with the shared memory of one block
-template <uint32_t kThreads, bool kWide, bool kPacked>
+template <uint32_t kThreads, bool kWide, bool kPacked, uint32_t kPackedShared = kPackedSmemStack>
 struct BlockStack {
-    static constexpr uint32_t kShared = kWide ? kWideSmemStack : kPacked ? kPackedSmemStack : kSmemStack;
+    static constexpr uint32_t kShared = kWide ? kWideSmemStack : kPacked ? kPackedShared : kSmemStack;
     using Lane = typename std::conditional<kPacked, PackedStack<kThreads, kShared>, LaneStack<kThreads, kShared>>::type;
     typename std::conditional<kPacked, float4, uint2>::type top[kShared * kThreads];
     PTD void bind(Lane& lane) {
@@ -1440,6 +1451,153 @@ PTD void traverse_queue(const QueueShare& share, uint32_t max_visits, Ray& ray, 
             m = __ballot_sync(0xffffffffu, ray.at_leaf());
             if (__popc(m) <= Ray::kTestLeave) break;
         }
+    }
+}
+
+// The same without a queue: the rays that the warp's lanes hold, to their ends.
+template <class Ray, class S>
+PTD void traverse_warp(Ray& ray, S& stack) {
+    for (;;) {
+        const int busy = __popc(__ballot_sync(0xffffffffu, ray.busy()));
+        if (busy == 0) return;
+        const int keep = max(1, (busy * Ray::kVisitKeep) >> 5), leave = busy >> 3;
+        unsigned m;
+        do {
+            if (ray.at_node()) ray.visit(stack, nullptr);
+            if (ray.at_node()) ray.visit(stack, nullptr);
+            m = __ballot_sync(0xffffffffu, ray.at_node());
+        } while (__popc(m) >= keep);
+        m = __ballot_sync(0xffffffffu, ray.at_leaf());
+        while (m != 0u) {
+            if (ray.at_leaf()) ray.test(stack, nullptr);
+            m = __ballot_sync(0xffffffffu, ray.at_leaf());
+            if (__popc(m) <= leave) break;
+        }
+    }
+}
+
+// The paths of a round, from the shading of its hits and misses to their ends,
+// without a launch between their rounds.  A round of few rays takes as long as
+// its longest ray, and the launches of a round of 19,200 paths 33 us; here a
+// path waits only for those of its block.
+//
+// A path has 2 to 16 lanes, as many as leave every path its lanes: they shade
+// its hit together (see estimate_e_dielectric), then the first traces its next
+// ray while the second traces its shadow ray, whose light is added before the
+// next hit's emission, as in the rounds.  A group of lanes takes another path
+// of the round when its own ends.  The block shades together: its warps, 4 a
+// scheduler, would else each fetch the 40 KB of shading instructions by
+// themselves (half of all stalls; 160x120 paths of the room 276 us without the
+// barrier, 260 with one of each scheduler's warps, 241 with this one).
+// 128 registers, 16 warps an SM; 24 warps of 80 registers were slower.
+// `env` gives a path's scene, world and bounces; all threads of the block.
+template <bool kAlpha, class Ray, class S, class Env>
+PTD void finish_paths(const Env& env, const Queues& q, uint32_t first_round, Ray& ray, S& stack) {
+    const Stage st = stage_of(q, first_round);
+    uint32_t* const cnt = round_counters(q, first_round);
+    const uint32_t hits = cnt[kCntHits], misses = cnt[kCntMisses];
+    const uint32_t* list = cnt[kCntSorted] ? q.hit_sorted : q.hit_list;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < misses; j += gridDim.x * blockDim.x) {
+        const uint32_t slot = q.miss_list[j];
+        const float4 o4 = st.o[slot], d4 = st.d[slot], t4 = st.T[slot];
+        const uint32_t path = __float_as_uint(o4.w);
+        const float4 c4 = q.color[path];
+        PathState ps;
+        ps.d = mk(d4.x, d4.y, d4.z);
+        ps.throughput = mk(t4.x, t4.y, t4.z);
+        ps.prev_pdf = t4.w;
+        ps.color = mk(c4.x, c4.y, c4.z);
+        shade_miss(env.world(path), first_round, ps);
+        q.color[path] = make_float4(ps.color.x, ps.color.y, ps.color.z, 0.0f);
+    }
+    __syncwarp();
+    const unsigned lane = lane_id();
+    const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+    uint32_t log2 = 4u;
+    while (log2 > 1u && (warps << (5u - log2)) < hits) log2 -= 1u;
+    const uint32_t share = 32u >> log2, dealt = warps * share;
+    Spread spread;
+    spread.log2 = log2;
+    spread.index = lane & ((1u << log2) - 1u);
+    spread.mask = ((1u << (1u << log2)) - 1u) << (lane - spread.index);
+    const bool leads = spread.index == 0u;
+    const unsigned leader = lane - spread.index;
+    const unsigned before = (1u << leader) - 1u;
+
+    bool has = false, alive = false;
+    PathState ps;
+    ShadowRay sr;
+    sr.valid = false;
+    uint32_t path = 0, round = 0, hit = 0;
+    float ht = 0.0f, hv = 0.0f, hw = 0.0f;
+    Rng<false> rng;
+    rng.s = 0u;
+    const auto load = [&](uint32_t i) {
+        has = alive = i < hits;
+        if (!has) return;
+        const uint32_t slot = list[i];
+        const float4 o4 = st.o[slot], d4 = st.d[slot], t4 = st.T[slot], h4 = q.hit[slot];
+        path = __float_as_uint(o4.w);
+        const float4 c4 = q.color[path];
+        ps.o = mk(o4.x, o4.y, o4.z);
+        ps.d = mk(d4.x, d4.y, d4.z);
+        ps.throughput = mk(t4.x, t4.y, t4.z);
+        ps.prev_pdf = t4.w;
+        ps.color = mk(c4.x, c4.y, c4.z);
+        rng.s = __float_as_uint(d4.w);
+        ht = h4.x;
+        hit = __float_as_uint(h4.y);
+        hv = h4.z;
+        hw = h4.w;
+        round = first_round;
+    };
+    load(((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * share + (lane >> log2));
+    bool more = dealt < hits;
+    for (;;) {
+        if (more) {
+            const unsigned idle = __ballot_sync(0xffffffffu, !has && leads);
+            const uint32_t want = (uint32_t)__popc(idle);
+            if (want != 0u) {
+                uint32_t base = 0;
+                if (lane == 0u) base = atomicAdd(cnt + kCntTail, want);
+                base = dealt + __shfl_sync(0xffffffffu, base, 0);
+                if (!has) load(base + (uint32_t)__popc(idle & before));
+                more = base + want < hits;
+            }
+        }
+        if (!__syncthreads_or(has)) break;
+        __syncwarp();
+        if (alive) alive = shade_hit<false, kAlpha, true>(env.world(path), round, env.max_bounces(path), ps, ht, hit, hv, hw, rng, nullptr, &sr, spread);
+        __syncwarp();
+        round += 1u;
+        ray.set_idle();
+        const bool shadow = !kAlpha && sr.valid && spread.index == 1u, extend = alive && leads;
+        if (extend || shadow) {
+            env.enter(ray, path);
+            ray.rng.s = rng.s;
+            ray.init(extend ? ps.o : sr.o, extend ? ps.d : sr.d, extend ? kFltMax : sr.dist, extend ? kClosestRay : sr.light_tri, stack);
+        }
+        traverse_warp(ray, stack);
+        if constexpr (!kAlpha) {
+            const int32_t blocked = __shfl_sync(0xffffffffu, ray.hit, leader + 1u);
+            if (sr.valid && blocked != 1) ps.color = ps.color + sr.contribution;
+            sr.valid = false;
+        }
+        const int32_t found = __shfl_sync(0xffffffffu, ray.hit, leader);
+        ht = __shfl_sync(0xffffffffu, ray.hit_t(), leader);
+        hv = __shfl_sync(0xffffffffu, ray.hv, leader);
+        hw = __shfl_sync(0xffffffffu, ray.hw, leader);
+        if constexpr (kAlpha) rng.s = __shfl_sync(0xffffffffu, ray.rng.s, leader);
+        hit = (uint32_t)found;
+        if (alive && found == -1) {
+            shade_miss(env.world(path), round, ps);
+            alive = false;
+        }
+        if (has && !alive) {
+            if (leads) q.color[path] = make_float4(ps.color.x, ps.color.y, ps.color.z, 0.0f);
+            has = false;
+        }
+        __syncwarp();
     }
 }
 

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : P
     if constexpr (!kAlpha) shadows = (what & kTraceShadows) ? cnt[kCntShadows] : 0u;
     if (rays != 0u) {
         const Stage st = stage_of(q, round);
-        RayOf<kRec, kAlpha, false, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
+        RayOf<kRec, kAlpha, kFindClosest, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
         uint32_t slot = 0, path = 0;
         traverse_queue(
             QueueShare(0u, rays, rays + shadows), kVisits, ray, stack, istack,
@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : P
     }
     if constexpr (!kAlpha) {
         if (shadows == 0u) return;
-        RayOf<kRec, false, true, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
+        RayOf<kRec, false, kFindAny, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
         uint32_t path = 0;
         f3 contribution = mk(0.0f, 0.0f, 0.0f);
         traverse_queue(
@@ -174,10 +174,11 @@ __global__ void __launch_bounds__(kExtendThreads, kWide ? PT_WIDE_MIN_BLOCKS : P
 template <bool kRec, bool kAlpha, bool kSpread, int kThreads>
 __global__ void __launch_bounds__(kThreads, kThreads == kShadeThreads ? PT_SHADE_MIN_BLOCKS
                                                                       : PT_SHADE_MIN_BLOCKS * kShadeThreads / kThreads)
-    shade_kernel(World w, Queues q, uint32_t round, uint32_t max_bounces) {
+    shade_kernel(World w, Queues q, uint32_t round, uint32_t max_bounces, uint32_t tail_hits) {
     after_previous();
     const Stage st = stage_of(q, round);
     uint32_t* const cnt = round_counters(q, round);
+    if (tail_hits != 0u && cnt[kCntHits] <= tail_hits) return;  // finished by the tail kernel
     const ShadeRange range = ShadeRange::of<kSpread>(q, cnt);
     const BlockTurns turns(range.count());
     const uint32_t wi = threadIdx.x >> 5;
@@ -256,6 +257,31 @@ __global__ void __launch_bounds__(kThreads, kThreads == kShadeThreads ? PT_SHADE
             }
         }
     }
+}
+
+// the paths of one scene and depth (see finish_paths)
+struct TileEnv {
+    const World& w;
+    uint32_t bounces;
+    PTD const World& world(uint32_t) const { return w; }
+    PTD uint32_t max_bounces(uint32_t) const { return bounces; }
+    template <class Ray>
+    PTD void enter(Ray&, uint32_t) const {}
+};
+
+// Finishes the paths of a round that has at most `most_hits`; the round's
+// shading then does nothing, and the rounds after it are empty.
+template <bool kAlpha, bool kTri36, bool kWide, bool kPacked>
+__global__ void __launch_bounds__(kTailThreads, 1)
+    tail_kernel(World w, Fast f, Queues q, uint32_t round, uint32_t max_bounces, uint32_t most_hits) {
+    using Stacks = BlockStack<kTailThreads, kWide, kPacked, kTailSmemStack>;
+    __shared__ Stacks stacks;
+    typename Stacks::Lane stack;
+    stacks.bind(stack);
+    after_previous();
+    if (round_counters(q, round)[kCntHits] > most_hits) return;
+    RayOf<false, kAlpha, kFindEither, kTri36, kWide, kPacked, OneScene> ray(OneScene{w, f});
+    finish_paths<kAlpha>(TileEnv{w, max_bounces}, q, round, ray, stack);
 }
 
 // accumulate, trace.slang:1299-1308, samples of the group in order
@@ -377,7 +403,7 @@ __global__ void debug_intersect_wide_kernel(World w, Fast f, uint64_t n, const f
                                             const float* t_max, int32_t* hit, float* hit_t) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    WideRay<false, OneScene> ray(OneScene{w, f});
+    WideRay<kFindClosest, OneScene> ray(OneScene{w, f});
     LocalStack stack;
     ray.init(mk(origins[3 * i], origins[3 * i + 1], origins[3 * i + 2]),
              mk(directions[3 * i], directions[3 * i + 1], directions[3 * i + 2]), t_max ? t_max[i] : kFltMax, -1, stack);
@@ -600,17 +626,59 @@ struct SortCfg {
 #endif
 constexpr int kSmallShadeThreads = 128;
 
+// no hit sort in a group of at most this many paths: its sorted rounds are the
+// first few, and three launches a round cost 795 against 778 us (100k
+// triangles, 640x360x1); at 1 M paths 1200 against 1222 (10k, 481x271x8)
+#ifndef PT_UNSORTED_PATHS
+#define PT_UNSORTED_PATHS (1u << 18)
+#endif
+
+// The rounds from which a group's paths are finished by the tail kernel: from
+// `first` on when a round has at most kTailHits hits, from `always` on in any
+// case.  Up to 2^17 paths the rounds' launches and longest rays cost more than
+// their better use of lanes gives, from the start (a frame of 160x120 paths of
+// the room: 237 us from round 0, 258 from 2, 397 never; 100x70x16 of 10k
+// triangles 360, 403, 560), up to 2^18 from round 1 (640x360 of 100k triangles
+// 841 from 0, 795 from 1, 810 from 2, 1140 never).  Above that the full rounds
+// go faster as launches of their own; after round 4 Russian roulette has ended
+// most paths (256x256x16 of the room 1352 from 4, 1258 from 5, 1310 never), and
+// open scenes thin out earlier (481x271x8 of 10k triangles with coverage 1172
+// with the rule's hits, 1205 with 2^15, 1288 from round 5, 1535 never;
+// 960x540x4 of 1M triangles 3611, 4100 with 2^18, 3784 never).  Groups of over
+// 2^21 paths overlap with one another, and at 2^22 the gain is -2 to 3 %.
+// Beside other groups the tail's blocks, which fill their SMs at a third of the
+// rate, are in the way: four groups of 128x128x16 paths of the room 1605 us
+// without it, 2089 with; up to 2^16 paths a group they still gain (four of
+// 64x64x16: the room 1133 without, 939 with, 1M triangles 3061, 2397).
+constexpr uint32_t kTailHits = 1u << 17;
+struct TailRule {
+    uint32_t first = 0xffffffffu, always = 0xffffffffu;
+    static TailRule of(uint32_t paths, bool alone) {
+        TailRule r;
+        if (!alone) {
+            if (paths <= (1u << 16)) r.first = r.always = 1u;
+        } else if (paths <= (1u << 18))
+            r.first = r.always = paths <= (1u << 17) ? 0u : 1u;
+        else if (paths <= (1u << 21)) {
+            r.first = 2u;
+            r.always = 5u;
+        }
+        return r;
+    }
+};
+
 // One group of paths through raygen, max_bounces + 1 rounds of trace / (hit
 // sort) / shade, and accumulate on `stream`; the accumulation runs on
 // `acc_stream` (null: `stream`) after `done` marks the group's end there.
 // kTri36 reads the reference's 36-byte triangles instead of the padded copy.
+// `alone`: no other group is expected to run beside it.
 // `serial`: a round's shadow rays are traced right after its shading, by a
 // launch of their own (the recording kernels, whose records follow the path's
 // order, and profiling).
 template <bool kRec, bool kAlpha, bool kTri36, bool kWide, bool kPacked, class TimerF>
 cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const ptd::Queues& q,
                       const ptk::Tile& tile, const ptd::Group& g, ptk::Sinks sinks, cudaStream_t stream,
-                      TimerF&& timer, bool serial, const SortCfg& sort = SortCfg(), cudaStream_t acc_stream = nullptr,
+                      TimerF&& timer, bool alone, bool serial, const SortCfg& sort = SortCfg(), cudaStream_t acc_stream = nullptr,
                       cudaEvent_t done = nullptr) {
     using namespace ptd;
     const bool small = !kRec && g.paths <= PT_SMALL_PATHS;
@@ -627,19 +695,34 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
         return timer(cls, stream, [&] { return launch_after(tracer, trace_blocks, kExtendThreads, stream, w, f, q, round, what); });
     };
     const bool shadows = !kAlpha;
+    const TailRule rule = kRec || serial ? TailRule() : TailRule::of(g.paths, alone);
     for (uint32_t round = 0; round <= tile.max_bounces; ++round) {
         const bool both = shadows && !serial && round > 0;
         PTW_TRY(trace(PT_KC_EXTEND, round, kTraceRays | (both ? kTraceShadows : 0u)));
-        if (sort.counts && sort.min_hits <= g.paths) {
+        uint32_t tail_hits = 0u;  // rounds of at most this many hits are finished by the tail kernel
+        if constexpr (!kRec) {
+            if (round >= rule.first) {
+                const bool all = round >= rule.always;
+                const auto tail = tail_kernel<kAlpha, kTri36, kWide, kPacked>;
+                PTW_TRY(timer(PT_KC_SHADE, stream, [&] {
+                    return launch_after(tail, (uint32_t)sms, kTailThreads, stream, w, f, q, round, tile.max_bounces,
+                                        all ? 0xffffffffu : kTailHits);
+                }));
+                if (all) break;
+                tail_hits = kTailHits;
+            }
+        }
+        const uint32_t sort_hits = std::max(sort.min_hits, tail_hits + 1u);
+        if (sort.counts && sort_hits <= g.paths && g.paths > PT_UNSORTED_PATHS) {
             PTW_TRY(timer(PT_KC_SORT, stream, [&] {
                 cudaError_t e = launch_after(sort_count_kernel<PT_SORT_KEY>, (uint32_t)sms * 4u, kSortThreads, stream, w,
-                                             q, round, sort.counts, sort.min_hits, sort.tri_shift);
+                                             q, round, sort.counts, sort_hits, sort.tri_shift);
                 if (e == cudaSuccess)
                     e = launch_after(sort_scan_kernel<0>, 1u, 1024u, stream, q, round, sort.counts,
-                                     sort.counts + kSortBuckets, sort.min_hits);
+                                     sort.counts + kSortBuckets, sort_hits);
                 if (e == cudaSuccess)
                     e = launch_after(sort_scatter_kernel<PT_SORT_KEY>, (uint32_t)sms * 4u, kSortThreads, stream, w, q,
-                                     round, sort.counts + kSortBuckets, sort.min_hits, sort.tri_shift);
+                                     round, sort.counts + kSortBuckets, sort_hits, sort.tri_shift);
                 return e;
             }));
         }
@@ -648,11 +731,11 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
                 if (small) {
                     const auto spread = shade_kernel<kRec, kAlpha, true, kSmallShadeThreads>;
                     return launch_after(spread, (uint32_t)sms * resident_blocks(spread, kSmallShadeThreads),
-                                        kSmallShadeThreads, stream, w, q, round, tile.max_bounces);
+                                        kSmallShadeThreads, stream, w, q, round, tile.max_bounces, tail_hits);
                 }
             }
             return launch_after(shader, (uint32_t)sms * resident_blocks(shader, kShadeThreads), kShadeThreads, stream, w,
-                                q, round, tile.max_bounces);
+                                q, round, tile.max_bounces, tail_hits);
         }));
         // the last round's shadow rays, or every round's
         if (shadows && (serial || round == tile.max_bounces)) PTW_TRY(trace(PT_KC_SHADOW, round + 1u, kTraceShadows));
@@ -676,7 +759,7 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
 
 cudaError_t trace(Wavefront* wf, const ptd::World& w_in, const ptk::Tile& tile, uint32_t first, uint32_t samples,
                   ptk::Sinks sinks, cudaStream_t stream, const Timer& timer, uint32_t precision, bool overlap,
-                  bool serial) {
+                  bool alone, bool serial) {
     precision = effective_precision(w_in, precision, sinks.any());
     ptd::World w = w_in;
     if (precision & PT_PRECISION_HALF_ATTRIBUTES) {
@@ -765,13 +848,13 @@ cudaError_t trace(Wavefront* wf, const ptd::World& w_in, const ptk::Tile& tile, 
         cudaError_t e;
         const auto group_of = [&](auto alpha, auto wide_form, auto packed) {
             return run_group<false, decltype(alpha)::value, false, decltype(wide_form)::value, decltype(packed)::value>(
-                wf->sms, w, f, q, tile, g, sinks, gs, timer, serial, sort, as, l.done);
+                wf->sms, w, f, q, tile, g, sinks, gs, timer, alone, serial, sort, as, l.done);
         };
         using std::false_type;
         using std::true_type;
         if (record)
-            e = w.any_alpha ? run_group<true, true, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, true)
-                            : run_group<true, false, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, true);
+            e = w.any_alpha ? run_group<true, true, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, false, true)
+                            : run_group<true, false, false, false, false>(wf->sms, w, f, q, tile, g, sinks, gs, timer, false, true);
         else if (wide)
             e = group_of(false_type(), true_type(), false_type());
         else if (f.packed)
@@ -1033,8 +1116,8 @@ extern "C" int pt_trace_noalloc(const pt_device_world* world, const pt_trace_par
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto untimed = [](int, cudaStream_t, auto&& launch) { return launch(); };
     const cudaError_t e = w.any_alpha
-                              ? ptw::run_group<false, true, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed, false)
-                              : ptw::run_group<false, false, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed, false);
+                              ? ptw::run_group<false, true, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed, true, false)
+                              : ptw::run_group<false, false, true, false, false>(g_noalloc_devices[dev].sms, w, f, q, t, g, ptk::Sinks{nullptr, nullptr}, s, untimed, true, false);
     return noalloc_cuda(error, error_size, e, "trace launch");
 } catch (...) {
     std::string message;
