@@ -74,6 +74,7 @@ struct WaveBufs {
 constexpr uint32_t kMaxScenes = 256;
 constexpr uint32_t kMaxSlots = 1u << 16;
 constexpr uint32_t kRounds = PT_MAX_BOUNCES_LIMIT + 1;
+constexpr uint32_t kWaveSizes = 4;
 constexpr uint32_t kEngineSortShift = 10;  // sort bucket = triangle index / 1024
 
 // ---------------------------------------------------------------- kernels
@@ -219,10 +220,11 @@ __global__ void __launch_bounds__(kThreads, blocks_for(kWide ? PT_WIDE_MIN_BLOCK
 
 template <bool kAlpha, int kThreads = kShadeThreads>
 __global__ void __launch_bounds__(kThreads, blocks_for(PT_SHADE_MIN_BLOCKS, kShadeThreads, kThreads))
-    shade_kernel(const SceneDev* scenes, const JobDev* jobs, WaveBufs b, uint32_t bounce) {
+    shade_kernel(const SceneDev* scenes, const JobDev* jobs, WaveBufs b, uint32_t bounce, uint32_t tail_hits) {
     after_previous();
     const Stage st = stage_of(b.q, bounce);
     uint32_t* const cnt = round_counters(b.q, bounce);
+    if (tail_hits != 0u && cnt[kCntHits] <= tail_hits) return;  // finished by the tail kernel
     const ShadeRange range = ShadeRange::of<false>(b.q, cnt);
     const BlockTurns turns(range.count());
     const uint32_t wi = threadIdx.x >> 5;
@@ -282,6 +284,35 @@ __global__ void __launch_bounds__(kThreads, blocks_for(PT_SHADE_MIN_BLOCKS, kSha
             }
         }
     }
+}
+
+// each path in its job's scene, to its job's depth (see finish_paths)
+template <bool kWide>
+struct WaveEnv {
+    const SceneDev* scenes;
+    const JobDev* jobs;
+    const uint32_t* tag;
+    PTD const World& world(uint32_t path) const { return scenes[tag[path] & 0xffu].w; }
+    PTD uint32_t max_bounces(uint32_t path) const { return jobs[tag[path] >> 8].max_bounces; }
+    template <class Ray>
+    PTD void enter(Ray& ray, uint32_t path) const {
+        ray.sc = lane_scene<kWide>(scenes, tag[path] & 0xffu);
+    }
+};
+
+// Finishes the paths of a round that has at most `most_hits` (see tail_kernel
+// of trace_wavefront.cu)
+template <bool kAlpha, bool kWide, bool kPacked>
+__global__ void __launch_bounds__(kTailThreads, 1)
+    tail_kernel(const SceneDev* scenes, const JobDev* jobs, WaveBufs b, uint32_t round, uint32_t most_hits) {
+    using Stacks = BlockStack<kTailThreads, kWide, kPacked, kTailSmemStack>;
+    __shared__ Stacks stacks;
+    typename Stacks::Lane stack;
+    stacks.bind(stack);
+    after_previous();
+    if (round_counters(b.q, round)[kCntHits] > most_hits) return;
+    RayOf<false, kAlpha, kFindEither, false, kWide, kPacked, LaneScene<SceneDev>> ray(LaneScene<SceneDev>{scenes, 0u, nullptr, nullptr});
+    finish_paths<kAlpha>(WaveEnv<kWide>{scenes, jobs, b.tag}, b.q, round, ray, stack);
 }
 
 // accumulate, trace.slang:1299-1308: one block per item, samples in order;
@@ -574,8 +605,8 @@ struct pt_engine {
     ptb::WaveBufs wb{};
     uint32_t max_items = 0;
     bool wave_ready = false;
-    // one captured wave per kind and number of bounce rounds
-    cudaGraphExec_t graph[kWaveKinds][kRounds] = {};
+    // one captured wave per kind, size and number of bounce rounds
+    cudaGraphExec_t graph[kWaveKinds][kWaveSizes][kRounds] = {};
     std::deque<Flight> flights;
     std::vector<cudaEvent_t> event_pool;
     pt_engine_stats stats{};
@@ -615,11 +646,12 @@ uint64_t wave_bytes(uint32_t paths) {
 
 void drop_graphs(pt_engine* e) {
     for (auto& kind : e->graph)
-        for (auto& g : kind)
-            if (g) {
-                cudaGraphExecDestroy(g);
-                g = nullptr;
-            }
+        for (auto& size : kind)
+            for (auto& g : size)
+                if (g) {
+                    cudaGraphExecDestroy(g);
+                    g = nullptr;
+                }
 }
 
 int setup_wave(pt_engine* e) {
@@ -676,9 +708,29 @@ void launch_persistent(void (*kernel)(P...), pt_engine* e, uint32_t threads, A&&
     launch_after(kernel, (uint32_t)e->sms * resident_blocks(kernel, (int)threads), threads, e->stream, std::forward<A>(args)...);
 }
 
+// The sizes of waves that differ in their launches: the most paths of each.
+constexpr uint32_t wave_sizes[kWaveSizes] = {1u << 17, 1u << 18, 1u << 21, 0xffffffffu};
+uint32_t wave_size(uint32_t paths) {
+    uint32_t k = 0;
+    while (paths > wave_sizes[k]) ++k;
+    return k;
+}
+// One wave runs at a time, so its last rounds have the GPU to themselves: the
+// rounds of a group alone, and larger waves too once few hits are left (512x512x16
+// of 1M triangles 6.63 -> 6.49 ms, 16 mixed jobs 50.0 -> 49.2, the room 4.32 both
+// ways; with 2^16 hits the room 4.41).
+TailRule wave_rule(uint32_t size) {
+    TailRule r = TailRule::of(wave_sizes[size], true);
+    if (size == kWaveSizes - 1u) {
+        r.first = 5u;
+        r.hits = 1u << 15;
+    }
+    return r;
+}
+
 // the launches of one wave (captured into a graph, or issued directly)
 template <bool kAlpha, bool kWideBvh, bool kPacked>
-cudaError_t issue_wave(pt_engine* e, uint32_t rounds) {
+cudaError_t issue_wave(pt_engine* e, uint32_t size, uint32_t rounds) {
     const cudaStream_t s = e->stream;
     const ItemDev* ring = e->d_ring.as<const ItemDev>();
     Ctrl* ctrl = e->d_ctrl.as<Ctrl>();
@@ -698,50 +750,62 @@ cudaError_t issue_wave(pt_engine* e, uint32_t rounds) {
         }
         return launch_persistent(trace_kernel<kAlpha, kWide, kPacked, 128>, e, 128, scenes, e->wb, round, e->cfg.steps_per_refill);
     };
-    const auto shade = [&](uint32_t round) {
-        if (st == 128u) return launch_persistent(shade_kernel<kAlpha, 128>, e, 128, scenes, jobs, e->wb, round);
-        if (st == 256u) return launch_persistent(shade_kernel<kAlpha, 256>, e, 256, scenes, jobs, e->wb, round);
-        if (st == 512u) return launch_persistent(shade_kernel<kAlpha, 512>, e, 512, scenes, jobs, e->wb, round);
-        return launch_persistent(shade_kernel<kAlpha, 1024>, e, 1024, scenes, jobs, e->wb, round);
+    const auto shade = [&](uint32_t round, uint32_t tail_hits) {
+        if (st == 128u) return launch_persistent(shade_kernel<kAlpha, 128>, e, 128, scenes, jobs, e->wb, round, tail_hits);
+        if (st == 256u) return launch_persistent(shade_kernel<kAlpha, 256>, e, 256, scenes, jobs, e->wb, round, tail_hits);
+        if (st == 512u) return launch_persistent(shade_kernel<kAlpha, 512>, e, 512, scenes, jobs, e->wb, round, tail_hits);
+        return launch_persistent(shade_kernel<kAlpha, 1024>, e, 1024, scenes, jobs, e->wb, round, tail_hits);
     };
+    const TailRule rule = wave_rule(size);
+    bool finished = false;
     for (uint32_t round = 0; round < rounds; ++round) {
         trace(round);
-        if (e->cfg.sort_min_hits != 0xffffffffu) {
+        uint32_t tail_hits = 0u;
+        if (round >= rule.first) {
+            finished = round >= rule.always;
+            tail_hits = rule.hits;
+            launch_after(tail_kernel<kAlpha, kWide, kPacked>, (uint32_t)e->sms, (uint32_t)kTailThreads, s, scenes, jobs, e->wb,
+                         round, finished ? 0xffffffffu : rule.hits);
+            if (finished) break;
+        }
+        const uint32_t sort_hits = std::max(e->cfg.sort_min_hits, tail_hits + 1u);
+        if (e->cfg.sort_min_hits != 0xffffffffu && wave_sizes[size] > kUnsortedPaths) {
             // hits of all jobs by triangle bucket (1024 triangles per bucket)
             launch_after(sort_count_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round, e->sort_counts,
-                         e->cfg.sort_min_hits, kEngineSortShift);
+                         sort_hits, kEngineSortShift);
             launch_after(sort_scan_kernel<0>, 1u, 1024u, s, e->wb.q, round, e->sort_counts, e->sort_counts + kSortBuckets,
-                         e->cfg.sort_min_hits);
+                         sort_hits);
             launch_after(sort_scatter_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round,
-                         e->sort_counts + kSortBuckets, e->cfg.sort_min_hits, kEngineSortShift);
+                         e->sort_counts + kSortBuckets, sort_hits, kEngineSortShift);
         }
-        shade(round);
+        shade(round, tail_hits);
     }
-    if constexpr (!kAlpha) trace(rounds);  // the last round's shadow rays
+    if (!kAlpha && !finished) trace(rounds);  // the last round's shadow rays
     launch_after(accumulate_kernel, per_wave_blocks, 256u, s, ctrl, ring, jobs, e->wb, e->d_done.as<uint32_t>());
     cudaMemcpyAsync(e->h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
     cudaMemcpyAsync(e->h_done, e->d_done.p, kMaxSlots * 4, cudaMemcpyDeviceToHost, s);
     return cudaGetLastError();
 }
 
-cudaError_t issue_any_wave(pt_engine* e, uint32_t kind, uint32_t rounds) {
+cudaError_t issue_any_wave(pt_engine* e, uint32_t kind, uint32_t size, uint32_t rounds) {
     const bool wide = (e->cfg.precision & PT_PRECISION_WIDE_BVH) != 0, plain = (kind & kWavePlain) != 0;
-    if (kind & kWaveAlpha) return plain ? issue_wave<true, false, false>(e, rounds) : issue_wave<true, false, true>(e, rounds);
-    if (wide) return issue_wave<false, true, false>(e, rounds);
-    return plain ? issue_wave<false, false, false>(e, rounds) : issue_wave<false, false, true>(e, rounds);
+    if (kind & kWaveAlpha) return plain ? issue_wave<true, false, false>(e, size, rounds) : issue_wave<true, false, true>(e, size, rounds);
+    if (wide) return issue_wave<false, true, false>(e, size, rounds);
+    return plain ? issue_wave<false, false, false>(e, size, rounds) : issue_wave<false, false, true>(e, size, rounds);
 }
 
 // one wave of `rounds` bounce rounds (the deepest job of the wave needs
 // max_bounces + 1; a path never takes more, so shallower waves skip the
 // launches of rounds that would find empty queues)
-int launch_wave(pt_engine* e, uint32_t kind, uint32_t rounds) {
+int launch_wave(pt_engine* e, uint32_t kind, uint32_t paths, uint32_t rounds) {
+    const uint32_t size = wave_size(paths);
     if (rounds < 1 || rounds > kRounds) rounds = kRounds;
-    cudaGraphExec_t& exec = e->graph[kind][rounds - 1];
+    cudaGraphExec_t& exec = e->graph[kind][size][rounds - 1];
     if (e->cfg.use_graphs && !exec) {
         cudaGraph_t g = nullptr;
         int rc = e->cuda(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal), "graph capture");
         if (rc) return rc;
-        const cudaError_t le = issue_any_wave(e, kind, rounds);
+        const cudaError_t le = issue_any_wave(e, kind, size, rounds);
         const cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
         if ((rc = e->cuda(le, "wave capture"))) return rc;
         if ((rc = e->cuda(ce, "graph capture"))) return rc;
@@ -755,7 +819,7 @@ int launch_wave(pt_engine* e, uint32_t kind, uint32_t rounds) {
     if (e->cfg.use_graphs)
         rc = e->cuda(cudaGraphLaunch(exec, e->stream), "graph launch");
     else
-        rc = e->cuda(issue_any_wave(e, kind, rounds), "wave launch");
+        rc = e->cuda(issue_any_wave(e, kind, size, rounds), "wave launch");
     if (rc) return rc;
     cudaEventRecord(f.stop, e->stream);
     e->flights.push_back(f);
@@ -821,8 +885,8 @@ double feed_key(const Job& j, std::chrono::steady_clock::time_point now) {
 // its pending items in tile order while they fit the wave's path budget and
 // item limit.  Writes them to the ring and the ring's tail, so the wave's
 // planner (which takes every item up to the budget) consumes exactly these.
-// Returns the number of items fed; *kind and *rounds describe the wave.
-int feed_wave(pt_engine* e, size_t* fed, uint32_t* kind, uint32_t* rounds) {
+// Returns the number of items fed; *kind, *wave_paths and *rounds describe the wave.
+int feed_wave(pt_engine* e, size_t* fed, uint32_t* kind, uint32_t* wave_paths, uint32_t* rounds) {
     *fed = 0;
     *kind = 0;
     *rounds = 1;
@@ -868,6 +932,7 @@ int feed_wave(pt_engine* e, size_t* fed, uint32_t* kind, uint32_t* rounds) {
                      "wave feed");
     if (rc) return rc;
     *fed = wave.size();
+    *wave_paths = (uint32_t)paths;
     return PT_OK;
 }
 
@@ -934,11 +999,11 @@ int harvest(pt_engine* e, bool block) {
 int pump(pt_engine* e) {
     while (e->flights.size() < PT_ENGINE_FLIGHTS) {
         size_t fed = 0;
-        uint32_t kind = 0, rounds = 1;
-        int rc = feed_wave(e, &fed, &kind, &rounds);
+        uint32_t kind = 0, paths = 0, rounds = 1;
+        int rc = feed_wave(e, &fed, &kind, &paths, &rounds);
         if (rc) return rc;
         if (fed == 0) break;
-        if ((rc = launch_wave(e, kind, rounds))) return rc;
+        if ((rc = launch_wave(e, kind, paths, rounds))) return rc;
     }
     return PT_OK;
 }

@@ -626,47 +626,6 @@ struct SortCfg {
 #endif
 constexpr int kSmallShadeThreads = 128;
 
-// no hit sort in a group of at most this many paths: its sorted rounds are the
-// first few, and three launches a round cost 795 against 778 us (100k
-// triangles, 640x360x1); at 1 M paths 1200 against 1222 (10k, 481x271x8)
-#ifndef PT_UNSORTED_PATHS
-#define PT_UNSORTED_PATHS (1u << 18)
-#endif
-
-// The rounds from which a group's paths are finished by the tail kernel: from
-// `first` on when a round has at most kTailHits hits, from `always` on in any
-// case.  Up to 2^17 paths the rounds' launches and longest rays cost more than
-// their better use of lanes gives, from the start (a frame of 160x120 paths of
-// the room: 237 us from round 0, 258 from 2, 397 never; 100x70x16 of 10k
-// triangles 360, 403, 560), up to 2^18 from round 1 (640x360 of 100k triangles
-// 841 from 0, 795 from 1, 810 from 2, 1140 never).  Above that the full rounds
-// go faster as launches of their own; after round 4 Russian roulette has ended
-// most paths (256x256x16 of the room 1352 from 4, 1258 from 5, 1310 never), and
-// open scenes thin out earlier (481x271x8 of 10k triangles with coverage 1172
-// with the rule's hits, 1205 with 2^15, 1288 from round 5, 1535 never;
-// 960x540x4 of 1M triangles 3611, 4100 with 2^18, 3784 never).  Groups of over
-// 2^21 paths overlap with one another, and at 2^22 the gain is -2 to 3 %.
-// Beside other groups the tail's blocks, which fill their SMs at a third of the
-// rate, are in the way: four groups of 128x128x16 paths of the room 1605 us
-// without it, 2089 with; up to 2^16 paths a group they still gain (four of
-// 64x64x16: the room 1133 without, 939 with, 1M triangles 3061, 2397).
-constexpr uint32_t kTailHits = 1u << 17;
-struct TailRule {
-    uint32_t first = 0xffffffffu, always = 0xffffffffu;
-    static TailRule of(uint32_t paths, bool alone) {
-        TailRule r;
-        if (!alone) {
-            if (paths <= (1u << 16)) r.first = r.always = 1u;
-        } else if (paths <= (1u << 18))
-            r.first = r.always = paths <= (1u << 17) ? 0u : 1u;
-        else if (paths <= (1u << 21)) {
-            r.first = 2u;
-            r.always = 5u;
-        }
-        return r;
-    }
-};
-
 // One group of paths through raygen, max_bounces + 1 rounds of trace / (hit
 // sort) / shade, and accumulate on `stream`; the accumulation runs on
 // `acc_stream` (null: `stream`) after `done` marks the group's end there.
@@ -706,14 +665,14 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
                 const auto tail = tail_kernel<kAlpha, kTri36, kWide, kPacked>;
                 PTW_TRY(timer(PT_KC_SHADE, stream, [&] {
                     return launch_after(tail, (uint32_t)sms, kTailThreads, stream, w, f, q, round, tile.max_bounces,
-                                        all ? 0xffffffffu : kTailHits);
+                                        all ? 0xffffffffu : rule.hits);
                 }));
                 if (all) break;
-                tail_hits = kTailHits;
+                tail_hits = rule.hits;
             }
         }
         const uint32_t sort_hits = std::max(sort.min_hits, tail_hits + 1u);
-        if (sort.counts && sort_hits <= g.paths && g.paths > PT_UNSORTED_PATHS) {
+        if (sort.counts && sort_hits <= g.paths && g.paths > kUnsortedPaths) {
             PTW_TRY(timer(PT_KC_SORT, stream, [&] {
                 cudaError_t e = launch_after(sort_count_kernel<PT_SORT_KEY>, (uint32_t)sms * 4u, kSortThreads, stream, w,
                                              q, round, sort.counts, sort_hits, sort.tri_shift);

@@ -7,6 +7,7 @@ import pytest
 
 import pathtracer as pt
 from pathtracer import abi
+from pathtracer.engine import Engine
 from worlds import non_opaque_world
 
 pytestmark = pytest.mark.gpu
@@ -64,3 +65,34 @@ def test_groups_beside_one_another(worlds, size):
     plain = accumulation(u, size, 16, 8, abi.PT_KERNEL_PLAIN, calls=5)
     wave = accumulation(u, size, 16, 8, abi.PT_KERNEL_WAVEFRONT, calls=5)
     assert plain.tobytes() == wave.tobytes()
+
+
+@pytest.mark.parametrize("size,spp", [((40, 30), 1), ((129, 127), 10), ((300, 217), 8), ((520, 258), 16)])
+@pytest.mark.parametrize("scene", ["room", "field", "coverage"])
+def test_waves_of_every_size(worlds, scene, size, spp):
+    """One request per wave: up to 2^17, 2^18 and 2^21 paths, and more."""
+    u = worlds[scene][1]
+    eng = Engine(wave_paths=1 << 22)
+    cam = abi.Camera.from_buffer_copy(u.camera.contents)
+    job = eng.submit(eng.add_scene(u), cam, *size, spp, 7)
+    eng.wait_idle(timeout_ms=60000)
+    plain = accumulation(u, size, spp, 7, abi.PT_KERNEL_PLAIN)
+    assert eng.read(job, *size, abi.PT_TILE_ACCUMULATION).tobytes() == plain.tobytes()
+    eng.close()
+
+
+def test_waves_of_jobs_of_different_depths(worlds):
+    """Small jobs of all three scenes and depths 0..9 in the same waves."""
+    eng = Engine(wave_paths=1 << 20, tile_size=16)
+    ids = {name: eng.add_scene(u) for name, (_, u) in worlds.items()}
+    jobs = []
+    for depth in range(10):
+        name = sorted(worlds)[depth % 3]
+        u = worlds[name][1]
+        cam = abi.Camera.from_buffer_copy(u.camera.contents)
+        jobs.append((u, depth, eng.submit(ids[name], cam, 30 + depth, 23, 3, depth)))
+    eng.wait_idle(timeout_ms=60000)
+    for u, depth, job in jobs:
+        plain = accumulation(u, (30 + depth, 23), 3, depth, abi.PT_KERNEL_PLAIN)
+        assert eng.read(job, 30 + depth, 23, abi.PT_TILE_ACCUMULATION).tobytes() == plain.tobytes()
+    eng.close()
