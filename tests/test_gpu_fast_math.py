@@ -1,5 +1,5 @@
 """The range-free division, reciprocal and square root of the shading kernels against the IEEE operators, and the
-dielectric sample built on them against the one built on the operators, bit for bit."""
+dielectric sample built on them, alone and two at a time, against the one built on the operators, bit for bit."""
 import subprocess
 
 import pytest
@@ -116,6 +116,15 @@ __global__ void samples(unsigned long long* bad, unsigned long long* count) {
         used += 1u;
         redone += redo;
         if (!redo && !agree(fast, want)) atomicAdd(bad + 5, 1ull);
+        // two samples packed: this one and the next, in either place
+        const float r2 = rand_next(s), tpr2 = kTwoPi * rand_next(s);
+        bool redo2 = false, pair_redo = false, swapped_redo = false;
+        float a, b, c, e;
+        const float fast2 = dielectric_sample_fast(d, r2, tpr2, &redo2);
+        dielectric_pair_fast(d, r1, tpr, r2, tpr2, &a, &b, &pair_redo);
+        dielectric_pair_fast(d, r2, tpr2, r1, tpr, &c, &e, &swapped_redo);
+        if (pair_redo != (redo || redo2) || swapped_redo != pair_redo) atomicAdd(bad + 5, 1ull);
+        if (!pair_redo && (!agree(a, fast) || !agree(b, fast2) || !agree(c, fast2) || !agree(e, fast))) atomicAdd(bad + 5, 1ull);
     }
     atomicAdd(count, (unsigned long long)used);
     atomicAdd(count + 1, (unsigned long long)redone);
