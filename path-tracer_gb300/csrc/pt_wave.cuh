@@ -250,8 +250,10 @@ struct LaneScene {
 #ifndef PT_VISIT_TWICE
 #define PT_VISIT_TWICE 1
 #endif
+// the 8-wide traversal turns earlier: its visits cost about 100 instructions whatever the lanes
+// (1M triangles, 960x540x16: 12.05 ms with 16, 11.84 with 20, 11.78 with 24, 11.81 with 28)
 #ifndef PT_WIDE_VISIT_KEEP
-#define PT_WIDE_VISIT_KEEP 16
+#define PT_WIDE_VISIT_KEEP 24
 #endif
 #ifndef PT_WIDE_TEST_LEAVE
 #define PT_WIDE_TEST_LEAVE 0
