@@ -209,7 +209,7 @@ struct Rec {
     PTD void interior() {}
     PTD void leaf() {}
     PTD void tri() {}
-    PTD void draw() {}
+    PTD void draws(uint32_t) {}
 };
 template <>
 struct Rec<true> {
@@ -228,7 +228,7 @@ struct Rec<true> {
         c->triangle_tests += 1;
         if (shadow) c->shadow_triangle_tests += 1;
     }
-    PTD void draw() { c->rand_draws += 1; }
+    PTD void draws(uint32_t n) { c->rand_draws += n; }
 };
 
 template <bool kRec>
@@ -236,7 +236,7 @@ struct Rng {
     uint32_t s;
     Rec<kRec> rec;
     PTD float operator()() {
-        rec.draw();
+        rec.draws(1u);
         return rand_next(s);
     }
 };
@@ -1196,10 +1196,13 @@ PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_co
     // the samples in order: `sample(r1, tpr)` gives one's term.  The checked
     // samples are a second loop that an estimate falls back to as a whole: as a
     // branch inside the one loop they cost 6 % of shading and 12 KB of code.
+    // (Both draw from `s`, not from rng: an estimate that is taken twice makes
+    // its 32 draws once.)
     const uint32_t start = rng.s;
+    uint32_t s = start;
     const auto sum_of = [&](auto&& sample) {
         float sum = 0.0f;
-        rng.s = start;
+        s = start;
         if (kSpread && !kRec && spread.log2 > 0u) {
             const uint32_t lanes = 1u << spread.log2, first = (uint32_t)__ffs(spread.mask) - 1u;
             uint32_t at = kRngJump.a[spread.index] * start + kRngJump.c[spread.index];
@@ -1212,12 +1215,12 @@ PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_co
                 for (uint32_t k = 0; k < lanes; ++k) sum += __shfl_sync(spread.mask, term, first + k);
                 at = ja * at + jc;
             }
-            rng.s = kRngJump.a[16] * start + kRngJump.c[16];
+            s = kRngJump.a[16] * start + kRngJump.c[16];
         } else {
 #pragma unroll 1
             for (int i = 0; i < 16; ++i) {
-                const float r1 = rng();
-                sum += sample(r1, kTwoPi * rng());
+                const float r1 = rand_next(s);
+                sum += sample(r1, kTwoPi * rand_next(s));
             }
         }
         return sum;
@@ -1231,7 +1234,7 @@ PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_co
             // two samples at a time: the shading of 1M triangles 960x540x16 2.72 -> 2.64 ms
 #pragma unroll 1
             for (int i = 0; i < 8; ++i) {
-                const float ra = rng(), ta = kTwoPi * rng(), rb = rng(), tb = kTwoPi * rng();
+                const float ra = rand_next(s), ta = kTwoPi * rand_next(s), rb = rand_next(s), tb = kTwoPi * rand_next(s);
                 float a, b;
                 dielectric_pair_fast(t, ra, ta, rb, tb, &a, &b, &redo);
                 sum += a;
@@ -1241,6 +1244,8 @@ PTD f3 estimate_e_dielectric(f3 wo, float opl, f2 alpha, float ior_m, f3 spec_co
     }
     if (kSpread && !kRec && spread.log2 > 0u) redo = __any_sync(spread.mask, redo);
     if (__builtin_expect(redo, 0)) sum = sum_of([&](float r1, float tpr) { return dielectric_sample(t, r1, tpr); });
+    rng.s = s;
+    rng.rec.draws(32u);
     return spec_color * sum / 16.0f;
 }
 
