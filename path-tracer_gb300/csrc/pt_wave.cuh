@@ -272,18 +272,21 @@ constexpr int32_t kFinished = -2, kIdle = -1;
 PTD float below(float t) { return t > 0.0f ? __uint_as_float(__float_as_uint(t) - 1u) : -1.0f; }
 PTD float above(float t) { return __uint_as_float(__float_as_uint(t) + 1u); }
 
+// the smaller, NaN when one of them is
+PTD float min_or_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // A box's entry distance, at least 2^-149, and exit distance, at most `limit`
-// (see BinaryRay): the box is accepted when *t_near <= *t_far.
+// (see BinaryRay), NaN when no plane gives a number: the box is accepted when
+// *t_near <= *t_far.
 PTD void slabs(float4 lo, float4 hi, f3 rcp, f3 nod, float limit, float* t_near, float* t_far) {
     const float t0x = fma_(lo.x, rcp.x, nod.x), t0y = fma_(lo.y, rcp.y, nod.y), t0z = fma_(lo.z, rcp.z, nod.z);
     const float t1x = fma_(hi.x, rcp.x, nod.x), t1y = fma_(hi.y, rcp.y, nod.y), t1z = fma_(hi.z, rcp.z, nod.z);
     *t_near = max3f(fmaxf(fminf(t0x, t1x), 0x1p-149f), fminf(t0y, t1y), fminf(t0z, t1z));
-    *t_far = min3f(fminf(fmaxf(t0x, t1x), limit), fmaxf(t0y, t1y), fmaxf(t0z, t1z));
-}
-// no axis of the ray gives a slab distance that is a number (see BinaryRay)
-PTD bool boxless(f3 nod) {
-    const float inf = __int_as_float(0x7f800000);
-    return !(fabsf(nod.x) < inf) && !(fabsf(nod.y) < inf) && !(fabsf(nod.z) < inf);
+    *t_far = min_or_nan(limit, min3f(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fmaxf(t0z, t1z)));
 }
 
 // What a traversal looks for (the template argument kFind): the closest hit
@@ -301,11 +304,13 @@ constexpr int32_t kClosestRay = -2;
 //
 // The slab test of trace.slang:597-609 accepts a box when t_near <= t_far,
 // t_far > 0 and t_near < hit_t.  Here that is one comparison,
-// max(t_near, 2^-149) <= min(t_far, below(hit_t)): the same for every finite
-// value (2^-149 is the smallest positive float; with hit_t = 2^-149 no
-// triangle can be nearer, whatever is visited).  Only when all three axes are
-// NaN does it differ, so such a ray (never accepted by the reference either:
-// each axis then rejects or is NaN) gets the limit -1, which rejects all.
+// max(t_near, 2^-149) <= min(t_far, below(hit_t)): the same for every value
+// (2^-149 is the smallest positive float; with hit_t = 2^-149 no triangle can
+// be nearer, whatever is visited).  min and max skip NaN, except the last min:
+// when no plane of the box gives a number (a box of NaNs, or a ray without any
+// extent), t_far stays NaN and the box is rejected, as by the shader.  Of two
+// children entered at or before the origin and at exactly 2^-149 the second is
+// visited first, as at a tie.
 template <bool kRec, bool kAlpha, int kFind, bool kTri36, class Scene>
 struct BinaryRay {
     static constexpr int kVisitKeep = PT_VISIT_KEEP, kTestLeave = PT_TEST_LEAVE, kRefillAt = PT_REFILL_AT;
@@ -333,7 +338,7 @@ struct BinaryRay {
         rcp = mk(ptd::rcp(dir.x), ptd::rcp(dir.y), ptd::rcp(dir.z));
         s = make_shear(dir, rcp);
         nod = -o * rcp;
-        limit = boxless(nod) ? -1.0f : below(t_max);
+        limit = below(t_max);
         hv = hw = 0.0f;
         hit = -1;
         light_tri = light;
@@ -650,7 +655,7 @@ struct PackedRay {
         rp = mk(rcp.x < 0.0f ? 0.0f : rcp.x, rcp.y < 0.0f ? 0.0f : rcp.y, rcp.z < 0.0f ? 0.0f : rcp.z);
         rn = mk(rcp.x < 0.0f ? rcp.x : 0.0f, rcp.y < 0.0f ? rcp.y : 0.0f, rcp.z < 0.0f ? rcp.z : 0.0f);
         oct = (rcp.x < 0.0f ? 1u : 0u) | (rcp.y < 0.0f ? 2u : 0u) | (rcp.z < 0.0f ? 4u : 0u);
-        limit = boxless(nod) ? -1.0f : below(t_max);
+        limit = below(t_max);
         hv = hw = 0.0f;
         hit = -1;
         light_tri = light;
