@@ -10,6 +10,7 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <deque>
@@ -58,8 +59,9 @@ struct ItemDev {
 };
 
 struct Ctrl {
-    unsigned long long head;  // ring position of the next wave's first item
-    uint32_t feed_items, feed_paths;  // what the host fed for the next wave
+    unsigned long long feed_first;  // what the host fed for the next wave: the ring position of its first item,
+    uint32_t feed_items, feed_paths;  // their number and their paths
+    unsigned long long head;  // ring position after the last wave's items
     uint32_t wave_items, wave_paths;
     unsigned long long waves;
 };
@@ -81,10 +83,10 @@ constexpr uint32_t kEngineSortShift = 10;  // sort bucket = triangle index / 102
 
 // takes the fed items off the ring and clears the rounds' counters (one block)
 __global__ void __launch_bounds__(1024) plan_kernel(Ctrl* ctrl, const ItemDev* ring, uint64_t ring_cap, WaveBufs b) {
-    const unsigned long long head = ctrl->head;
+    const unsigned long long first = ctrl->feed_first;
     const uint32_t n = ctrl->feed_items, paths = ctrl->feed_paths;
     for (uint32_t k = threadIdx.x; k < n; k += blockDim.x) {
-        const uint32_t at = (uint32_t)((head + k) % ring_cap);
+        const uint32_t at = (uint32_t)((first + k) % ring_cap);
         b.wave_item[k] = at;
         b.wave_off[k] = ring[at].offset;
     }
@@ -92,7 +94,7 @@ __global__ void __launch_bounds__(1024) plan_kernel(Ctrl* ctrl, const ItemDev* r
     __syncthreads();
     if (threadIdx.x == 0) {
         b.wave_off[n] = paths;
-        ctrl->head = head + n;
+        ctrl->head = first + n;
         ctrl->wave_items = n;
         ctrl->wave_paths = paths;
         ctrl->waves += 1;
@@ -807,20 +809,29 @@ int launch_wave(pt_engine* e, uint32_t kind, uint32_t paths, uint32_t rounds) {
         if (rc) return rc;
         const cudaError_t le = issue_any_wave(e, kind, size, rounds);
         const cudaError_t ce = cudaStreamEndCapture(e->stream, &g);
-        if ((rc = e->cuda(le, "wave capture"))) return rc;
-        if ((rc = e->cuda(ce, "graph capture"))) return rc;
-        rc = e->cuda(cudaGraphInstantiate(&exec, g, 0), "graph instantiate");
-        cudaGraphDestroy(g);
+        rc = e->cuda(le, "wave capture");
+        if (!rc) rc = e->cuda(ce, "graph capture");
+        if (!rc) rc = e->cuda(cudaGraphInstantiate(&exec, g, 0), "graph instantiate");
+        if (rc) exec = nullptr;
+        if (g) cudaGraphDestroy(g);
         if (rc) return rc;
     }
     Flight f{e->event(), e->event()};
     cudaEventRecord(f.start, e->stream);
     int rc;
-    if (e->cfg.use_graphs)
+    if (e->cfg.use_graphs) {
         rc = e->cuda(cudaGraphLaunch(exec, e->stream), "graph launch");
-    else
+    } else {
+        // a wave of plain launches that is refused in its middle has run in part,
+        // and what it added to its jobs cannot be taken back
         rc = e->cuda(issue_any_wave(e, kind, size, rounds), "wave launch");
-    if (rc) return rc;
+        if (rc) e->sticky = rc;
+    }
+    if (rc) {
+        e->event_pool.push_back(f.start);
+        e->event_pool.push_back(f.stop);
+        return rc;
+    }
     cudaEventRecord(f.stop, e->stream);
     e->flights.push_back(f);
     return PT_OK;
@@ -881,59 +892,78 @@ double feed_key(const Job& j, std::chrono::steady_clock::time_point now) {
     return (double)j.pending_paths / (1.0 + age_ms / kAgeMs);
 }
 
-// Hands the next wave its work items: jobs in feed_key order, each giving
-// its pending items in tile order while they fit the wave's path budget and
-// item limit.  Writes them to the ring and the ring's tail, so the wave's
-// planner (which takes every item up to the budget) consumes exactly these.
-// Returns the number of items fed; *kind, *wave_paths and *rounds describe the wave.
-int feed_wave(pt_engine* e, size_t* fed, uint32_t* kind, uint32_t* wave_paths, uint32_t* rounds) {
-    *fed = 0;
-    *kind = 0;
-    *rounds = 1;
+// The work items of the next wave and what its launches must handle.
+struct Wave {
+    std::vector<ItemDev> items;
+    std::vector<std::pair<Job*, size_t>> taken;  // the jobs they are of, and how many of each
+    uint64_t paths = 0;
+    uint32_t kind = 0, rounds = 1;
+};
+
+// Chooses the next wave's items: jobs in feed_key order, each giving its
+// pending items in tile order while they fit the wave's path budget and item
+// limit.  The jobs keep them until the wave is queued (take_wave), so that a
+// wave that cannot be fed or launched leaves nothing behind.
+Wave choose_wave(pt_engine* e) {
+    Wave wave;
     const auto now = std::chrono::steady_clock::now();
     std::vector<std::pair<double, Job*>> order;
     for (auto& [id, j] : e->jobs)
         if (!j.pending.empty()) order.emplace_back(feed_key(j, now), &j);
-    if (order.empty()) return PT_OK;
     std::stable_sort(order.begin(), order.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
-    std::vector<ItemDev> wave;
-    uint64_t paths = 0;
     const uint64_t budget = e->cfg.wave_paths;
     for (auto& [key, j] : order) {
-        while (!j->pending.empty() && wave.size() < e->max_items) {
-            const ItemDev& it = j->pending.front();
+        size_t count = 0;
+        for (const ItemDev& it : j->pending) {
             const uint64_t np = (uint64_t)it.w * it.h * it.samples;
-            if (!wave.empty() && paths + np > budget) break;
-            wave.push_back(it);
-            wave.back().offset = (uint32_t)paths;
-            paths += np;
-            j->pending_paths -= np;
-            j->pending.pop_front();
-            *kind |= (j->alpha ? kWaveAlpha : 0u) | (j->plain ? kWavePlain : 0u);
-            *rounds = std::max(*rounds, j->rounds);
+            if (wave.items.size() >= e->max_items || (!wave.items.empty() && wave.paths + np > budget)) break;
+            wave.items.push_back(it);
+            wave.items.back().offset = (uint32_t)wave.paths;
+            wave.paths += np;
+            count += 1;
         }
-        if (paths >= budget || wave.size() >= e->max_items) break;
+        if (count != 0) {
+            wave.taken.emplace_back(j, count);
+            wave.kind |= (j->alpha ? kWaveAlpha : 0u) | (j->plain ? kWavePlain : 0u);
+            wave.rounds = std::max(wave.rounds, j->rounds);
+        }
+        if (wave.paths >= budget || wave.items.size() >= e->max_items) break;
     }
-    if (e->tail + wave.size() - e->head_seen > e->ring_cap) return e->fail(PT_ERR_OUT_OF_LIMITS, "work ring full");
+    return wave;
+}
+
+// Writes the wave's items to the ring and says where they are: its planner
+// takes exactly these.
+int feed_wave(pt_engine* e, const Wave& wave) {
+    if (e->tail + wave.items.size() - e->head_seen > e->ring_cap) return e->fail(PT_ERR_OUT_OF_LIMITS, "work ring full");
     // copy into the ring (two pieces across the wrap); the copies read
     // pageable host memory, so they have taken it before they return
     size_t done = 0;
-    while (done < wave.size()) {
+    while (done < wave.items.size()) {
         const uint64_t pos = (e->tail + done) % e->ring_cap;
-        const size_t n = std::min<size_t>(wave.size() - done, e->ring_cap - pos);
-        int rc = e->cuda(cudaMemcpyAsync(e->d_ring.as<ItemDev>() + pos, wave.data() + done, n * sizeof(ItemDev),
+        const size_t n = std::min<size_t>(wave.items.size() - done, e->ring_cap - pos);
+        int rc = e->cuda(cudaMemcpyAsync(e->d_ring.as<ItemDev>() + pos, wave.items.data() + done, n * sizeof(ItemDev),
                                          cudaMemcpyHostToDevice, e->stream), "ring write");
         if (rc) return rc;
         done += n;
     }
-    e->tail += wave.size();
-    const uint32_t feed[2] = {(uint32_t)wave.size(), (uint32_t)paths};
-    int rc = e->cuda(cudaMemcpyAsync(&e->d_ctrl.as<Ctrl>()->feed_items, feed, sizeof feed, cudaMemcpyHostToDevice, e->stream),
-                     "wave feed");
-    if (rc) return rc;
-    *fed = wave.size();
-    *wave_paths = (uint32_t)paths;
-    return PT_OK;
+    Ctrl feed{};
+    feed.feed_first = e->tail;
+    feed.feed_items = (uint32_t)wave.items.size();
+    feed.feed_paths = (uint32_t)wave.paths;
+    static_assert(offsetof(Ctrl, feed_first) == 0 && offsetof(Ctrl, head) == 16, "the feed is the head of the block");
+    return e->cuda(cudaMemcpyAsync(e->d_ctrl.p, &feed, offsetof(Ctrl, head), cudaMemcpyHostToDevice, e->stream), "wave feed");
+}
+
+// the wave is queued: its items leave their jobs, and the ring's tail moves on
+void take_wave(pt_engine* e, const Wave& wave) {
+    for (auto& [j, count] : wave.taken)
+        for (size_t k = 0; k < count; ++k) {
+            const ItemDev& it = j->pending.front();
+            j->pending_paths -= (uint64_t)it.w * it.h * it.samples;
+            j->pending.pop_front();
+        }
+    e->tail += wave.items.size();
 }
 
 void free_accumulation(pt_engine* e, Accumulation& a) {
@@ -998,12 +1028,12 @@ int harvest(pt_engine* e, bool block) {
 #endif
 int pump(pt_engine* e) {
     while (e->flights.size() < PT_ENGINE_FLIGHTS) {
-        size_t fed = 0;
-        uint32_t kind = 0, paths = 0, rounds = 1;
-        int rc = feed_wave(e, &fed, &kind, &paths, &rounds);
+        const Wave wave = choose_wave(e);
+        if (wave.items.empty()) break;
+        int rc = feed_wave(e, wave);
+        if (!rc) rc = launch_wave(e, wave.kind, (uint32_t)wave.paths, wave.rounds);
         if (rc) return rc;
-        if (fed == 0) break;
-        if ((rc = launch_wave(e, kind, paths, rounds))) return rc;
+        take_wave(e, wave);
     }
     return PT_OK;
 }

@@ -1,0 +1,49 @@
+"""What follows when the CUDA runtime refuses a call on the host: the next call works, on the work that was asked for."""
+import pytest
+
+import wrapped_library
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    return wrapped_library.link(tmp_path_factory.mktemp("wrapped"))
+
+
+def test_a_refused_wave_is_launched_later(library):
+    """The items of a wave whose graph could not be made run in a later wave, once, as that wave's kernels need: the
+    refused job has coverage materials and more paths than the opaque one that follows it."""
+    wrapped_library.run(library, """
+        from worlds import non_opaque_world
+        worlds = [non_opaque_world(), pt.World.cornell_box()]
+        updates = [w.take_updates() for w in worlds]
+        sizes = [(300, 217), (40, 30)]
+        want = []
+        for u, size in zip(updates, sizes):
+            t = pt.PathTracer(u, size)
+            t.set_kernel(abi.PT_KERNEL_PLAIN)
+            t.set_max_bounces(6)
+            assert t.trace(8) == 8
+            want.append(t.read_tile(abi.PT_TILE_ACCUMULATION).tobytes())
+            t.close()
+        eng = Engine(wave_paths=1 << 20)
+        ids = [eng.add_scene(u) for u in updates]
+        cameras = [abi.Camera.from_buffer_copy(u.camera.contents) for u in updates]
+        for first in (0, 1):  # again when the graphs are there: nothing is refused, nothing is left of the first
+            jobs = []
+            for k in (0, 1):
+                count("refuse_instantiate").value = 1 if first == k == 0 else 0
+                try:
+                    jobs.append(eng.submit(ids[k], cameras[k], *sizes[k], 8, 6))
+                    assert count("instantiated").value > 0
+                except pt.PathTracerError as e:
+                    assert first == k == 0 and e.code == abi.PT_ERR_OOM, e
+                    jobs.append(1)  # the job is queued all the same
+                assert count("refuse_instantiate").value == 0
+            eng.wait_idle(timeout_ms=20000)
+            for k in (0, 1):
+                assert eng.status(jobs[k]) == (abi.PT_JOB_DONE, 8)
+                assert eng.read(jobs[k], *sizes[k], abi.PT_TILE_ACCUMULATION).tobytes() == want[k]
+        eng.close()
+        """)
