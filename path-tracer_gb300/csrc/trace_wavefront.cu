@@ -630,6 +630,10 @@ constexpr int kSmallShadeThreads = 128;
 // sort) / shade, and accumulate on `stream`; the accumulation runs on
 // `acc_stream` (null: `stream`) after `done` marks the group's end there.
 // kTri36 reads the reference's 36-byte triangles instead of the padded copy.
+// The first launch on a stream that the caller can queue work on (the call's
+// own of pt_trace_noalloc, the context's) is an ordinary one: launch_after()
+// waits for the kernel before it only, and the caller's last kernel may have
+// been launched the same way and finish before what was queued before it.
 // `alone`: no other group is expected to run beside it.
 // `serial`: a round's shadow rays are traced right after its shading, by a
 // launch of their own (the recording kernels, whose records follow the path's
@@ -648,6 +652,10 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
     if (small) trace_blocks = std::min(trace_blocks, (g.paths + kExtendThreads / 4 - 1) / (kExtendThreads / 4));
     PTW_TRY(timer(PT_KC_RAYGEN, stream, [&] {
         const uint32_t blocks = (std::max(g.paths, kCounterWords) + 255u) / 256u;
+        if constexpr (kTri36 || kRec) {
+            raygen_kernel<kRec><<<blocks, 256, 0, stream>>>(w, tile, g, q);
+            return cudaGetLastError();
+        }
         return launch_after(raygen_kernel<kRec>, blocks, 256, stream, w, tile, g, q);
     }));
     const auto trace = [&](int cls, uint32_t round, uint32_t what) {
@@ -705,7 +713,10 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
         PTW_TRY(cudaStreamWaitEvent(as, done, 0));
     }
     PTW_TRY(timer(PT_KC_ACCUMULATE, as, [&] {
-        return launch_after(accumulate_kernel, (g.pixels + 255u) / 256u, 256u, as, tile, g, q.color);
+        const uint32_t blocks = (g.pixels + 255u) / 256u;
+        if (as == stream) return launch_after(accumulate_kernel, blocks, 256u, as, tile, g, q.color);
+        accumulate_kernel<<<blocks, 256, 0, as>>>(tile, g, q.color);
+        return cudaGetLastError();
     }));
     if constexpr (kRec) {
         finalize_records_kernel<<<(g.paths + 255u) / 256u, 256, 0, stream>>>(tile, g, q, sinks);
