@@ -625,6 +625,7 @@ struct pt_engine {
     }
     int cuda(cudaError_t e, const char* what) {
         if (e == cudaSuccess) return PT_OK;
+        cudaGetLastError();  // reported here: the next launch does not find it again
         error = std::string(what) + ": " + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? PT_ERR_OOM : PT_ERR_CUDA;
     }

@@ -98,6 +98,7 @@ struct pt_ctx {
     }
     int cuda(cudaError_t e, const char* what) {
         if (e == cudaSuccess) return PT_OK;
+        cudaGetLastError();  // reported here: the next launch does not find it again
         error = std::string(what) + ": " + cudaGetErrorString(e);
         return e == cudaErrorMemoryAllocation ? PT_ERR_OOM : PT_ERR_CUDA;
     }
@@ -362,13 +363,18 @@ bool check_staged(pt_ctx* c, const pt_scene_upload* s, SceneCheck* result) {
     const uint32_t count = (uint32_t)s->node_count, blocks = (count + 255u) / 256u;
     cudaError_t e = cudaMemsetAsync(check, 0, sizeof(SceneCheck), c->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(parent, 0xff, parents, c->stream);
-    if (e != cudaSuccess) return false;
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
     link_nodes_kernel<<<blocks, 256, 0, c->stream>>>(c->stage_nodes.as<pt_bvh_node>(), count, s->triangle_count, parent, check);
     check_nodes_kernel<<<blocks, 256, 0, c->stream>>>(c->stage_nodes.as<pt_bvh_node>(), count, parent, check);
     check_materials_kernel<<<(unsigned)((s->triangle_count + 255) / 256), 256, 0, c->stream>>>(
         c->stage_attr.as<pt_triangle_attribute>(), s->triangle_count, s->material_count, check);
-    return cudaGetLastError() == cudaSuccess &&
-           cudaMemcpyAsync(result, check, sizeof *result, cudaMemcpyDeviceToHost, c->stream) == cudaSuccess;
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(result, check, sizeof *result, cudaMemcpyDeviceToHost, c->stream);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
 }
 
 int validate_lights(pt_ctx* c, const pt_scene_uniforms& s, uint64_t scene_alias_live, uint64_t sky_alias_count,

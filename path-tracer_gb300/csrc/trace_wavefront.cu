@@ -949,6 +949,7 @@ int noalloc_fail(char* error, size_t size, int code, const char* msg) {
 
 int noalloc_cuda(char* error, size_t size, cudaError_t e, const char* what) {
     if (e == cudaSuccess) return PT_OK;
+    cudaGetLastError();  // reported here: the next launch does not find it again
     if (error && size) snprintf(error, size, "%s: %s", what, cudaGetErrorString(e));
     return PT_ERR_CUDA;
 }

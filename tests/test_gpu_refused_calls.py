@@ -47,3 +47,26 @@ def test_a_refused_wave_is_launched_later(library):
                 assert eng.read(jobs[k], *sizes[k], abi.PT_TILE_ACCUMULATION).tobytes() == want[k]
         eng.close()
         """)
+
+
+def test_a_refused_launch_is_reported_once(library):
+    """The error of a refused launch is not found again by a later call that is in order."""
+    wrapped_library.run(library, """
+        world = pt.World.cornell_box()
+        u = world.take_updates()
+        images = []
+        for refused in (0, 1):
+            t = pt.PathTracer(u, (48, 32))
+            count("refuse_launch").value = refused
+            try:
+                t.trace(2)
+                assert not refused
+            except pt.PathTracerError as e:
+                assert refused and e.code == abi.PT_ERR_CUDA
+                t.apply_updates(u)
+                t.set_tile((48, 32), (0, 0), (48, 32))
+                t.trace(2)
+            images.append(t.read_tile(abi.PT_TILE_ACCUMULATION).tobytes())
+            t.close()
+        assert images[0] == images[1]
+        """)
