@@ -803,6 +803,12 @@ cudaError_t issue_any_wave(pt_engine* e, uint32_t kind, uint32_t size, uint32_t 
 int launch_wave(pt_engine* e, uint32_t kind, uint32_t paths, uint32_t rounds) {
     const uint32_t size = wave_size(paths);
     if (rounds < 1 || rounds > kRounds) rounds = kRounds;
+    // waves of the same launches share a graph: the tail kernel ends a wave at
+    // the rule's last round however deep its jobs are, and the 8-wide traversal
+    // needs no packed BVH
+    const uint32_t last = wave_rule(size).always;
+    if (last < rounds) rounds = last + 1u;
+    if (!(kind & kWaveAlpha) && (e->cfg.precision & PT_PRECISION_WIDE_BVH)) kind &= ~kWavePlain;
     cudaGraphExec_t& exec = e->graph[kind][size][rounds - 1];
     if (e->cfg.use_graphs && !exec) {
         cudaGraph_t g = nullptr;

@@ -1,4 +1,5 @@
-"""What follows when the CUDA runtime refuses a call on the host: the next call works, on the work that was asked for."""
+"""Calls of the CUDA runtime that a test has refused on the host, after which the next call works, on the work that was
+asked for; and the number of graphs that an engine makes."""
 import pytest
 
 import wrapped_library
@@ -69,4 +70,26 @@ def test_a_refused_launch_is_reported_once(library):
             images.append(t.read_tile(abi.PT_TILE_ACCUMULATION).tobytes())
             t.close()
         assert images[0] == images[1]
+        """)
+
+
+@pytest.mark.parametrize("precision", ["0", "abi.PT_PRECISION_WIDE_BVH"])
+def test_waves_of_equal_launches_share_a_graph(library, precision):
+    """Waves that the tail kernel ends are the same launches for every depth beyond its round (0 up to 2^17 paths, 1 up
+    to 2^18, 5 up to 2^21), so a depth that was not met before makes no graph."""
+    wrapped_library.run(library, f"""
+        world = pt.World.cornell_box()
+        u = world.take_updates()
+        eng = Engine(wave_paths=1 << 22, precision={precision})
+        sid = eng.add_scene(u)
+        cam = abi.Camera.from_buffer_copy(u.camera.contents)
+        made = []
+        for size, spp in (((64, 64), 4), ((128, 120), 15), ((300, 200), 16)):
+            before = count("instantiated").value
+            for depth in (0, 1, 2, 3, 4, 5, 6, 7, 9, 12, 16):
+                eng.submit(sid, cam, *size, spp, depth)
+                eng.wait_idle(timeout_ms=20000)
+            made.append(count("instantiated").value - before)
+        assert made == [1, 2, 6], made
+        eng.close()
         """)
