@@ -112,7 +112,6 @@ PTD float fract(float x) { return x - floorf(x); }
 PTD float signf(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : 0.0f); }
 PTD f3 reflect(f3 i, f3 n) { return i - (2.0f * dot(n, i)) * n; }
 PTD bool any_positive(f3 v) { return v.x > 0.0f || v.y > 0.0f || v.z > 0.0f; }
-PTD float comp(f3 v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : v.z); }
 
 // WGSL u32(f32): truncation, saturating, NaN -> 0
 PTD uint32_t to_u32(float x) { return __float2uint_rz(x); }
@@ -366,20 +365,6 @@ PTD f3 vndf_view(f3 wo, f2 a) { return normalize(mk(wo.x * a.x, wo.y * a.y, wo.z
 PTD f3 sample_vndf_sc(f3 wo, f2 a, float r, float sin_2pr, float cos_2pr) {
     const f3 ww = vndf_view(wo, a);
     return sample_vndf_ww(ww, 1.0f + ww.z, a, r, sin_2pr, cos_2pr);
-}
-// 1: sin and cos of one argument share one reduction (same bits either way)
-#ifndef PT_SHARED_SINCOS
-#define PT_SHARED_SINCOS 1
-#endif
-PTD f3 sample_vndf(f3 wo, f2 a, float r, float two_pi_r) {
-    float sn, cs;
-#if PT_SHARED_SINCOS
-    ptm::sincosf_(two_pi_r, &sn, &cs);
-#else
-    sn = ptm::sinf_(two_pi_r);
-    cs = ptm::cosf_(two_pi_r);
-#endif
-    return sample_vndf_sc(wo, a, r, sn, cs);
 }
 
 // alpha_anisotropic, trace.slang:369-375
@@ -1117,17 +1102,17 @@ PTD void dielectric_pair_fast(const DielectricTerms& t, float r1a, float tpra, f
     r = fma_(k, two(-ptm::kPio2C2), r);
     r = fma_(k, two(-ptm::kPio2C3), r);
     const Two r2 = r * r;
-    Two p = fma_(two(0x1.612462p-33f), r2, two(-0x1.ae6456p-26f));
-    p = fma_(p, r2, two(0x1.71de3ap-19f));
-    p = fma_(p, r2, two(-0x1.a01a02p-13f));
-    p = fma_(p, r2, two(0x1.111112p-7f));
-    p = fma_(p, r2, two(-0x1.555556p-3f));
+    Two p = fma_(two(ptm::kSin13), r2, two(ptm::kSin11));
+    p = fma_(p, r2, two(ptm::kSin9));
+    p = fma_(p, r2, two(ptm::kSin7));
+    p = fma_(p, r2, two(ptm::kSin5));
+    p = fma_(p, r2, two(ptm::kSin3));
     const Two si = fma_(r * r2, p, r);
-    Two c4 = fma_(two(-0x1.93974ap-37f), r2, two(0x1.1eed8ep-29f));
-    c4 = fma_(c4, r2, two(-0x1.27e4fcp-22f));
-    c4 = fma_(c4, r2, two(0x1.a01a02p-16f));
-    c4 = fma_(c4, r2, two(-0x1.6c16c2p-10f));
-    c4 = fma_(c4, r2, two(0x1.555556p-5f));
+    Two c4 = fma_(two(ptm::kCos14), r2, two(ptm::kCos12));
+    c4 = fma_(c4, r2, two(ptm::kCos10));
+    c4 = fma_(c4, r2, two(ptm::kCos8));
+    c4 = fma_(c4, r2, two(ptm::kCos6));
+    c4 = fma_(c4, r2, two(ptm::kCos4));
     const Two co = fma_(r2 * r2, c4, two(1.0f) + two(-0.5f) * r2);
     const auto quadrant = [](float u, float s, float c, float* sn, float* cs) {
         const uint32_t q = __float_as_uint(u);

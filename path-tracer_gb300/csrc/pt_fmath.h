@@ -121,25 +121,31 @@ constexpr float kLn2 = 0x1.62e430p-1f;
 constexpr float kLog2e = 0x1.715476p+0f;
 constexpr float kSqrt2 = 0x1.6a09e6p+0f;
 
+// Taylor coefficients of sin and cos, by the power of their term
+constexpr float kSin3 = -0x1.555556p-3f, kSin5 = 0x1.111112p-7f, kSin7 = -0x1.a01a02p-13f,
+                kSin9 = 0x1.71de3ap-19f, kSin11 = -0x1.ae6456p-26f, kSin13 = 0x1.612462p-33f;
+constexpr float kCos4 = 0x1.555556p-5f, kCos6 = -0x1.6c16c2p-10f, kCos8 = 0x1.a01a02p-16f,
+                kCos10 = -0x1.27e4fcp-22f, kCos12 = 0x1.1eed8ep-29f, kCos14 = -0x1.93974ap-37f;
+
 // sin(r) and cos(r) for |r| <= pi/4 (Taylor to r^13 / r^14)
 PT_HD float sin_kernel(float r) {
     const float r2 = r * r;
-    float p = 0x1.612462p-33f;
-    p = fma_(p, r2, -0x1.ae6456p-26f);
-    p = fma_(p, r2, 0x1.71de3ap-19f);
-    p = fma_(p, r2, -0x1.a01a02p-13f);
-    p = fma_(p, r2, 0x1.111112p-7f);
-    p = fma_(p, r2, -0x1.555556p-3f);
+    float p = kSin13;
+    p = fma_(p, r2, kSin11);
+    p = fma_(p, r2, kSin9);
+    p = fma_(p, r2, kSin7);
+    p = fma_(p, r2, kSin5);
+    p = fma_(p, r2, kSin3);
     return fma_(r * r2, p, r);
 }
 PT_HD float cos_kernel(float r) {
     const float r2 = r * r;
-    float p = -0x1.93974ap-37f;
-    p = fma_(p, r2, 0x1.1eed8ep-29f);
-    p = fma_(p, r2, -0x1.27e4fcp-22f);
-    p = fma_(p, r2, 0x1.a01a02p-16f);
-    p = fma_(p, r2, -0x1.6c16c2p-10f);
-    p = fma_(p, r2, 0x1.555556p-5f);
+    float p = kCos14;
+    p = fma_(p, r2, kCos12);
+    p = fma_(p, r2, kCos10);
+    p = fma_(p, r2, kCos8);
+    p = fma_(p, r2, kCos6);
+    p = fma_(p, r2, kCos4);
     const float t = 1.0f - 0.5f * r2;
     return fma_(r2 * r2, p, t);
 }

@@ -348,12 +348,7 @@ PTD bool shade_hit(const World& w, uint32_t bounce, uint32_t max_bounces, PathSt
     const float two_pi_r = kTwoPi * rng();
     const float r1 = rng();
     float sin_2pr, cos_2pr;  // every branch below uses both
-#if PT_SHARED_SINCOS
     ptm::sincosf_(two_pi_r, &sin_2pr, &cos_2pr);
-#else
-    sin_2pr = ptm::sinf_(two_pi_r);
-    cos_2pr = ptm::cosf_(two_pi_r);
-#endif
     f3 wi;
     if (rng() < b.p_ggx) {
         wi = reflect(-wo, sample_vndf_sc(wo, b.alpha, r1, sin_2pr, cos_2pr));
