@@ -156,17 +156,17 @@ def build_world():
     return world, world.take_updates()
 
 
-def algorithmic_bytes(t: dict, emissive: int, paths: int) -> dict:
+def algorithmic_bytes(t: dict, emissive: int, paths: int, node_bytes: int) -> dict:
     """Bytes the work must read or write at least once (roofline numerator), per kernel class:
-    every traversal 32 (root) + 64 per interior node (both children) + 36 per
-    triangle test; every hit 112 attribute + 224 material + 36 hit triangle;
-    every triangle-light sample 16 * (2 + ceil(log2 E)) alias entries; every
-    sky sample 2 * 12; every escaped ray 64 (bilinear sky); every path 48
-    (accumulation read + write, storage texture write)."""
+    every traversal 32 (root) + node_bytes per interior node (both children: 64 as uploaded, 32 in
+    the wavefront kernels' packed form) + 36 per triangle test; every hit 112 attribute + 224 material
+    + 36 hit triangle; every triangle-light sample 16 * (2 + ceil(log2 E)) alias entries; every sky
+    sample 2 * 12; every escaped ray 64 (bilinear sky); every path 48 (accumulation read + write,
+    storage texture write)."""
     alias = 16 * (2 + math.ceil(math.log2(max(emissive, 1))))
-    extend = (32 * t["extend_rays"] + 64 * (t["interior_visits"] - t["shadow_interior_visits"])
+    extend = (32 * t["extend_rays"] + node_bytes * (t["interior_visits"] - t["shadow_interior_visits"])
               + 36 * (t["triangle_tests"] - t["shadow_triangle_tests"]))
-    shadow = 32 * t["shadow_rays"] + 64 * t["shadow_interior_visits"] + 36 * t["shadow_triangle_tests"]
+    shadow = 32 * t["shadow_rays"] + node_bytes * t["shadow_interior_visits"] + 36 * t["shadow_triangle_tests"]
     shade = 372 * t["hits"] + alias * t["light_samples"] + 24 * t["sky_light_samples"] + 64 * t["sky_misses"]
     accumulate = 48 * paths
     total = extend + shadow + shade + accumulate
@@ -597,7 +597,8 @@ def run_ours(args):
         remaining -= n
     rays_per_step = totals["extend_rays"] + totals["shadow_rays"]
     paths_per_step = WIDTH * HEIGHT * spp
-    bytes_per_step = algorithmic_bytes(totals, emissive, paths_per_step)
+    packed = args.kernel == "wavefront" and not PRECISIONS[args.precision] & abi.PT_PRECISION_WIDE_BVH
+    bytes_per_step = algorithmic_bytes(totals, emissive, paths_per_step, 32 if packed else 64)
 
     for _ in range(max(args.warmup, 0)):
         step()
