@@ -61,12 +61,12 @@ PRECISIONS = {"fp32": 0, "wide": 1, "half": 6, "compressed": 7}
 # (1920x1080, 64 spp, FP32 form), measured by a single-pass ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum) of the first 16-spp group's
 # 9 extend launches
-TRAFFIC_PER_LAUNCH: dict = {("wavefront", "extend", "fp32"): 577.2e6}
+TRAFFIC_PER_LAUNCH: dict = {("wavefront", "extend", "fp32"): 577.3e6}
 # warp instructions per path per launch of each kernel class (smsp__inst_executed.sum of the 9 launches
 # of each class of one 960x540 16-spp image of this scene, over 9 launches x 8,294,400 paths; the
 # per-path work of a launch does not depend on the image size); with the launch's paths and its
 # CUDA-event time they give the fraction of the SMs' issue slots the kernel fills
-WARP_INST_PER_PATH: dict = {("wavefront", "fp32"): {"extend": 67.08, "shade": 30.52, "shadow": 28.67},
+WARP_INST_PER_PATH: dict = {("wavefront", "fp32"): {"extend": 66.42, "shade": 30.52, "shadow": 28.51},
                              ("wavefront", "compressed"): {"extend": 106.43, "shade": 31.14, "shadow": 33.49}}
 SMS, SCHEDULERS_PER_SM = 152, 4
 

@@ -274,8 +274,9 @@ int pt_get_stream(pt_ctx* ctx, void** stream);
 
 /* per-kernel timing with CUDA events (0 = off).  While it is on, the
  * wavefront stages of pt_trace run one after another (consecutive groups and
- * a bounce's shadow stage otherwise overlap), so each kernel's time is its
- * own; the total time of a trace is then longer than with profiling off. */
+ * a bounce's shadow stage otherwise overlap, and the rounds of small groups are
+ * finished by one kernel), so each kernel's time is its own; the total time of
+ * a trace is then longer than with profiling off. */
 #define PT_KERNEL_CLASS_COUNT 7
 #define PT_KC_RAYGEN 0
 #define PT_KC_EXTEND 1

@@ -55,7 +55,7 @@ typedef struct pt_engine_config {
     uint32_t sort_min_hits;     /* a bounce with at least this many hits sorts them by triangle bucket
                                    (1024 triangles each, BVH order) before shading; 0 = 65536,
                                    0xffffffff = never */
-    uint32_t traversal_threads; /* threads per block of the extend and shadow kernels: 64, 128 or 256
+    uint32_t traversal_threads; /* threads per block of the traversal kernels: 64, 128 or 256
                                    (the register budget per thread stays the same); 0 = 128 */
     uint32_t shade_threads;     /* threads per block of the shading kernel: 128, 256, 512 or 1024
                                    (64 registers per thread); 0 = 1024 */

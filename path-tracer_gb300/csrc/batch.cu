@@ -1,10 +1,11 @@
 // batch.cu - the batched render engine of include/pt_batch.h.
 //
 // Device side: a ring of work items (job, tile, sample range); per wave a
-// planner kernel packs queued items into the wave's path budget, then raygen
-// -> (extend -> shade -> shadow) x 17 rounds -> accumulate run over every
-// path of the wave, each path looking up its job and scene.  The whole wave
-// is one captured CUDA graph.  Host side: the scene cache (content hash, HBM
+// planner kernel takes the items that the host fed for it, then raygen ->
+// (trace -> shade) x the rounds of its deepest job -> accumulate run over every
+// path of the wave, each path looking up its job and scene; a round's shadow
+// rays are traced with the next round's rays, and the last rounds run as one
+// tail kernel.  The whole wave is one captured CUDA graph.  Host side: the scene cache (content hash, HBM
 // budget, LRU eviction), jobs and their resident accumulation buffers, the
 // ring producer, wave launching and completion polling, and the autotuner.
 #include <atomic>
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(kThreads, blocks_for(PT_SHADE_MIN_BLOCKS, kSha
         PathState ps;
         uint32_t p = 0, rs = 0;
         if (i != 0xffffffffu) {
-            // the entries before miss_span are misses (the extend kernel filed them so): no hit record to read
+            // the entries before miss_span are misses (the trace kernel filed them so): no hit record to read
             const bool miss = base + lane < range.miss_span;
             const float4 o4 = st.o[i], d4 = st.d[i], t4 = st.T[i];
             const float4 h4 = miss ? make_float4(0.0f, __int_as_float(-1), 0.0f, 0.0f) : b.q.hit[i];

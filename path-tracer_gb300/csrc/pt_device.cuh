@@ -64,8 +64,10 @@ PTD float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 // The same bits as 1 / b, a / b and sqrtf(x) where no step leaves the normal
 // range: |b| in [2^-120, 2^120]; for a quotient b > 0 or a not +0 (the sign of
 // a zero quotient), |b| in [2^-60, 2^60], and a zero or |a| and |a / b| in
-// [2^-100, 2^100]; x in [2^-96, 2^126].  Checked against the operators over
-// every significand (tests/test_gpu_fast_math.py).
+// [2^-100, 2^100]; x in [2^-96, 2^126].  Checked against the operators: the
+// reciprocal and the root over every significand and exponent
+// (tests/test_gpu_fast_math.py), the quotient and the packed forms over 10^9
+// random and hard ones of the whole range (tests/test_gpu_quotients.py).
 PTD float rcp_in_range(float b) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));

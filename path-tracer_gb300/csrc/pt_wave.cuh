@@ -36,7 +36,7 @@ struct Queues {
     uint32_t* miss_list;  // slots whose ray left the scene
     uint32_t* hit_sorted = nullptr;  // the hit list sorted by key (when the round's kCntSorted != 0)
     // beside the hit list, each filed hit's triangle-bucket sort key (triangle
-    // >> key_shift, at most the last bucket), written by the extend kernel so
+    // >> key_shift, at most the last bucket), written by the trace kernel so
     // that the sort reads its keys in order instead of gathering the hit
     // records; null: the sort computes the keys itself
     uint32_t* hit_keys = nullptr;
@@ -91,7 +91,9 @@ PTD void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #ifndef PT_EXTEND_THREADS
 #define PT_EXTEND_THREADS 128
 #endif
-// 9 resident blocks of the traversal kernels per SM: at most 56 registers, no spills
+// 9 resident blocks of the traversal kernels per SM: 56 registers (the packed
+// traversal spills 60 bytes stored, 36 loaded a thread for it, the engine's 80 and
+// 40; with 8 blocks of 64 registers it is slower, see PackedRay)
 #ifndef PT_EXTEND_MIN_BLOCKS
 #define PT_EXTEND_MIN_BLOCKS 9
 #endif
@@ -1072,7 +1074,7 @@ constexpr uint32_t kSortBuckets = PT_SORT_BUCKETS;  // a multiple of 1024, at mo
 static_assert(kSortBuckets % 1024 == 0 && kSortBuckets <= 8192, "sort buckets: 1024 .. 8192 in steps of 1024");
 constexpr uint32_t kSortPerThread = kSortBuckets / 1024;
 
-// Files finished extend rays under hits (with their record and sort key) or
+// Files finished rays of a round under hits (with their record and sort key) or
 // misses, so that the shading kernel runs warps of hits only and warps of
 // misses only, and takes the warp's next queue entries: the three reservations
 // (hit list, miss list, ray queue) are one atomic instruction of three lanes,
@@ -1439,7 +1441,11 @@ PTD void traverse_warp(Ray& ray, S& stack) {
 // scheduler, would else each fetch the 40 KB of shading instructions by
 // themselves (half of all stalls; 160x120 paths of the room 276 us without the
 // barrier, 260 with one of each scheduler's warps, 241 with this one).
-// 128 registers, 16 warps an SM; 24 warps of 80 registers were slower.
+// 128 registers, 16 warps an SM; 24 warps of 80 registers were slower.  What a
+// warp waits for now, in cycles an instruction: the block's longest ray, at the
+// barrier (9.3 of 13.8 in the room, 4.0 of 10.7 in 640x360 of 100k triangles),
+// its own loads (0.6, 2.6), fixed latencies (2.0, 2.0), instruction fetch (0.9,
+// 0.7); 26 and 33 % of the issue slots.
 // `env` gives a path's scene, world and bounces; all threads of the block.
 template <bool kAlpha, class Ray, class S, class Env>
 PTD void finish_paths(const Env& env, const Queues& q, uint32_t first_round, Ray& ray, S& stack) {
@@ -1558,17 +1564,36 @@ constexpr uint32_t kUnsortedPaths = 1u << 18;
 
 // The rounds from which a group's paths are finished by the tail kernel: from
 // `first` on when a round has at most `hits` hits, from `always` on in any
-// case.  Up to 2^17 paths the rounds' launches and longest rays cost more than
-// their better use of lanes gives, from the start (a frame of 160x120 paths of
-// the room: 237 us from round 0, 258 from 2, 397 never; 100x70x16 of 10k
-// triangles 360, 403, 560), up to 2^18 from round 1 (640x360 of 100k triangles
-// 841 from 0, 795 from 1, 810 from 2, 1140 never).  Above that the full rounds
-// go faster as launches of their own; after round 4 Russian roulette has ended
-// most paths (256x256x16 of the room 1352 from 4, 1258 from 5, 1310 never), and
-// open scenes thin out earlier (481x271x8 of 10k triangles with coverage 1172
-// with the rule's hits, 1205 with 2^15, 1288 from round 5, 1535 never;
-// 960x540x4 of 1M triangles 3611, 4100 with 2^18, 3784 never).  Groups of over
-// 2^21 paths overlap with one another, and at 2^22 the gain is -2 to 3 %.
+// case.  Few paths: a round's launches and its longest ray cost more than the
+// better use of lanes gives, from the start.  More: the full rounds go faster
+// as launches of their own; after round 4 Russian roulette has ended most
+// paths, and open scenes thin out earlier.  The lines lie where these cross
+// (us a frame, 8 bounces, max. 8 or 1 samples a pixel; 152 SMs):
+//
+//   scene, paths              from 0  from 1  from 2  2^17 hits, 5  never
+//   room             65,536      270     273     290            307    391
+//   10k, coverage    98,304      466     453     477            499    742
+//   100k             98,304      585     586     619            642    866
+//   1M               98,304      783     826     883            913  1,218
+//   room            131,072      393     387     351            370    424
+//   100k            131,072      630     612     640            661    897
+//   1M              131,072      925     905     975            992  1,263
+//   100k            163,840      684     623     664            685    906
+//   10k, coverage   262,144      653     558     580            609    865
+//   100k            262,144      882     769     777            798  1,006
+//   1M              262,144    1,294   1,161   1,115          1,154  1,443
+//   room, 1 sample  327,680      632     590     577            609    583
+//   100k            327,680      949     851     825            855  1,088
+//   1M              524,288    2,323   1,935   1,778          1,828  1,925
+//   room          2,097,152    2,107   1,794   1,604          1,257  1,299
+//   1M            2,097,152    6,971   5,171   4,400          3,494  3,699
+//   10k, coverage 2,621,440    3,986   2,469   2,193          2,246  2,497
+//   room          4,194,304    7,652   6,385   5,470          3,732  3,670
+//   1M            4,194,304   14,954  10,894   8,928          6,093  6,228
+//
+// (2^15 hits and 2^18 instead of 2^17: 481x271x8 of 10k triangles with coverage
+// 1205 against 1172, 960x540x4 of 1M 4100 against 3611.)  Groups of over 2^21
+// paths overlap with one another.
 // Beside other groups the tail's blocks, which fill their SMs at a third of the
 // rate, are in the way: four groups of 128x128x16 paths of the room 1605 us
 // without it, 2089 with; up to 2^16 paths a group they still gain (four of

@@ -8,7 +8,9 @@
 //               (trace.slang:887-1296); appends continuing rays to the next
 //               queue and NEE shadow rays to the shadow queue
 //   shadow      any-hit traversal (trace.slang:614-717); adds unoccluded
-//               light contributions
+//               light contributions (by the launch that extends the next
+//               bounce's rays)
+//   tail        a bounce's paths to their ends, in groups of few paths
 //   accumulate  per pixel, samples in order (trace.slang:1299-1308)
 // Queue lengths live on the device; the host never waits between stages.
 #pragma once

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == kShadeThreads ? PT_SHADE
         PathState ps;
         uint32_t p = 0, rs = 0;
         if (i != 0xffffffffu) {
-            // the entries before miss_span are misses (the extend kernel filed them so): no hit record to read
+            // the entries before miss_span are misses (the trace kernel filed them so): no hit record to read
             const bool miss = base + lane < range.miss_span;
             const float4 o4 = st.o[i], d4 = st.d[i], t4 = st.T[i];
             const float4 h4 = miss ? make_float4(0.0f, __int_as_float(-1), 0.0f, 0.0f) : q.hit[i];
@@ -648,7 +648,7 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
     const auto tracer = trace_kernel<kRec, kAlpha, kTri36, kWide, kPacked>;
     const auto shader = shade_kernel<kRec, kAlpha, false, kShadeThreads>;
     uint32_t trace_blocks = (uint32_t)sms * resident_blocks(tracer, kExtendThreads);
-    // 8 rays a warp at least (usable_lanes)
+    // 8 rays a warp at least (QueueShare)
     if (small) trace_blocks = std::min(trace_blocks, (g.paths + kExtendThreads / 4 - 1) / (kExtendThreads / 4));
     PTW_TRY(timer(PT_KC_RAYGEN, stream, [&] {
         const uint32_t blocks = (std::max(g.paths, kCounterWords) + 255u) / 256u;
@@ -810,7 +810,7 @@ cudaError_t trace(Wavefront* wf, const ptd::World& w_in, const ptk::Tile& tile, 
         sort.counts = q.hit_sorted + wf->capacity;  // kSortBuckets counts, then kSortBuckets offsets
         sort.min_hits = PT_SORT_MIN_HITS;
         while (((uint64_t)ptd::kSortBuckets << sort.tri_shift) < wf->tri_count && sort.tri_shift < 31u) sort.tri_shift += 1u;
-        if (PT_SORT_KEY == 1) {  // the extend kernel files each hit's bucket beside the hit list
+        if (PT_SORT_KEY == 1) {  // the trace kernel files each hit's bucket beside the hit list
             q.hit_keys = sort.counts + 2 * ptd::kSortBuckets;
             q.key_shift = sort.tri_shift;
         }
