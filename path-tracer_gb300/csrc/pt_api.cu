@@ -882,11 +882,18 @@ int pt_display_tile(pt_ctx* c, uint8_t* host_rgba8) try {
 int pt_synchronize(pt_ctx* c, uint32_t timeout_ms) try {
     if (!c) return PT_ERR_INVALID_ARG;
     cudaSetDevice(c->device);
-    if (timeout_ms == 0) return c->cuda(cudaStreamSynchronize(c->stream), "synchronize");
+    // (nothing is left that the next trace could overlap)
+    if (timeout_ms == 0) {
+        c->touched();
+        return c->cuda(cudaStreamSynchronize(c->stream), "synchronize");
+    }
     const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(timeout_ms);
     for (;;) {
         const cudaError_t e = cudaStreamQuery(c->stream);
-        if (e == cudaSuccess) return PT_OK;
+        if (e == cudaSuccess) {
+            c->touched();
+            return PT_OK;
+        }
         if (e != cudaErrorNotReady) return c->cuda(e, "synchronize");
         if (std::chrono::steady_clock::now() >= deadline) return c->fail(PT_ERR_TIMEOUT, "queued work did not finish in time");
         std::this_thread::sleep_for(std::chrono::microseconds(200));

@@ -1568,7 +1568,7 @@ constexpr uint32_t kUnsortedPaths = 1u << 18;
 // better use of lanes gives, from the start.  More: the full rounds go faster
 // as launches of their own; after round 4 Russian roulette has ended most
 // paths, and open scenes thin out earlier.  The lines lie where these cross
-// (us a frame, 8 bounces, max. 8 or 1 samples a pixel; 152 SMs):
+// (us a frame, 8 bounces, 1 to 16 samples a pixel; 152 SMs):
 //
 //   scene, paths              from 0  from 1  from 2  2^17 hits, 5  never
 //   room             65,536      270     273     290            307    391

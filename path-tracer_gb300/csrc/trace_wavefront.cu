@@ -624,6 +624,16 @@ struct SortCfg {
 #ifndef PT_SMALL_PATHS
 #define PT_SMALL_PATHS (1u << 20)
 #endif
+// Beside other groups, which fill the SMs, spread hits only add work: from 2^15
+// paths on (us a group of 32 in a row, with and without: 128x128x1 of 1M triangles
+// 342, 355; 256x256x1 562, 556; 256x256x2 of 1M 750, 693, of 100k 520, 461, of the
+// room 270, 239, of 1M in the 8-wide form 924, 809; 640x360x1 there 1045, 955).  With
+// coverage the shading's chain has the shadow rays in it and pays up to 2^18
+// (320x256x1 325, 353; 640x360x1 415, 432; 800x600x1 601, 601; 1280x720x1 856, 831).
+constexpr uint32_t kSmallBeside = 1u << 15, kSmallBesideCoverage = 1u << 18;
+uint32_t small_paths(bool alone, bool coverage) {
+    return alone ? PT_SMALL_PATHS : coverage ? kSmallBesideCoverage : kSmallBeside;
+}
 constexpr int kSmallShadeThreads = 128;
 
 // One group of paths through raygen, max_bounces + 1 rounds of trace / (hit
@@ -644,7 +654,7 @@ cudaError_t run_group(int sms, const ptd::World& w, const ptd::Fast& f, const pt
                       TimerF&& timer, bool alone, bool serial, const SortCfg& sort = SortCfg(), cudaStream_t acc_stream = nullptr,
                       cudaEvent_t done = nullptr) {
     using namespace ptd;
-    const bool small = !kRec && g.paths <= PT_SMALL_PATHS;
+    const bool small = !kRec && g.paths <= small_paths(alone, kAlpha);
     const auto tracer = trace_kernel<kRec, kAlpha, kTri36, kWide, kPacked>;
     const auto shader = shade_kernel<kRec, kAlpha, false, kShadeThreads>;
     uint32_t trace_blocks = (uint32_t)sms * resident_blocks(tracer, kExtendThreads);
