@@ -594,6 +594,7 @@ struct pt_engine {
     Buf d_jobs, d_done;
     uint32_t* h_done = nullptr;  // pinned mirror of the per-slot finished-item counters
     Ctrl* h_ctrl = nullptr;      // pinned mirror of the ring control block
+    uint32_t* h_plain = nullptr;  // mapped: the uploaded scene's nodes that a packed BVH would hold no planes of
     std::map<uint64_t, Job> jobs;
     uint64_t next_job = 1;
     std::deque<uint64_t> done_unreported;
@@ -1109,7 +1110,9 @@ int upload_scene(pt_engine* e, Scene& s, const pt_world_updates* u) {
     }
     if (!rc) rc = put(s.lut, lut, sizeof lut, "sRGB table");
     if (!rc && s.packable) {
-        rc = e->cuda(s.packed.alloc(packed_bytes(sc->node_count)), "packed BVH");
+        *e->h_plain = 0u;
+        rc = e->cuda(ptw::count_plain(s.nodes.as<pt_bvh_node>(), sc->node_count, e->h_plain, e->stream), "packed BVH");
+        if (!rc) rc = e->cuda(s.packed.alloc(packed_bytes(sc->node_count)), "packed BVH");
         if (!rc) rc = e->cuda(ptw::pack_bvh(s.nodes.as<pt_bvh_node>(), sc->node_count, s.packed.as<float4>(), e->stream), "packed BVH");
     }
     if (!rc) rc = e->cuda(s.tri4.alloc(sc->triangle_count * 16 * ptd::kTriStride), "triangle layout");
@@ -1150,6 +1153,8 @@ int upload_scene(pt_engine* e, Scene& s, const pt_world_updates* u) {
     rc = e->cuda(cudaMemcpyAsync(e->d_scenes.as<SceneDev>() + s.slot, &d, sizeof d, cudaMemcpyHostToDevice, e->stream),
                  "scene record");
     if (!rc) rc = e->cuda(cudaStreamSynchronize(e->stream), "scene upload");
+    // (waves of a scene that is not packable read no packed BVH: it stays where it is)
+    if (!rc && s.packable) s.packable = ptw::packable(sc->node_count, sc->node_count, sc->triangle_count, 0u, *e->h_plain);
     return rc;
 }
 
@@ -1259,6 +1264,7 @@ int pte_create(const pt_engine_config* cfg, pt_engine** out) try {
     if (!rc) rc = e->cuda(cudaMemset(e->d_ctrl.p, 0, sizeof(Ctrl)), "ring control");
     if (!rc) rc = e->cuda(cudaHostAlloc((void**)&e->h_done, (size_t)kMaxSlots * 4, cudaHostAllocDefault), "pinned counters");
     if (!rc) rc = e->cuda(cudaHostAlloc((void**)&e->h_ctrl, sizeof(Ctrl), cudaHostAllocDefault), "pinned counters");
+    if (!rc) rc = e->cuda(cudaHostAlloc((void**)&e->h_plain, sizeof(uint32_t), cudaHostAllocMapped), "pinned counters");
     if (!rc) {
         memset(e->h_done, 0, (size_t)kMaxSlots * 4);
         memset(e->h_ctrl, 0, sizeof(Ctrl));
@@ -1305,6 +1311,7 @@ void pte_destroy(pt_engine* e) {
     if (e->pool) cudaMemPoolDestroy(e->pool);
     if (e->h_done) cudaFreeHost(e->h_done);
     if (e->h_ctrl) cudaFreeHost(e->h_ctrl);
+    if (e->h_plain) cudaFreeHost(e->h_plain);
     if (e->stream) cudaStreamDestroy(e->stream);
     delete e;
 }
@@ -1436,7 +1443,7 @@ int pte_scene_add(pt_engine* e, const pt_world_updates* u, uint64_t* scene_id) t
     s->caller_refs = 1;
     s->last_use = e->use_clock;
     s->any_alpha = any_alpha;
-    s->packable = ptw::packable(sc->node_count, tree_nodes, sc->triangle_count, max_leaf);
+    s->packable = ptw::packable(sc->node_count, tree_nodes, sc->triangle_count, max_leaf, 0u);  // by its shape
     int rc = upload_scene(e, *s, u);
     if (rc) return rc;
     e->scene_slots[slot] = h;

@@ -65,6 +65,7 @@ struct pt_ctx {
     DevBuf geo, attr, mat, nodes, srgb, linear, sky, sky_alias, scene_alias, srgb_lut;
     DevBuf stage_geo, stage_attr, stage_mat, stage_nodes, stage_srgb, stage_linear;  // next scene upload
     DevBuf check;  // its validation: the result and each node's parent
+    uint32_t* plain_nodes = nullptr;  // mapped host memory: its nodes that a packed BVH would hold no planes of
     uint64_t tri_count = 0, mat_count = 0, node_count = 0, sky_alias_count = 0, scene_alias_live = 0;
     uint32_t srgb_count = 0, linear_count = 0;
     pt_camera camera{};
@@ -456,6 +457,16 @@ int apply(pt_ctx* c, const pt_world_updates* u, bool initial) {
                 return rc;
             }
             staged = true;
+            // counted beside the host's work; read when the stream has finished
+            if (!c->plain_nodes) rc = c->cuda(cudaHostAlloc((void**)&c->plain_nodes, sizeof(uint32_t), cudaHostAllocMapped), "BVH");
+            if (!rc) {
+                *c->plain_nodes = 0u;
+                rc = c->cuda(ptw::count_plain(c->stage_nodes.as<pt_bvh_node>(), s->node_count, c->plain_nodes, c->stream), "BVH");
+            }
+            if (rc) {
+                cudaStreamSynchronize(c->stream);
+                return rc;
+            }
         }
     }
     // ---- validate everything before touching the live device state
@@ -579,8 +590,8 @@ int apply(pt_ctx* c, const pt_world_updates* u, bool initial) {
         c->alpha_modes.resize(s->material_count);
         for (uint64_t i = 0; i < s->material_count; ++i) c->alpha_modes[i] = s->materials[i].alpha_mode;
         c->scene_alias_live = 0;
-        c->packable = ptw::packable(s->node_count, tree_nodes, s->triangle_count, max_leaf);
-        if (c->wavefront) ptw::world_changed(c->wavefront, c->packable);
+        c->packable = false;  // until the count of its plain nodes is there
+        if (c->wavefront) ptw::world_changed(c->wavefront, false);
     }
     if (const pt_skybox_upload* k = u->skybox) {
         const size_t px = (size_t)k->uniforms.width * k->uniforms.height;
@@ -611,6 +622,10 @@ int apply(pt_ctx* c, const pt_world_updates* u, bool initial) {
     // host pointers are borrowed for this call only
     rc = c->cuda(cudaStreamSynchronize(c->stream), "world upload");
     if (rc) return rc;
+    if (const pt_scene_upload* s = u->scene) {
+        c->packable = ptw::packable(s->node_count, tree_nodes, s->triangle_count, max_leaf, *c->plain_nodes);
+        if (c->wavefront) ptw::world_changed(c->wavefront, c->packable);
+    }
     c->world_ready = true;
     return PT_OK;
 }
@@ -775,6 +790,7 @@ void pt_destroy(pt_ctx* c) {
                       &c->scene_alias, &c->srgb_lut, &c->accum, &c->image, &c->comp, &c->fp64, &c->display, &c->records, &c->totals,
                       &c->stage_geo, &c->stage_attr, &c->stage_mat, &c->stage_nodes, &c->stage_srgb, &c->stage_linear, &c->check})
         b->release();
+    if (c->plain_nodes) cudaFreeHost(c->plain_nodes);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }

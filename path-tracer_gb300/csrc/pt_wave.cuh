@@ -542,6 +542,24 @@ __global__ void __launch_bounds__(256) pack_bvh_kernel(const float4* nodes, uint
     r[1] = make_float4(hi[0], hi[1], hi[2], __uint_as_float(pack_ref(nodes, node_count, l + 1u) | own_hi));
 }
 
+// Adds to *plain (in host memory or on the device) the interior nodes that would
+// be records without planes; the nodes may be anything.
+template <int kUnused>
+__global__ void __launch_bounds__(256) count_plain_kernel(const float4* nodes, uint64_t node_count, uint32_t* plain) {
+    __shared__ uint32_t sum;
+    if (threadIdx.x == 0u) sum = 0u;
+    __syncthreads();
+    uint32_t mine = 0u;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < node_count; i += (uint64_t)gridDim.x * blockDim.x) {
+        float lo[3], hi[3];
+        uint32_t a, b;
+        if (__float_as_uint(nodes[2 * i + 1].w) == 0u && !pack_planes(nodes, node_count, i, lo, hi, &a, &b)) mine += 1u;
+    }
+    if (mine) atomicAdd(&sum, mine);
+    __syncthreads();
+    if (threadIdx.x == 0u && sum) atomicAdd_system(plain, sum);
+}
+
 // bytes of the packed BVH of a tree
 constexpr size_t packed_bytes(uint64_t nodes) { return 32 + 32 * (nodes / 2 + 1); }
 

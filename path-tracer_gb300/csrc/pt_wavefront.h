@@ -31,8 +31,11 @@ void destroy(Wavefront* wf);
 void world_changed(Wavefront* wf, bool packable);
 
 // whether a BVH whose `reached` nodes hang off the root, with at most
-// max_leaf triangles in a leaf, can be packed
-bool packable(uint64_t nodes, uint64_t reached, uint64_t tris, uint32_t max_leaf);
+// max_leaf triangles in a leaf and `plain` interior nodes whose record would
+// hold no planes (count_plain), is to be packed
+bool packable(uint64_t nodes, uint64_t reached, uint64_t tris, uint32_t max_leaf, uint32_t plain);
+// adds the number of those nodes to *plain (device memory, or mapped host memory) on `stream`
+cudaError_t count_plain(const pt_bvh_node* nodes, uint64_t n, uint32_t* plain, cudaStream_t stream);
 // the packed BVH of a packable tree, on `stream` (ptd::packed_bytes bytes)
 cudaError_t pack_bvh(const pt_bvh_node* nodes, uint64_t n, float4* packed, cudaStream_t stream);
 

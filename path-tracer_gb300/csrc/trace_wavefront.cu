@@ -888,8 +888,22 @@ cudaError_t convert_half_attributes(const pt_triangle_attribute* in, uint64_t n,
     return cudaGetLastError();
 }
 
-bool packable(uint64_t nodes, uint64_t reached, uint64_t tris, uint32_t max_leaf) {
-    return reached == nodes && nodes < ptd::kPackedMaxNodes && tris < ptd::kPackedMaxTris && max_leaf <= ptd::kPackedMaxLeaf;
+// Nodes without planes are visited from the uploaded boxes, in a turn of their
+// own, and cost more than the packed ones save from one in 64 interior nodes
+// (half of the nodes) on.  Calls in a row, us, packed and on the uploaded nodes:
+// 640x360x4 of 496k triangles, none of the nodes plain 942, 952; 3 % 1023, 955;
+// 12 % 1135, 956; 49 % 1385, 971; 1280x720x8 4644, 4817; 5076, 4827; of 18k
+// triangles 653, 652; 688, 648.  The framework's builders make none.
+bool packable(uint64_t nodes, uint64_t reached, uint64_t tris, uint32_t max_leaf, uint32_t plain) {
+    return reached == nodes && nodes < ptd::kPackedMaxNodes && tris < ptd::kPackedMaxTris &&
+           max_leaf <= ptd::kPackedMaxLeaf && 128ull * plain <= nodes;
+}
+
+cudaError_t count_plain(const pt_bvh_node* nodes, uint64_t n, uint32_t* plain, cudaStream_t stream) {
+    const uint64_t blocks = std::min<uint64_t>((n + 255) / 256, 1024);
+    if (blocks == 0) return cudaSuccess;
+    ptd::count_plain_kernel<0><<<(unsigned)blocks, 256, 0, stream>>>(reinterpret_cast<const float4*>(nodes), n, plain);
+    return cudaGetLastError();
 }
 
 cudaError_t pack_bvh(const pt_bvh_node* nodes, uint64_t n, float4* packed, cudaStream_t stream) {
