@@ -161,6 +161,16 @@ struct pt_ctx {
     // previous call's groups (ctx_ops counts such work).
     uint64_t ctx_ops = 0, ops_at_trace = ~0ull;
     void touched() { ctx_ops += 1; }
+    // A synchronisation leaves nothing that the next trace could overlap.  A
+    // program that synchronises after each call is taken to go on so: its next
+    // call is alone.  (After several calls in a row the next ones are expected to
+    // overlap: alone, the first would hold up the others, 3 calls of 256x256x16 of
+    // 10k triangles with coverage 2950 -> 3164 us.)
+    uint64_t calls = 0;  // traces since the last synchronisation
+    void synchronized() {
+        if (calls == 1) touched();
+        calls = 0;
+    }
     void harvest() {
         for (Timing& t : pending) {
             cudaEventSynchronize(t.stop);
@@ -672,6 +682,7 @@ int trace_impl(pt_ctx* c, uint32_t samples, uint32_t* traced, pt_path_record* ho
     const uint32_t n = samples < PT_MAX_SAMPLES_PER_TRACE ? samples : PT_MAX_SAMPLES_PER_TRACE;
     if (traced) *traced = 0;
     if (n == 0) return PT_OK;
+    c->calls += 1;
     const ptd::World w = c->view();
     const ptk::Tile t = tile_of(c);
     const size_t tile_px = (size_t)c->tile_w * c->tile_h;
@@ -898,16 +909,15 @@ int pt_display_tile(pt_ctx* c, uint8_t* host_rgba8) try {
 int pt_synchronize(pt_ctx* c, uint32_t timeout_ms) try {
     if (!c) return PT_ERR_INVALID_ARG;
     cudaSetDevice(c->device);
-    // (nothing is left that the next trace could overlap)
     if (timeout_ms == 0) {
-        c->touched();
+        c->synchronized();
         return c->cuda(cudaStreamSynchronize(c->stream), "synchronize");
     }
     const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(timeout_ms);
     for (;;) {
         const cudaError_t e = cudaStreamQuery(c->stream);
         if (e == cudaSuccess) {
-            c->touched();
+            c->synchronized();
             return PT_OK;
         }
         if (e != cudaErrorNotReady) return c->cuda(e, "synchronize");
