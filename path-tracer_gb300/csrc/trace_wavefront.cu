@@ -628,9 +628,10 @@ struct SortCfg {
 // paths on (us a group of 32 in a row, with and without: 128x128x1 of 1M triangles
 // 342, 355; 256x256x1 562, 556; 256x256x2 of 1M 750, 693, of 100k 520, 461, of the
 // room 270, 239, of 1M in the 8-wide form 924, 809; 640x360x1 there 1045, 955).  With
-// coverage the shading's chain has the shadow rays in it and pays up to 2^18
-// (320x256x1 325, 353; 640x360x1 415, 432; 800x600x1 601, 601; 1280x720x1 856, 831).
-constexpr uint32_t kSmallBeside = 1u << 15, kSmallBesideCoverage = 1u << 18;
+// coverage the shading's chain has the shadow rays in it and pays up to 2^19
+// (10k triangles, 3 calls a synchronisation: 100x200x16 512, 549; 800x600x1 615, 647;
+// 800x800x1 755, 737; 32: 320x256x1 326, 351; 800x600x1 601, 596; 1000x960x1 936, 893).
+constexpr uint32_t kSmallBeside = 1u << 15, kSmallBesideCoverage = 1u << 19;
 uint32_t small_paths(bool alone, bool coverage) {
     return alone ? PT_SMALL_PATHS : coverage ? kSmallBesideCoverage : kSmallBeside;
 }

@@ -1,5 +1,5 @@
 """Calls in a row, whose groups overlap, and calls after a synchronisation, whose groups run alone: on both sides of the
-sizes at which a hit's lanes share its shading (2^15 paths beside other groups, 2^18 with coverage materials, 2^20
+sizes at which a hit's lanes share its shading (2^15 paths beside other groups, 2^19 with coverage materials, 2^20
 alone), in every form.  Against the plain kernel, bit for bit."""
 import pytest
 
@@ -19,7 +19,7 @@ def worlds():
 @pytest.mark.parametrize("synchronised", [False, True])
 @pytest.mark.parametrize("scene,precision,size,spp", [
     ("room", 0, (128, 16), 16), ("room", 0, (129, 16), 16), ("room", abi.PT_PRECISION_WIDE_BVH, (129, 16), 16),
-    ("coverage", 0, (128, 128), 16), ("coverage", 0, (129, 128), 16), ("room", 0, (256, 256), 16), ("room", 0, (257, 256), 16)])
+    ("coverage", 0, (256, 128), 16), ("coverage", 0, (257, 128), 16), ("room", 0, (256, 256), 16), ("room", 0, (257, 256), 16)])
 def test_equal_to_the_plain_kernel(worlds, scene, precision, size, spp, synchronised):
     out = []
     for kernel in (abi.PT_KERNEL_PLAIN, abi.PT_KERNEL_WAVEFRONT):
