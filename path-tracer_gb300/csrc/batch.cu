@@ -709,8 +709,8 @@ int setup_wave(pt_engine* e) {
 
 // one launch of a persistent stage kernel: the blocks that stay resident on every SM
 template <class... P, class... A>
-void launch_persistent(void (*kernel)(P...), pt_engine* e, uint32_t threads, A&&... args) {
-    launch_after(kernel, (uint32_t)e->sms * resident_blocks(kernel, (int)threads), threads, e->stream, std::forward<A>(args)...);
+cudaError_t launch_persistent(void (*kernel)(P...), pt_engine* e, uint32_t threads, A&&... args) {
+    return launch_after(kernel, (uint32_t)e->sms * resident_blocks(kernel, (int)threads), threads, e->stream, std::forward<A>(args)...);
 }
 
 // The sizes of waves that differ in their launches: the most paths of each.
@@ -733,7 +733,14 @@ TailRule wave_rule(uint32_t size) {
     return r;
 }
 
-// the launches of one wave (captured into a graph, or issued directly)
+#define PTB_TRY(x)                        \
+    do {                                  \
+        const cudaError_t e_ = (x);       \
+        if (e_ != cudaSuccess) return e_; \
+    } while (0)
+
+// the launches of one wave (captured into a graph, or issued directly); none
+// after one that is refused, whose queues the next would read
 template <bool kAlpha, bool kWideBvh, bool kPacked>
 cudaError_t issue_wave(pt_engine* e, uint32_t size, uint32_t rounds) {
     const cudaStream_t s = e->stream;
@@ -743,7 +750,8 @@ cudaError_t issue_wave(pt_engine* e, uint32_t size, uint32_t rounds) {
     const JobDev* jobs = e->d_jobs.as<const JobDev>();
     const uint32_t per_wave_blocks = (uint32_t)e->sms * 8u;
     plan_kernel<<<1, 1024, 0, s>>>(ctrl, ring, e->ring_cap, e->wb);
-    launch_after(raygen_kernel, per_wave_blocks, 256u, s, ctrl, ring, jobs, e->wb);
+    PTB_TRY(cudaGetLastError());
+    PTB_TRY(launch_after(raygen_kernel, per_wave_blocks, 256u, s, ctrl, ring, jobs, e->wb));
     constexpr bool kWide = kWideBvh && !kAlpha;
     const uint32_t tt = e->cfg.traversal_threads, st = e->cfg.shade_threads;
     // persistent launches: as many blocks as stay resident, for the block shape of the configuration
@@ -764,32 +772,31 @@ cudaError_t issue_wave(pt_engine* e, uint32_t size, uint32_t rounds) {
     const TailRule rule = wave_rule(size);
     bool finished = false;
     for (uint32_t round = 0; round < rounds; ++round) {
-        trace(round);
+        PTB_TRY(trace(round));
         uint32_t tail_hits = 0u;
         if (round >= rule.first) {
             finished = round >= rule.always;
             tail_hits = rule.hits;
-            launch_after(tail_kernel<kAlpha, kWide, kPacked>, (uint32_t)e->sms, (uint32_t)kTailThreads, s, scenes, jobs, e->wb,
-                         round, finished ? 0xffffffffu : rule.hits);
+            PTB_TRY(launch_after(tail_kernel<kAlpha, kWide, kPacked>, (uint32_t)e->sms, (uint32_t)kTailThreads, s, scenes, jobs,
+                                 e->wb, round, finished ? 0xffffffffu : rule.hits));
             if (finished) break;
         }
         const uint32_t sort_hits = std::max(e->cfg.sort_min_hits, tail_hits + 1u);
         if (e->cfg.sort_min_hits != 0xffffffffu && wave_sizes[size] > kUnsortedPaths) {
             // hits of all jobs by triangle bucket (1024 triangles per bucket)
-            launch_after(sort_count_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round, e->sort_counts,
-                         sort_hits, kEngineSortShift);
-            launch_after(sort_scan_kernel<0>, 1u, 1024u, s, e->wb.q, round, e->sort_counts, e->sort_counts + kSortBuckets,
-                         sort_hits);
-            launch_after(sort_scatter_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round,
-                         e->sort_counts + kSortBuckets, sort_hits, kEngineSortShift);
+            PTB_TRY(launch_after(sort_count_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round,
+                                 e->sort_counts, sort_hits, kEngineSortShift));
+            PTB_TRY(launch_after(sort_scan_kernel<0>, 1u, 1024u, s, e->wb.q, round, e->sort_counts,
+                                 e->sort_counts + kSortBuckets, sort_hits));
+            PTB_TRY(launch_after(sort_scatter_kernel<1>, (uint32_t)e->sms * 4u, kSortThreads, s, World{}, e->wb.q, round,
+                                 e->sort_counts + kSortBuckets, sort_hits, kEngineSortShift));
         }
-        shade(round, tail_hits);
+        PTB_TRY(shade(round, tail_hits));
     }
-    if (!kAlpha && !finished) trace(rounds);  // the last round's shadow rays
-    launch_after(accumulate_kernel, per_wave_blocks, 256u, s, ctrl, ring, jobs, e->wb, e->d_done.as<uint32_t>());
-    cudaMemcpyAsync(e->h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
-    cudaMemcpyAsync(e->h_done, e->d_done.p, kMaxSlots * 4, cudaMemcpyDeviceToHost, s);
-    return cudaGetLastError();
+    if (!kAlpha && !finished) PTB_TRY(trace(rounds));  // the last round's shadow rays
+    PTB_TRY(launch_after(accumulate_kernel, per_wave_blocks, 256u, s, ctrl, ring, jobs, e->wb, e->d_done.as<uint32_t>()));
+    PTB_TRY(cudaMemcpyAsync(e->h_ctrl, ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s));
+    return cudaMemcpyAsync(e->h_done, e->d_done.p, kMaxSlots * 4, cudaMemcpyDeviceToHost, s);
 }
 
 cudaError_t issue_any_wave(pt_engine* e, uint32_t kind, uint32_t size, uint32_t rounds) {

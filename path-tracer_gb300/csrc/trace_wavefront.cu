@@ -844,7 +844,13 @@ cudaError_t trace(Wavefront* wf, const ptd::World& w_in, const ptk::Tile& tile, 
         else
             e = w.any_alpha ? group_of(true_type(), false_type(), false_type())
                             : group_of(false_type(), false_type(), false_type());
-        PTW_TRY(e);
+        if (e != cudaSuccess) {
+            // a group that is refused in its middle may leave sort counts behind:
+            // the next call reserves anew, which waits for the device and clears them
+            wf->capacity = 0;
+            wf->have_start = false;
+            return e;
+        }
         if (!record) {
             PTW_TRY(cudaEventRecord(l.freed, stream));
             l.pending = true;

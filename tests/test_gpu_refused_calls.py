@@ -93,3 +93,56 @@ def test_waves_of_equal_launches_share_a_graph(library, precision):
         assert made == [1, 2, 6], made
         eng.close()
         """)
+
+
+def test_a_trace_refused_in_its_middle_leaves_nothing_behind(library):
+    """Every launch of a group in turn (with the hit sort's, whose counts the next group would find) is refused; the
+    call after it gives the image it would have given."""
+    wrapped_library.run(library, """
+        world = pt.World.cornell_box()
+        u = world.take_updates()
+        t = pt.PathTracer(u, (640, 640))
+        t.set_max_bounces(2)
+
+        def image():
+            t.set_tile((640, 640), (0, 0), (640, 640))
+            t.trace(4)
+            return t.read_tile(abi.PT_TILE_ACCUMULATION).tobytes()
+
+        want, refused = image(), 0
+        for first in range(40):
+            count("accept_launches").value, count("refuse_launch").value = first, 1
+            try:
+                assert image() == want
+            except pt.PathTracerError as e:
+                assert e.code == abi.PT_ERR_CUDA
+                refused += 1
+            done = count("refuse_launch").value == 1  # the group has fewer launches
+            count("accept_launches").value = count("refuse_launch").value = 0
+            assert image() == want
+            if done:
+                break
+        assert done and refused >= 12, refused
+        t.close()
+        """)
+
+
+def test_a_wave_of_plain_launches_refused_in_its_middle_ends_the_engine(library):
+    """Nothing follows the refused launch, and the engine says so from then on."""
+    wrapped_library.run(library, """
+        world = pt.World.cornell_box()
+        u = world.take_updates()
+        cam = abi.Camera.from_buffer_copy(u.camera.contents)
+        for first in (0, 1, 5):
+            eng = Engine(wave_paths=1 << 22, use_graphs=False)
+            sid = eng.add_scene(u)
+            count("accept_launches").value, count("refuse_launch").value = first, 1
+            for attempt in range(2):
+                try:
+                    eng.submit(sid, cam, 640, 640, 4, 3)
+                    assert False
+                except pt.PathTracerError as e:
+                    assert e.code == abi.PT_ERR_CUDA
+            assert count("refuse_launch").value == 0
+            eng.close()
+        """)

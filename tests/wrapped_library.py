@@ -1,8 +1,8 @@
 """libpt.so linked once more from its objects with some CUDA calls wrapped, so that a test can count them or have one
 refused on the host: cudaGraphInstantiate (pt_test_instantiated counts it, pt_test_refuse_instantiate refuses as many
 calls as it says) and cudaLaunchKernelExC, by which programmatic launches are made (pt_test_watched_launches counts those
-on the stream pt_test_watched_stream; pt_test_refuse_launch has as many as it says refused by the CUDA runtime, for
-blocks of more threads than there can be).  A script that uses it runs in a process of its own."""
+on the stream pt_test_watched_stream; after pt_test_accept_launches more, pt_test_refuse_launch has as many as it says
+refused by the CUDA runtime, for blocks of more threads than there can be).  A script that uses it runs in a process of its own."""
 import subprocess
 import sys
 import textwrap
@@ -12,7 +12,7 @@ from pathtracer import build
 WRAPS = r"""
 #include <cuda_runtime.h>
 extern "C" {
-int pt_test_instantiated = 0, pt_test_refuse_instantiate = 0, pt_test_refuse_launch = 0, pt_test_watched_launches = 0;
+int pt_test_instantiated = 0, pt_test_refuse_instantiate = 0, pt_test_accept_launches = 0, pt_test_refuse_launch = 0, pt_test_watched_launches = 0;
 void* pt_test_watched_stream = nullptr;
 cudaError_t __real_cudaGraphInstantiate(cudaGraphExec_t*, cudaGraph_t, unsigned long long);
 cudaError_t __wrap_cudaGraphInstantiate(cudaGraphExec_t* exec, cudaGraph_t graph, unsigned long long flags) {
@@ -26,7 +26,8 @@ cudaError_t __wrap_cudaGraphInstantiate(cudaGraphExec_t* exec, cudaGraph_t graph
 cudaError_t __real_cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**);
 cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* kernel, void** args) {
     pt_test_watched_launches += config->stream == pt_test_watched_stream;
-    if (pt_test_refuse_launch <= 0) return __real_cudaLaunchKernelExC(config, kernel, args);
+    if (pt_test_refuse_launch <= 0 || pt_test_accept_launches-- > 0) return __real_cudaLaunchKernelExC(config, kernel, args);
+    pt_test_accept_launches = 0;
     pt_test_refuse_launch -= 1;
     cudaLaunchConfig_t refused = *config;
     refused.blockDim.x = 4096;
